@@ -106,6 +106,13 @@ struct MGHost {
     int nlev = 0;
     MGHostLevel lev[MG_MAX + 1];
 };
+struct DevSys;
+// The aggregation hierarchy of system S from its cells (hierarchy.cu): level
+// k+1 groups the rows of level k by the 2x2x2 block of their cell
+// coordinates, until a level has at most kMGCoarsest rows or MG_MAX levels
+// exist.
+constexpr int kMGCoarsest = 512;
+void build_hierarchy(DevSys &S, cudaStream_t st);
 
 struct DevSys {
     int n = 0, npad = 0, nchunks = 0, d0 = 0;
