@@ -255,8 +255,8 @@ NS3D_API int ns3d_close(ns3d_handle *h);
 typedef struct ns3d_profile {
     /* index 0-4: the phases of a BiCGSTAB iteration inside the loop kernel
      * (K1 p-update, K2 SpMV+dot, K3 s-update, K4 SpMV+dots, K5 x/r-update):
-     * launches = iterations, ms = time between the grid barriers that end the
-     * phases (global timer of block 0).  index 5: launches of the loop kernel,
+     * launches = iterations, ms = time between the barriers (of the grid; of
+     * the block in small sets) that end the phases (global timer of block 0).  index 5: launches of the loop kernel,
      * ms by CUDA events.  rows: row-iterations of active systems. */
     int64_t launches[6];
     double ms[6];

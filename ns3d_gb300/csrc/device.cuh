@@ -117,9 +117,9 @@ struct KSys {  // one system of a solve set (device array)
     KState *st;
 };
 
-// chunk partials held per system (the FP64 loop uses 5 per chunk, the FP32
-// loop 5 per quarter chunk)
-constexpr int PART_PER_CHUNK = 20;
+// doubles held per chunk for reduction partials (the FP64 loop uses 5, the
+// FP32 loop 5 per quarter chunk, the one-chunk-per-block FP64 loop 84)
+constexpr int PART_PER_CHUNK = 84;
 
 // A solve set as a kernel argument (passed by value, read from constant
 // memory): the systems in chunk order, sys[0].chunk_begin == 0.  A solver

@@ -156,6 +156,12 @@ __device__ __forceinline__ void finish_loop(KState *st) {
     st->info = (st->error <= st->tol) ? 0 : 2;
 }
 
+__device__ __forceinline__ bool state_active(const KState &k) { return (k.done | k.paused) == 0; }
+
+}  // namespace ns3d
+#include "krylov_chunk.cuh"
+namespace ns3d {
+
 #define NS3D_CHUNK_LOOP                                                        \
     for (int c = blockIdx.x; c < A.total_chunks; c += gridDim.x) {            \
         const int sidx = sys_of_chunk(A, c);                                   \
@@ -231,15 +237,23 @@ __global__ void __launch_bounds__(LANES) k_kr_init(const __grid_constant__ KSetA
     }
 }
 
-// p = v = 0; x = 0 for a zero right-hand side
+// p = v = 0; x = 0 for a zero right-hand side; for the one-chunk-per-block
+// loop (`tags`) also the words it exchanges (krylov_chunk.cuh)
 template <int CAP>
-__global__ void k_kr_init2(const __grid_constant__ KSetArgT<CAP> A) {
+__global__ void k_kr_init2(const __grid_constant__ KSetArgT<CAP> A, bool tags) {
     NS3D_CHUNK_LOOP
         Row4 z;
 #pragma unroll
         for (int m = 0; m < RPL; ++m) z.v[m] = 0.0;
         st4(S.p + r0, z);
         st4(S.v + r0, z);
+        if (tags) {
+            for (double *q : {S.y, S.s, S.z, S.t}) st4(q + r0, z);
+            for (int k = threadIdx.x; k < TAG_KINDS * TAG_REPS; k += LANES) {
+                unsigned long long *slot = chunk_tag_words(S) + 2 * ((size_t)k * S.nchunks + lc);
+                slot[0] = slot[1] = 0;
+            }
+        }
         if (__ldcg(&S.st->zero_rhs)) st4(S.x + r0, z);
     }
 }
@@ -281,8 +295,6 @@ constexpr int kSpmvUnroll = NS3D_SPMV_UNROLL;
 #endif
 constexpr bool kNbrSmem = NS3D_NBR_SMEM != 0;
 constexpr size_t kNbrSmemBytes = kNbrSmem ? (size_t)LOOP_GROUPS * 6 * CH * sizeof(int) : 0;
-
-__device__ __forceinline__ bool state_active(const KState &k) { return (k.done | k.paused) == 0; }
 
 template <int CAP>
 __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
@@ -625,7 +637,7 @@ void launch_krylov_init(const KSetArgT<CAP> &A, cudaStream_t st) {
     if (A.total_chunks <= 0) return;
     count_launches(2);
     k_kr_init<CAP><<<kr_grid(A.total_chunks), LANES, 0, st>>>(A);
-    k_kr_init2<CAP><<<kr_grid(A.total_chunks), LANES, 0, st>>>(A);
+    k_kr_init2<CAP><<<kr_grid(A.total_chunks), LANES, 0, st>>>(A, A.total_chunks <= device_sm_count());
 }
 
 // Blocks of a loop-kernel launch.  Every block must be resident at once
@@ -683,6 +695,21 @@ cudaError_t launch_krylov_loop(const KSetArgT<CAP> &A, GridBar *bar, LoopProf *p
     KSetArgT<CAP> a = A;
     void *args[] = {&a, &bar, &prof, &max_iters};
     count_launches(1);
+    // A set whose share of the SMs gives every chunk a block runs one chunk
+    // per block (krylov_chunk.cuh), a larger one several chunks per block: a
+    // block has one thread per row of its chunk, and the exchange needs every
+    // block resident.  Measured, us per iteration, several per block -> one:
+    // 5 chunks 35.4 -> 14.8, 44 chunks 38.4 -> 21.0, 141 chunks 39.9 -> 23.3.
+    if (grid >= A.total_chunks && A.total_chunks <= device_sm_count()) {
+        static std::atomic<bool> ready{false};
+        if (!ready.load()) {
+            e = cudaFuncSetAttribute((const void *)k_kr_chunk<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)kChunkSmemBytes);
+            if (e != cudaSuccess) return e;
+            ready = true;
+        }
+        return cudaLaunchCooperativeKernel((const void *)k_kr_chunk<CAP>, A.total_chunks, CH, args, kChunkSmemBytes, st);
+    }
     return cudaLaunchCooperativeKernel((const void *)k_kr_loop<CAP>, grid, LOOP_THREADS, args, kNbrSmemBytes, st);
 }
 

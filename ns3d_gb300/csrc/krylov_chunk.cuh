@@ -1,0 +1,394 @@
+// krylov_chunk.cuh -- the BiCGSTAB loop of small solve sets: one 1024-row
+// chunk per block, one row per thread (included by krylov.cu).
+//
+// What bounds a small set is latency, not bytes: at 5 chunks an iteration of
+// the group kernel (k_kr_loop) took 35 us, of which its 128 threads per chunk
+// spent most waiting for their eight rows' loads in turn and in five grid
+// barriers of 1.5 us.  Here
+//   - the block keeps its chunk (coefficients, columns and vectors, 160 KB) in
+//     shared memory for the whole launch; the only data that blocks exchange
+//     are y, z and the chunk partials;
+//   - the exchange needs no grid barrier.  Every exchanged double travels as
+//     two 8-byte words that each hold 32 bits of it and the 32-bit epoch
+//     (iteration number) it belongs to; a reader polls the words it needs
+//     until both carry the epoch.  A word is valid by itself, so no fence is
+//     needed: an all-reduce over the chunk partials takes 0.5-0.8 us instead
+//     of barrier, fence and load (2.1 us), y and z reach a neighbouring block
+//     in 1.3 us instead of 2.2 us;
+//   - neighbours inside the chunk are read from shared memory;
+//   - the systems of a set do not wait for each other.
+// The arithmetic and its order are those of k_kr_loop: rows are multiplied by
+// spmv_row's chain, lane l of a chunk accumulates rows l, l + 128, ... (the
+// operands pass through shared memory), then the same trees.
+//
+// A word is rewritten only after every reader has read it: y of iteration
+// i + 1 is stored after the reduction that ends iteration i, which needs a
+// partial of every block of the system, stored after its last read of y.  The
+// same holds for z and each partial.  The words start at zero (k_kr_init2)
+// and the epoch, the system's iteration count of this solve, at 1.
+//
+// The words of y live in S.y (low halves) and S.s (high halves), those of z
+// in S.z and S.t, those of the partials in S.part (chunk_tag_words).
+//
+// What bounds it now: per block and iteration 27 x 1024 FP64 operations at
+// two per clock (6.7 us), three reductions of about 2.3 us (a chain of eight
+// 68-cycle FMAs, two trees, one exchange, one division) and two exchanges of
+// y and z.
+#pragma once
+
+namespace ns3d {
+
+// Copies of each chunk partial: block b polls copy b % TAG_REPS, because one
+// copy polled by 152 blocks takes 2.9 us where 44 blocks take 0.8 us.
+constexpr int TAG_REPS = 8;
+constexpr int TAG_KINDS = 5;  // <r0,v>, <t,t>, <t,s>, <r0,r>, <r,r>
+// S.part of a system: [0, 4 n) the plain partials of k_kr_init and
+// k_kr_restart, then 2 words per kind, copy and chunk
+__device__ __forceinline__ unsigned long long *chunk_tag_words(const KSys &S) {
+    return reinterpret_cast<unsigned long long *>(S.part + 4 * (size_t)S.nchunks);
+}
+static_assert(PART_PER_CHUNK >= 4 + 2 * TAG_KINDS * TAG_REPS, "tagged partials");
+
+constexpr size_t kChunkSmemBytes = (size_t)(7 + 10) * CH * sizeof(double) + (size_t)6 * CH * sizeof(int);
+
+__device__ __forceinline__ unsigned long long tag_lo(double v, unsigned int ep) {
+    return ((unsigned long long)ep << 32) | (unsigned int)__double2loint(v);
+}
+__device__ __forceinline__ unsigned long long tag_hi(double v, unsigned int ep) {
+    return ((unsigned long long)ep << 32) | (unsigned int)__double2hiint(v);
+}
+__device__ __forceinline__ double tag_value(unsigned long long lo, unsigned long long hi) {
+    return __hiloint2double((int)(unsigned int)hi, (int)(unsigned int)lo);
+}
+__device__ __forceinline__ bool tag_ok(unsigned long long lo, unsigned long long hi, unsigned int ep) {
+    return (unsigned int)(lo >> 32) == ep && (unsigned int)(hi >> 32) == ep;
+}
+__device__ __forceinline__ unsigned long long ld_word(const void *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_word(void *p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ void ld_words(const void *p, unsigned long long &a, unsigned long long &b) {
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st_words(void *p, unsigned long long a, unsigned long long b) {
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+
+// Bounded polling: false when the wait has run out (the same limit as the
+// grid barrier's), after setting bar->err and the thread's flag; the block
+// stops at its next barrier, which combines the flags.
+struct PollLimit {
+    GridBar *bar;
+    int &bad;
+    unsigned int polls = 0;
+    unsigned long long t0 = 0;
+    __device__ PollLimit(GridBar *b, int &f) : bar(b), bad(f) {}
+    __device__ __forceinline__ bool again() {
+        if ((++polls & 255u) != 0) return true;
+        const unsigned long long now = global_ns();
+        if (polls == 256u) t0 = now;
+        const unsigned long long lim = bar->limit_ns ? bar->limit_ns : kBarrierLimitNs;
+        if (now - t0 <= lim && polls <= 0x7fffffffu) return true;
+        atomicExch(&bar->err, 1);
+        bad = 1;
+        return false;
+    }
+};
+
+// The column values of the thread's row, slots W, E, S, N, B, T: neighbours
+// in the chunk from `own` (shared), the others from their tagged words; a
+// missing neighbour gets the row's own value (its product is skipped).
+// Outside the chunk a row has W and E and, at the chunk's ends, one of S and
+// N and one of B and T: those four are polled at once (a second round trip
+// costs 0.6 us; polling all six at once needs registers that spill).
+__device__ __forceinline__ void gather_tagged(const int *s_col, int base, int t, const double *own, const double *lo,
+                                              const double *hi, unsigned int ep, double (&x)[6], GridBar *bar,
+                                              int &bad) {
+    unsigned int need = 0;
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+        const int c = s_col[d * CH];
+        const unsigned int q = (unsigned int)(c - base);
+        const bool ext = c >= 0 && q >= (unsigned int)CH;
+        x[d] = own[!ext && c >= 0 ? q : t];
+        need |= (unsigned int)ext << d;
+    }
+    PollLimit limit(bar, bad);
+    while (need) {
+        const bool north = (need >> 2 & 1u) == 0, top = (need >> 4 & 1u) == 0;
+        const unsigned int bit[4] = {need & 1u, need & 2u, need & (north ? 8u : 4u), need & (top ? 32u : 16u)};
+        const int slot[4] = {0, 1, north ? 3 : 2, top ? 5 : 4};
+        unsigned long long a[4], b[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (bit[k]) {
+                const int c = s_col[slot[k] * CH];
+                a[k] = ld_word(lo + c);
+                b[k] = ld_word(hi + c);
+            }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (bit[k] && tag_ok(a[k], b[k], ep)) {
+                const double val = tag_value(a[k], b[k]);
+                if (k < 2) x[k] = val;
+                else if (k == 2) (north ? x[3] : x[2]) = val;
+                else (top ? x[5] : x[4]) = val;
+                need &= ~bit[k];
+            }
+        if (need && !limit.again()) return;
+    }
+}
+
+// The tree sum of lanes_tree_sum over the 128 threads of one group, of which
+// only the first `n` hold a value and the others +0: a level that would only
+// add those zeros is left out (v + 0 = v; no value here is -0).  FP64 adds
+// have a latency of 68 cycles, a level with its shuffle 94.  Valid in the
+// group's first thread; with n <= 32 only its first warp takes part.
+__device__ __forceinline__ double group_tree(double v, int n, int lane, double *red, GroupSync sync) {
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1)
+        if (off < n) v = v + __shfl_down_sync(0xffffffffu, v, off);
+    if (n <= 32) return v;
+    if ((lane & 31) == 0) red[lane >> 5] = v;
+    sync();
+    double r = 0.0;
+    if (lane < 32) {
+        r = lane < LANES / 32 ? red[lane] : 0.0;
+        if (n > 64) r = r + __shfl_down_sync(0xffffffffu, r, 2);
+        r = r + __shfl_down_sync(0xffffffffu, r, 1);
+    }
+    return r;
+}
+
+// One dot product of a system over all its chunks, by one group of 128
+// threads: the chunk's partial from the operands in shared memory, published
+// in TAG_REPS copies, and the sum of all chunks' partials in the fixed order.
+// Valid in the group's first thread.  Every thread of the group calls
+// `published` once its part in publishing is done.
+template <class Published>
+__device__ __forceinline__ double dot_all(const KSys &S, int lc, int kind, const double *a, const double *b, int lane,
+                                          unsigned int ep, unsigned int want, double *red, GroupSync sync,
+                                          GridBar *bar, int &bad, Published published) {
+    const int n = S.nchunks;
+    double acc = 0.0;
+    const int rows = min(CH, S.n - lc * CH);
+#pragma unroll
+    for (int m = 0; m < RPL; ++m)
+        if (lane + m * LANES < rows) acc = __fma_rn(a[lane + m * LANES], b[lane + m * LANES], acc);
+    double part = group_tree(acc, LANES, lane, red, sync);
+    unsigned long long *slots = chunk_tag_words(S) + 2 * (size_t)(kind * TAG_REPS) * n;
+    if (lane < 32) {
+        part = __shfl_sync(0xffffffffu, part, 0);
+        if (lane < TAG_REPS) st_words(slots + 2 * ((size_t)lane * n + lc), tag_lo(part, ep), tag_hi(part, ep));
+    }
+    published();
+    if (n <= 32 && lane >= 32) return 0.0;  // the first warp alone combines them
+    const unsigned long long *mine = slots + 2 * (size_t)(blockIdx.x % TAG_REPS) * n;
+    PollLimit limit(bar, bad);
+    double sum = 0.0;
+    for (int i = lane; i < n; i += LANES) {
+        unsigned long long lo, hi;
+        while (true) {
+            ld_words(mine + 2 * (size_t)i, lo, hi);
+            if (tag_ok(lo, hi, want) || !limit.again()) break;
+        }
+        sum = sum + tag_value(lo, hi);
+    }
+    return group_tree(sum, min(n, LANES), lane, red + LANES / 32, sync);
+}
+
+template <int CAP>
+__global__ void __launch_bounds__(CH, 1)
+    k_kr_chunk(const __grid_constant__ KSetArgT<CAP> A, GridBar *bar, LoopProf *prof, int max_iters) {
+    static_assert(CH == 1024, "one thread per row of a chunk");
+    extern __shared__ double sm_chunk[];
+    // the chunk: coefficients and vectors, [7 + 10][CH]
+    double *const s_cf = sm_chunk;
+    double *const s_r0 = s_cf + 7 * CH, *const s_x = s_r0 + CH, *const s_p = s_x + CH, *const s_y = s_p + CH,
+                  *const s_v = s_y + CH, *const s_s = s_v + CH, *const s_z = s_s + CH, *const s_t = s_z + CH,
+                  *const s_r = s_t + CH, *const s_invd = s_r + CH;
+    int *const s_col = reinterpret_cast<int *>(s_invd + CH) + threadIdx.x;  // [6][CH]: the thread's columns
+    __shared__ KState st;
+    __shared__ double s_red[2][2 * (LANES / 32)], s_other, s_ratio;
+    const int t = threadIdx.x, gi = t / LANES;
+    const KSys &S = A.sys[sys_of_chunk(A, (int)blockIdx.x)];
+    const int lc = (int)blockIdx.x - S.chunk_begin, base = lc * CH, row = base + t;
+    if (t == 0) st = *S.st;
+    const bool timing = prof != nullptr && blockIdx.x == 0 && t == 0;
+    __shared__ unsigned long long s_tp[6];  // phase times of block 0
+    if (timing)
+        for (int k = 0; k < 6; ++k) s_tp[k] = 0;
+    __syncthreads();
+    if (!state_active(st)) return;  // the same in every block of the system
+    bool has[6];  // the row's entries
+    {
+        const size_t np = (size_t)S.npad;
+#pragma unroll
+        for (int d = 0; d < 7; ++d) s_cf[d * CH + t] = ro(S.coef + d * np + row);
+#pragma unroll
+        for (int d = 0; d < 6; ++d) {
+            const int c = ro(S.nbr + d * np + row);
+            s_col[d * CH] = c;
+            has[d] = c >= 0;
+        }
+    }
+    s_r0[t] = S.r0[row];
+    s_invd[t] = ro(S.invdiag + row);
+    s_p[t] = S.p[row];
+    s_v[t] = S.v[row];
+    s_r[t] = S.r[row];
+    s_x[t] = S.x[row];
+    const bool wlate = has[0] && s_col[0] == row - 1, eearly = has[1] && s_col[CH] == row + 1;
+    const bool rare = __any_sync(0xffffffffu, wlate || eearly);
+    // A x for the thread's row from its own value and the six columns'; the
+    // chain of spmv_row_nb
+    auto product = [&](double xp, const double (&xc)[6]) {
+        const double *cf = s_cf + t;
+        double acc = 0.0;
+        if (rare) {
+            if (!wlate && has[0]) acc = __fma_rn(cf[1 * CH], xc[0], acc);
+            if (has[2]) acc = __fma_rn(cf[3 * CH], xc[2], acc);
+            if (has[4]) acc = __fma_rn(cf[5 * CH], xc[4], acc);
+            if (wlate) acc = __fma_rn(cf[1 * CH], xc[0], acc);
+            acc = __fma_rn(cf[0], xp, acc);
+            if (eearly) acc = __fma_rn(cf[2 * CH], xc[1], acc);
+            if (has[5]) acc = __fma_rn(cf[6 * CH], xc[5], acc);
+            if (has[3]) acc = __fma_rn(cf[4 * CH], xc[3], acc);
+            if (!eearly && has[1]) acc = __fma_rn(cf[2 * CH], xc[1], acc);
+        } else {
+            if (has[0]) acc = __fma_rn(cf[1 * CH], xc[0], acc);
+            if (has[2]) acc = __fma_rn(cf[3 * CH], xc[2], acc);
+            if (has[4]) acc = __fma_rn(cf[5 * CH], xc[4], acc);
+            acc = __fma_rn(cf[0], xp, acc);
+            if (has[5]) acc = __fma_rn(cf[6 * CH], xc[5], acc);
+            if (has[3]) acc = __fma_rn(cf[4 * CH], xc[3], acc);
+            if (has[1]) acc = __fma_rn(cf[2 * CH], xc[1], acc);
+        }
+        return acc;
+    };
+    auto mark = [&](int k) {
+        if (timing) {
+            const unsigned long long now = global_ns();
+            s_tp[k] += now - s_tp[5];
+            s_tp[5] = now;
+        }
+    };
+    if (timing) s_tp[5] = global_ns();
+    // a test (ns3d_debug_barrier_timeout) makes every wait for a chunk partial
+    // run out: it waits for epochs that are never written
+    const unsigned int never = bar->bias ? 0x80000000u : 0u;
+    const GroupSync sync{gi + 1};
+    auto nothing = [] {};
+    int it = 0, bad = 0;
+    for (; it < max_iters; ++it) {
+        const unsigned int ep = (unsigned int)st.work + 1u;  // uniform: st changes only between block barriers
+        double xc[6];
+        // K1: p = r + beta (p - w v); y = D^-1 p
+        {
+            const double p = __fma_rn(st.beta, __fma_rn(-st.w, s_v[t], s_p[t]), s_r[t]);
+            const double y = s_invd[t] * p;
+            st_word(S.y + row, tag_lo(y, ep));
+            st_word(S.s + row, tag_hi(y, ep));
+            s_y[t] = y;
+            s_p[t] = p;
+        }
+        __syncthreads();
+        mark(0);
+        // K2: v = A y, <r0, v>
+        gather_tagged(s_col, base, t, s_y, S.y, S.s, ep, xc, bar, bad);
+        s_v[t] = product(s_y[t], xc);
+        if (__syncthreads_or(bad)) break;
+        if (gi == 0) {
+            const double d = dot_all(S, lc, 0, s_r0, s_v, t, ep, ep | never, s_red[0], sync, bar, bad, nothing);
+            if (t == 0) st.alpha = st.rho / d;
+        }
+        if (__syncthreads_or(bad)) break;
+        mark(1);
+        // K3: s = r - alpha v; z = D^-1 s
+        {
+            const double s = __fma_rn(-st.alpha, s_v[t], s_r[t]);
+            const double z = s_invd[t] * s;
+            st_word(S.z + row, tag_lo(z, ep));
+            st_word(S.t + row, tag_hi(z, ep));
+            s_z[t] = z;
+            s_s[t] = s;
+        }
+        __syncthreads();
+        mark(2);
+        // K4: t = A z, <t, t>, <t, s>
+        gather_tagged(s_col, base, t, s_z, S.z, S.t, ep, xc, bar, bad);
+        s_t[t] = product(s_z[t], xc);
+        if (__syncthreads_or(bad)) break;
+        if (gi < 2) {
+            const double d = dot_all(S, lc, 1 + gi, s_t, gi == 0 ? s_t : s_s, t % LANES, ep, ep | never, s_red[gi], sync,
+                                     bar, bad, nothing);
+            if (t == LANES) s_other = d;
+            asm volatile("bar.sync 3, %0;" ::"n"(2 * LANES) : "memory");
+            if (t == 0) st.w = (d > 0.0) ? s_other / d : 0.0;
+        }
+        if (__syncthreads_or(bad)) break;
+        mark(3);
+        // K5: r = s - w t, <r0, r>, <r, r>; x += alpha y + w z
+        const double alpha = st.alpha, w = st.w;
+        s_r[t] = __fma_rn(-w, s_t[t], s_s[t]);
+        __syncthreads();
+        if (gi < 2) {
+            // the partials are published: the other warps' FP64 work may start
+            auto published = [] { asm volatile("bar.arrive 4, %0;" ::"n"(CH) : "memory"); };
+            const double d = dot_all(S, lc, 3 + gi, gi == 0 ? s_r0 : s_r, s_r, t % LANES, ep, ep | never, s_red[gi], sync,
+                                     bar, bad, published);
+            if (t == LANES) s_other = d;
+            asm volatile("bar.sync 3, %0;" ::"n"(2 * LANES) : "memory");
+            if (t < 32) asm volatile("bar.sync 5, 64;" ::: "memory");  // s_ratio is written
+            if (t == 0) {
+                const double f0r = d, frr = s_other;
+                st.rr = frr;
+                st.iter += 1;
+                st.work += 1;
+                if (!(frr > st.tol2 && st.iter < st.maxit)) {
+                    finish_loop(&st);
+                } else if (fabs(f0r) < DBL_EPSILON * DBL_EPSILON * st.r0_sqnorm) {
+                    st.paused = 1;  // the host recomputes r = b - A x and r0
+                } else {
+                    st.beta = (f0r / st.rho) * s_ratio;
+                    st.rho = f0r;
+                }
+            }
+        } else {
+            // x and the second ratio of beta, in the time the partials travel:
+            // before they are published this FP64 work would delay them
+            if (gi == 2 && t < 2 * LANES + 32) {
+                if (t == 2 * LANES) s_ratio = alpha / w;
+                asm volatile("bar.arrive 5, 64;" ::: "memory");
+            }
+            asm volatile("bar.sync 4, %0;" ::"n"(CH) : "memory");
+            for (int q = t - 2 * LANES; q < CH; q += CH - 2 * LANES)
+                s_x[q] = __fma_rn(w, s_z[q], __fma_rn(alpha, s_y[q], s_x[q]));
+        }
+        if (__syncthreads_or(bad)) break;
+        mark(4);
+        if (!state_active(st)) {
+            ++it;
+            break;
+        }
+    }
+    S.p[row] = s_p[t];
+    S.v[row] = s_v[t];
+    S.r[row] = s_r[t];
+    S.x[row] = s_x[t];
+    if (lc == 0 && t == 0) {
+        st.counter = 0;
+        *S.st = st;
+    }
+    if (timing) {
+        for (int k = 0; k < 5; ++k) prof->ns[k] += s_tp[k];
+        prof->iters += it;
+        prof->ok = bad ? 0 : 1;
+    }
+}
+
+}  // namespace ns3d
