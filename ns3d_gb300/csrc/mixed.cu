@@ -273,11 +273,11 @@ struct MGView {
     int n, npad;
     const int *nbr;
     const float *coef, *invdiag;
-    float *x, *b, *t;
+    float *x, *b, *t, *t2;
 };
 
 // level k of the hierarchy of S (level 0: the FP32 system, solution x0 of
-// right-hand side b0, scratch S.t)
+// right-hand side b0, scratch S.t and S.p2)
 __device__ __forceinline__ MGView mg_level(const MSys &S, int k, const float *b0, float *x0) {
     MGView L;
     if (k == 0) {
@@ -289,6 +289,7 @@ __device__ __forceinline__ MGView mg_level(const MSys &S, int k, const float *b0
         L.x = x0;
         L.b = const_cast<float *>(b0);
         L.t = S.t;
+        L.t2 = S.p2;
     } else {
         const MGLevel &G = S.mg.lev[k];
         L.n = G.n;
@@ -299,23 +300,48 @@ __device__ __forceinline__ MGView mg_level(const MSys &S, int k, const float *b0
         L.x = G.x;
         L.b = G.b;
         L.t = G.t;
+        L.t2 = G.t2;
     }
     return L;
 }
 
-// row of A x at one level (slot d+1 couples through neighbour d; a missing
-// neighbour has a zero coefficient and gathers the row itself)
-__device__ __forceinline__ float mg_spmv(const MGView &L, int row, const float *x) {
+// row of A x at one level, x given by a function of the row (slot d+1 couples
+// through neighbour d; a missing neighbour has a zero coefficient and takes
+// the row itself)
+template <class F>
+__device__ __forceinline__ float mg_spmv_fn(const MGView &L, int row, F xf) {
     const size_t np = (size_t)L.npad;
     const int *nb = L.nbr + row;
     const float *cf = L.coef + row;
-    float acc = ro(cf) * x[row];
+    float acc = ro(cf) * xf(row);
 #pragma unroll
     for (int d = 0; d < 6; ++d) {
         const int c = ro(nb + d * np);
-        acc = __fmaf_rn(ro(cf + (d + 1) * np), x[c >= 0 ? c : row], acc);
+        acc = __fmaf_rn(ro(cf + (d + 1) * np), xf(c >= 0 ? c : row), acc);
     }
     return acc;
+}
+__device__ __forceinline__ float mg_spmv(const MGView &L, int row, const float *x) {
+    return mg_spmv_fn(L, row, [&](int c) { return x[c]; });
+}
+
+// The passes of a V-cycle, one row each.  Down: the residual t of the
+// level's Jacobi start x, then the restriction of t with the next level's
+// Jacobi start.  Up: the residual t2 of x with the coarse correction cx
+// added on the fly, then x with correction and one damped Jacobi sweep.
+__device__ __forceinline__ void mg_down(const MGView &L, int r) { L.t[r] = L.b[r] - mg_spmv(L, r, L.x); }
+__device__ __forceinline__ void mg_restrict(const MGLevel &C, const float *t, float w, int I) {
+    float acc = 0.0f;
+    for (int q = C.mstart[I]; q < C.mstart[I + 1]; ++q) acc += t[C.members[q]];
+    C.b[I] = acc;
+    C.x[I] = w * C.invdiag[I] * acc;
+}
+__device__ __forceinline__ void mg_up(const MGView &L, const int *agg, const float *cx, int r) {
+    L.t2[r] = L.b[r] - mg_spmv_fn(L, r, [&](int c) { return L.x[c] + cx[ro(agg + c)]; });
+}
+__device__ __forceinline__ void mg_finish(const MGView &L, const int *agg, const float *cx, float w, int r) {
+    const float x = L.x[r] + cx[ro(agg + r)];
+    L.x[r] = x + w * L.invdiag[r] * L.t2[r];
 }
 
 // Jacobi sweeps on the coarsest level by the calling block: x = w D^-1 b,
@@ -331,49 +357,203 @@ __device__ void mg_coarsest(const MGView &L, float w, int sweeps) {
     }
 }
 
+// ---- the tail of the hierarchy in shared memory ------------------------------
+// The levels of a few hundred rows cost a grid barrier (1.6 us) per pass and
+// next to no work, and the 30 sweeps on the coarsest one 15 us of L2 latency
+// in one block while the others waited.  Every block keeps the tail's
+// matrices in shared memory for the launch and runs it itself, on the same
+// restricted residual and with the same arithmetic: no grid barrier inside
+// the tail and none to hand out its result.
+struct TailLevel {
+    int n;
+    float *coef, *invdiag, *x, *x2, *b, *t;  // [7][n], [n], ...
+    int *nbr;                                // [6][n]
+    int *agg, *mstart, *members;             // levels above the first of the tail
+};
+using TailLevels = TailLevel[MG_MAX + 1];
+
+__device__ void mg_tail_load(const MGSet &G, float *mem, TailLevels &T) {
+    if (threadIdx.x == 0) {
+        float *q = mem;
+        for (int k = G.tail; k <= G.nlev; ++k) {
+            TailLevel &L = T[k];
+            const int n = L.n = G.lev[k].n;
+            L.coef = q;
+            L.invdiag = q + 7 * n;
+            L.x = q + 8 * n;
+            L.x2 = q + 9 * n;
+            L.b = q + 10 * n;
+            L.t = q + 11 * n;
+            L.nbr = reinterpret_cast<int *>(q + 12 * n);
+            q += 18 * n;
+            if (k > G.tail) {
+                const int nf = G.lev[k - 1].n;
+                L.mstart = reinterpret_cast<int *>(q);
+                L.members = L.mstart + n + 1;
+                L.agg = L.members + nf;
+                q += n + 1 + 2 * nf;
+            }
+        }
+    }
+    __syncthreads();
+    for (int k = G.tail; k <= G.nlev; ++k) {
+        const MGLevel &C = G.lev[k];
+        const TailLevel &L = T[k];
+        for (int r = threadIdx.x; r < L.n; r += blockDim.x) {
+#pragma unroll
+            for (int d = 0; d < 7; ++d) L.coef[d * L.n + r] = ro(C.coef + (size_t)d * C.npad + r);
+#pragma unroll
+            for (int d = 0; d < 6; ++d) {
+                const int c = ro(C.nbr + (size_t)d * C.npad + r);
+                L.nbr[d * L.n + r] = c >= 0 ? c : r;  // a missing neighbour takes the row itself
+            }
+            L.invdiag[r] = ro(C.invdiag + r);
+        }
+        if (k > G.tail) {
+            const int nf = G.lev[k - 1].n;
+            for (int r = threadIdx.x; r <= L.n; r += blockDim.x) L.mstart[r] = ro(C.mstart + r);
+            for (int r = threadIdx.x; r < nf; r += blockDim.x) {
+                L.members[r] = ro(C.members + r);
+                L.agg[r] = ro(C.agg + r);
+            }
+        }
+    }
+    __syncthreads();
+}
+
+template <class F>
+__device__ __forceinline__ float tail_spmv(const TailLevel &L, int r, F xf) {
+    float acc = L.coef[r] * xf(r);
+#pragma unroll
+    for (int d = 0; d < 6; ++d) acc = __fmaf_rn(L.coef[(d + 1) * L.n + r], xf(L.nbr[d * L.n + r]), acc);
+    return acc;
+}
+
+// One V-cycle of the tail by the calling block, right-hand side restricted
+// from the residual t of the level above; the result is T[G.tail].x.
+__device__ void mg_tail(const MGSet &G, TailLevels &T, const float *t) {
+    const int K = G.nlev, tid = threadIdx.x, nth = blockDim.x;
+    const float w = G.omega;
+    for (int k = G.tail; k <= K; ++k) {
+        const TailLevel &L = T[k];
+        const MGLevel &C = G.lev[k];
+        const bool first = k == G.tail;
+        const int *mstart = first ? C.mstart : L.mstart, *members = first ? C.members : L.members;
+        const float *src = first ? t : T[k - 1].t;
+        for (int I = tid; I < L.n; I += nth) {
+            float acc = 0.0f;
+            for (int q = mstart[I]; q < mstart[I + 1]; ++q) acc += first ? __ldcg(src + members[q]) : src[members[q]];
+            L.b[I] = acc;
+            L.x[I] = w * L.invdiag[I] * acc;
+        }
+        __syncthreads();
+        if (k == K) break;
+        for (int r = tid; r < L.n; r += nth) L.t[r] = L.b[r] - tail_spmv(L, r, [&](int c) { return L.x[c]; });
+        __syncthreads();
+    }
+    {
+        // sweeps on the coarsest level: x and x2 in turn, one barrier per sweep
+        const TailLevel &L = T[K];
+        float *from = L.x, *to = L.x2;
+        if (L.n <= nth) {  // one row per thread, its matrix row in registers, the warps with rows only
+            const int warps = (L.n + 31) / 32;
+            if (tid < 32 * warps) {
+                const int r = min(tid, L.n - 1);
+                float cf[7];
+                int nb[6];
+#pragma unroll
+                for (int d = 0; d < 7; ++d) cf[d] = L.coef[d * L.n + r];
+#pragma unroll
+                for (int d = 0; d < 6; ++d) nb[d] = L.nbr[d * L.n + r];
+                const float wd = w * L.invdiag[r], b = L.b[r];
+                float x = from[r];
+                for (int it = 0; it < G.sweeps; ++it) {
+                    float acc = cf[0] * x;
+#pragma unroll
+                    for (int d = 0; d < 6; ++d) acc = __fmaf_rn(cf[d + 1], from[nb[d]], acc);
+                    x += wd * (b - acc);
+                    if (tid < L.n) to[r] = x;
+                    float *const o = from;
+                    from = to;
+                    to = o;
+                    asm volatile("bar.sync 9, %0;" ::"r"(32 * warps) : "memory");
+                }
+            }
+            __syncthreads();
+            from = (G.sweeps & 1) ? L.x2 : L.x;
+        } else {
+            for (int it = 0; it < G.sweeps; ++it) {
+                for (int r = tid; r < L.n; r += nth)
+                    to[r] = from[r] + w * L.invdiag[r] * (L.b[r] - tail_spmv(L, r, [&](int c) { return from[c]; }));
+                __syncthreads();
+                float *const o = from;
+                from = to;
+                to = o;
+            }
+        }
+        if (from != L.x) {
+            for (int r = tid; r < L.n; r += nth) L.x[r] = from[r];
+            __syncthreads();
+        }
+    }
+    for (int k = K - 1; k >= G.tail; --k) {
+        const TailLevel &L = T[k], &C = T[k + 1];
+        for (int r = tid; r < L.n; r += nth)
+            L.t[r] = L.b[r] - tail_spmv(L, r, [&](int c) { return L.x[c] + C.x[C.agg[c]]; });
+        __syncthreads();
+        for (int r = tid; r < L.n; r += nth) {
+            const float x = L.x[r] + C.x[C.agg[r]];
+            L.x[r] = x + w * L.invdiag[r] * L.t[r];
+        }
+        __syncthreads();
+    }
+}
+
 // x0 = M^-1 b0: one V-cycle -- a damped Jacobi sweep from zero, the residual
 // restricted to the next level (sum over the block), ... , Jacobi sweeps on
-// the coarsest level in block 0, then on the way up the correction of the
-// coarser level added and one damped Jacobi sweep.  Every thread of the grid
-// calls it (grid barriers between the passes); false when a barrier failed.
-// The fine level's Jacobi start x0 = w D^-1 b0 is already written by the
-// loop phase that computed b0 (p or s), so the V-cycle starts with the
-// fine residual.  (Fusing the Jacobi start, residual and restriction into
-// one pass per coarse row -- one grid barrier per level instead of three,
-// neighbours' starts recomputed -- gave the same values but measured 3-8%
-// slower, on the coarse levels as on the fine one.)
-__device__ bool mg_apply(const MSys &S, const float *b0, float *x0, GridBar *bar, unsigned int &target,
+// the coarsest level, then on the way up the correction of the coarser level
+// added and one damped Jacobi sweep.  Every thread of the grid calls it (grid
+// barriers between the passes); false when a barrier failed.  The fine
+// level's Jacobi start x0 = w D^-1 b0 is already written by the loop phase
+// that computed b0 (p or s), so the V-cycle starts with the fine residual.
+// Two passes down and two up per level: the restriction writes the next
+// level's Jacobi start, and the correction is added where x is read (a pass
+// that adds it first costs a grid barrier and 12 bytes a row more).  The up
+// pass writes its residual to t2, because other blocks may still read t for
+// their tail.  (Fusing residual and restriction too, one pass per coarse row,
+// measured 3-8% slower: it walks the fine rows out of order.)
+// With the tail in shared memory an iteration of a 205 K-row system (five
+// levels) has 27 grid barriers instead of 53: six IDEAL outer iterations
+// 112.6 -> 83.1 ms; 3.6 M rows, six SIMPLEC outer iterations, 289 -> 271 ms.
+__device__ bool mg_apply(const MSys &S, const float *b0, float *x0, TailLevels &T, GridBar *bar, unsigned int &target,
                          int *s_ok) {
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int gth = gridDim.x * blockDim.x;
-    const int K = S.mg.nlev;
+    const int K = S.mg.nlev, tail = S.mg.tail;
     const float w = S.mg.omega;
     for (int k = 0; k < K; ++k) {
         const MGView L = mg_level(S, k, b0, x0);
-        const MGLevel &C = S.mg.lev[k + 1];
-        if (k > 0) {
-            for (int r = gtid; r < L.n; r += gth) L.x[r] = w * L.invdiag[r] * L.b[r];
-            if (!grid_sync(bar, target, s_ok)) return false;
-        }
-        for (int r = gtid; r < L.n; r += gth) L.t[r] = L.b[r] - mg_spmv(L, r, L.x);
+        for (int r = gtid; r < L.n; r += gth) mg_down(L, r);
         if (!grid_sync(bar, target, s_ok)) return false;
-        for (int I = gtid; I < C.n; I += gth) {
-            float acc = 0.0f;
-            for (int q = C.mstart[I]; q < C.mstart[I + 1]; ++q) acc += L.t[C.members[q]];
-            C.b[I] = acc;
+        if (k + 1 == tail) {
+            mg_tail(S.mg, T, L.t);
+            break;
         }
+        const MGLevel &C = S.mg.lev[k + 1];
+        for (int I = gtid; I < C.n; I += gth) mg_restrict(C, L.t, w, I);
         if (!grid_sync(bar, target, s_ok)) return false;
     }
-    if (blockIdx.x == 0) mg_coarsest(mg_level(S, K, b0, x0), w, S.mg.sweeps);
-    if (!grid_sync(bar, target, s_ok)) return false;
-    for (int k = K - 1; k >= 0; --k) {
+    if (tail > K) {
+        if (blockIdx.x == 0) mg_coarsest(mg_level(S, K, b0, x0), w, S.mg.sweeps);
+        if (!grid_sync(bar, target, s_ok)) return false;
+    }
+    for (int k = min(K, tail) - 1; k >= 0; --k) {
         const MGView L = mg_level(S, k, b0, x0);
-        const MGLevel &C = S.mg.lev[k + 1];
-        for (int r = gtid; r < L.n; r += gth) L.x[r] += C.x[C.agg[r]];
+        const int *agg = S.mg.lev[k + 1].agg;
+        const float *cx = k + 1 == tail ? T[tail].x : S.mg.lev[k + 1].x;
+        for (int r = gtid; r < L.n; r += gth) mg_up(L, agg, cx, r);
         if (!grid_sync(bar, target, s_ok)) return false;
-        for (int r = gtid; r < L.n; r += gth) L.t[r] = L.b[r] - mg_spmv(L, r, L.x);
-        if (!grid_sync(bar, target, s_ok)) return false;
-        for (int r = gtid; r < L.n; r += gth) L.x[r] += w * L.invdiag[r] * L.t[r];
+        for (int r = gtid; r < L.n; r += gth) mg_finish(L, agg, cx, w, r);
         if (!grid_sync(bar, target, s_ok)) return false;
     }
     return true;
@@ -420,29 +600,11 @@ __device__ bool mg_apply_set(const MSetArgT<CAP> &A, const KState *sst, const in
         if (on(q)) kmax = max(kmax, A.sys[q].mg.nlev);
     for (int k = 0; k < kmax; ++k) {
         auto part = [&](int q) { return on(q) && k < A.sys[q].mg.nlev; };
-        if (k > 0) {  // the fine level's start is written by the loop phase
-            mg_rows(A, part, [&](int q) { return A.sys[q].mg.lev[k].n; },
-                    [&](int q, int r) {
-                        const MGView L = lvl(q, k);
-                        const float w = A.sys[q].mg.omega;
-                        L.x[r] = w * L.invdiag[r] * L.b[r];
-                    });
-            if (!grid_sync(bar, target, s_ok)) return false;
-        }
         mg_rows(A, part, [&](int q) { return k == 0 ? A.sys[q].n : A.sys[q].mg.lev[k].n; },
-                [&](int q, int r) {
-                    const MGView L = lvl(q, k);
-                    L.t[r] = L.b[r] - mg_spmv(L, r, L.x);
-                });
+                [&](int q, int r) { mg_down(lvl(q, k), r); });
         if (!grid_sync(bar, target, s_ok)) return false;
         mg_rows(A, part, [&](int q) { return A.sys[q].mg.lev[k + 1].n; },
-                [&](int q, int I) {
-                    const MGView L = lvl(q, k);
-                    const MGLevel &C = A.sys[q].mg.lev[k + 1];
-                    float acc = 0.0f;
-                    for (int m = C.mstart[I]; m < C.mstart[I + 1]; ++m) acc += L.t[C.members[m]];
-                    C.b[I] = acc;
-                });
+                [&](int q, int I) { mg_restrict(A.sys[q].mg.lev[k + 1], lvl(q, k).t, A.sys[q].mg.omega, I); });
         if (!grid_sync(bar, target, s_ok)) return false;
     }
     {
@@ -458,20 +620,13 @@ __device__ bool mg_apply_set(const MSetArgT<CAP> &A, const KState *sst, const in
         auto part = [&](int q) { return on(q) && k < A.sys[q].mg.nlev; };
         auto rows = [&](int q) { return k == 0 ? A.sys[q].n : A.sys[q].mg.lev[k].n; };
         mg_rows(A, part, rows, [&](int q, int r) {
-            const MGView L = lvl(q, k);
             const MGLevel &C = A.sys[q].mg.lev[k + 1];
-            L.x[r] += C.x[C.agg[r]];
+            mg_up(lvl(q, k), C.agg, C.x, r);
         });
         if (!grid_sync(bar, target, s_ok)) return false;
         mg_rows(A, part, rows, [&](int q, int r) {
-            const MGView L = lvl(q, k);
-            L.t[r] = L.b[r] - mg_spmv(L, r, L.x);
-        });
-        if (!grid_sync(bar, target, s_ok)) return false;
-        mg_rows(A, part, rows, [&](int q, int r) {
-            const MGView L = lvl(q, k);
-            const float w = A.sys[q].mg.omega;
-            L.x[r] += w * L.invdiag[r] * L.t[r];
+            const MGLevel &C = A.sys[q].mg.lev[k + 1];
+            mg_finish(lvl(q, k), C.agg, C.x, A.sys[q].mg.omega, r);
         });
         if (!grid_sync(bar, target, s_ok)) return false;
     }
@@ -481,10 +636,11 @@ __device__ bool mg_apply_set(const MSetArgT<CAP> &A, const KState *sst, const in
 // y = M^-1 p (which = 0) or z = M^-1 s (1) for the multilevel systems of a set
 template <int CAP>
 __device__ __forceinline__ bool mg_precondition(const MSetArgT<CAP> &A, const KState *sst, const int *sdc,
-                                                int which, GridBar *bar, unsigned int &target, int *s_ok) {
+                                                int which, TailLevels &T, GridBar *bar, unsigned int &target,
+                                                int *s_ok) {
     if constexpr (CAP <= KMAX) {  // one solver instance's set: a single system
         const MSys &S = A.sys[0];
-        return which == 0 ? mg_apply(S, S.p, S.y, bar, target, s_ok) : mg_apply(S, S.s, S.z, bar, target, s_ok);
+        return which == 0 ? mg_apply(S, S.p, S.y, T, bar, target, s_ok) : mg_apply(S, S.s, S.z, T, bar, target, s_ok);
     } else {
         return mg_apply_set(A, sst, sdc, which, bar, target, s_ok);
     }
@@ -557,6 +713,10 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
         sst[threadIdx.x] = *A.sys[threadIdx.x].st;
         sdc[threadIdx.x] = A.sys[threadIdx.x].dc->done;
     }
+    extern __shared__ float tail_mem[];  // the tail of a single system's hierarchy (mg_tail_words)
+    __shared__ TailLevels s_tail;
+    if constexpr (!FUSED && CAP <= KMAX)
+        if (A.sys[0].mg.nlev > 0 && A.sys[0].mg.tail <= A.sys[0].mg.nlev) mg_tail_load(A.sys[0].mg, tail_mem, s_tail);
     unsigned int target = grid_sync_start(bar);
     __syncthreads();
     int it = 0;
@@ -715,7 +875,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
             }
             if (!grid_sync(bar, target, &s_ok)) break;
             // multilevel preconditioning: y = M^-1 p (replaces the Jacobi y)
-            if (mg_on && !mg_precondition(A, sst, sdc, 0, bar, target, &s_ok)) break;
+            if (mg_on && !mg_precondition(A, sst, sdc, 0, s_tail, bar, target, &s_ok)) break;
             // v = A y, <r0, v>
             for (int u = cbegin; u < total_units; u += gstride) {
                 const int si = msys_of_chunk(A, u / MSUB);
@@ -758,7 +918,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
                 }
             }
             if (!grid_sync(bar, target, &s_ok)) break;
-            if (mg_on && !mg_precondition(A, sst, sdc, 1, bar, target, &s_ok)) break;
+            if (mg_on && !mg_precondition(A, sst, sdc, 1, s_tail, bar, target, &s_ok)) break;
             // t = A z, <t, t>, <t, s>
             for (int u = cbegin; u < total_units; u += gstride) {
                 const int si = msys_of_chunk(A, u / MSUB);
@@ -984,6 +1144,9 @@ constexpr long kFusedRows = 1L << 19;
 // (the V-cycle runs in the five-phase loop)
 bool m32_fused(long rows, bool mg) { return rows <= kFusedRows && !mg; }
 
+// at most 21 words a row and one more a level (mg_tail_words)
+constexpr size_t kTailSmemMax = ((size_t)21 * MG_TAIL_ROWS + MG_MAX) * 4;
+
 template <int CAP>
 cudaError_t launch_m32_loop(const MSetArgT<CAP> &A, GridBar *bar, int max_iters, cudaStream_t st, int variant,
                             int share) {
@@ -997,9 +1160,14 @@ cudaError_t launch_m32_loop(const MSetArgT<CAP> &A, GridBar *bar, int max_iters,
     const bool fused = variant < 0 ? m32_fused(rows, mg) : (variant == 1 && !mg);
     const void *fn = fused ? (const void *)k_m32_loop<true, CAP> : (const void *)k_m32_loop<false, CAP>;
     static std::atomic<int> occ_cache[2];
+    const size_t tail_max = CAP <= KMAX && !fused ? kTailSmemMax : 0;
+    const size_t smem = tail_max && A.sys[0].mg.nlev > 0 ? mg_tail_words(A.sys[0].mg) * 4 : 0;
     int occ = occ_cache[fused].load();
     if (occ == 0) {
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, LOOP_THREADS, 0);
+        cudaError_t e = cudaSuccess;
+        if (tail_max) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tail_max);
+        if (e != cudaSuccess) return e;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, LOOP_THREADS, tail_max);
         if (e != cudaSuccess) return e;
         if (occ <= 0) return cudaErrorLaunchOutOfResources;
         occ_cache[fused] = occ;
@@ -1013,7 +1181,7 @@ cudaError_t launch_m32_loop(const MSetArgT<CAP> &A, GridBar *bar, int max_iters,
     MSetArgT<CAP> a = A;
     void *args[] = {&a, &bar, &max_iters};
     count_launches(1);
-    return cudaLaunchCooperativeKernel(fn, grid, LOOP_THREADS, args, 0, st);
+    return cudaLaunchCooperativeKernel(fn, grid, LOOP_THREADS, args, smem, st);
 }
 
 template <int CAP>

@@ -34,15 +34,28 @@ struct MGLevel {
     const int *agg;       // [rows of level k-1]: the row of this level each belongs to
     const int *mstart;    // [n + 1]: offsets into members
     const int *members;   // rows of level k-1 of each row, ascending
-    float *x, *b, *t;     // V-cycle vectors [npad]
+    float *x, *b, *t, *t2;  // V-cycle vectors [npad]
 };
 struct MGSet {
     int nlev;             // coarse levels (0: Jacobi preconditioning)
     int sweeps;           // Jacobi sweeps on the coarsest level
     float omega;          // damping of the Jacobi smoother
-    int pad_;
+    int tail;             // levels tail..nlev run in every block's shared memory (nlev + 1: none do)
     MGLevel lev[MG_MAX + 1];  // lev[1..nlev]; lev[0] unused (the system itself)
 };
+// The tail takes the levels from the coarsest up while they have at most this
+// many rows together: 85 bytes a row, so the largest tail leaves 90 KB of the
+// SM's 256 KB for the L1 that the fine levels' gathers need.
+constexpr int MG_TAIL_ROWS = 1792;
+// shared memory of the tail (32-bit words), the layout of TailLevels
+inline size_t mg_tail_words(const MGSet &mg) {
+    size_t w = 0;
+    for (int k = mg.tail; k <= mg.nlev; ++k) {
+        w += (size_t)18 * mg.lev[k].n;
+        if (k > mg.tail) w += (size_t)mg.lev[k].n + 1 + 2 * (size_t)mg.lev[k - 1].n;
+    }
+    return w;
+}
 
 struct MSys {
     int n, npad, nchunks, chunk_begin;

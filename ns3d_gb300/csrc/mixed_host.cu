@@ -88,7 +88,16 @@ void MixedSetT<CAP>::configure(const std::vector<SolveItem> &items, cudaStream_t
                 G.x = H.x.p;
                 G.b = H.b.p;
                 G.t = H.t.p;
+                G.t2 = H.t2.p;
             }
+            // the tail: the levels that fit in a block's shared memory (a
+            // merged set has no shared memory of its own per system)
+            m.mg.tail = m.mg.nlev + 1;
+            if (CAP <= KMAX)
+                for (int rows = 0; m.mg.tail > 1; --m.mg.tail) {
+                    rows += m.mg.lev[m.mg.tail - 1].n;
+                    if (rows > MG_TAIL_ROWS) break;
+                }
         }
     }
     std::memset(&set_, 0, sizeof set_);
