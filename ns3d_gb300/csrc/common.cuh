@@ -36,9 +36,7 @@ __device__ __forceinline__ double warp_tree_sum(double v) {
 }
 
 // Tree sum over LANES threads (lane = this thread's index among them) that
-// synchronize with `sync`: the block's __syncthreads when a block has exactly
-// LANES threads, a named barrier when a larger block holds several groups of
-// LANES threads.  Returns the tree sum in lane 0 (other lanes get an
+// synchronize with `sync`, the named barrier of their group.  Returns the tree sum in lane 0 (other lanes get an
 // unspecified value).  `sm` needs LANES doubles.
 template <class T, class Sync>
 __device__ __forceinline__ T lanes_tree_sum(T v, int lane, T *sm, Sync sync) {
@@ -88,9 +86,6 @@ __device__ __forceinline__ void lanes_tree_sum2(T a, T b, int lane, T *sm, T &ra
     sync();
 }
 
-struct BlockSync {
-    __device__ __forceinline__ void operator()() const { __syncthreads(); }
-};
 // named barrier `id` (1..15) over the LANES threads of one group
 struct GroupSync {
     int id;
@@ -99,34 +94,50 @@ struct GroupSync {
     }
 };
 
-// Block of exactly LANES threads; the tree sum in thread 0.
-__device__ __forceinline__ double block_tree_sum(double v, double *sm) {
-    return lanes_tree_sum<double>(v, threadIdx.x, sm, BlockSync());
-}
-__device__ __forceinline__ void block_tree_sum2(double a, double b, double *sm, double &ra, double &rb) {
-    lanes_tree_sum2<double>(a, b, threadIdx.x, sm, ra, rb, BlockSync());
-}
-
 __device__ __forceinline__ double dmaxv(double a, double b) { return (b > a) ? b : a; }
 __device__ __forceinline__ double dminv(double a, double b) { return (b < a) ? b : a; }
 
-// maxima / minima over the block (exact in any order); result in every thread
-template <bool MAX>
-__device__ __forceinline__ double block_extreme(double v, double *sm) {
-    const int t = threadIdx.x;
+// maximum / minimum over the LANES threads of a group (exact in any order);
+// valid in every thread.  sm: LANES / 32 doubles.
+template <bool MAX, class Sync>
+__device__ __forceinline__ double lanes_extreme(double v, int lane, double *sm, Sync sync) {
     for (int off = 16; off >= 1; off >>= 1) {
-        double o = __shfl_down_sync(0xffffffffu, v, off);
+        const double o = __shfl_down_sync(0xffffffffu, v, off);
         v = MAX ? dmaxv(v, o) : dminv(v, o);
     }
-    if ((t & 31) == 0) sm[t >> 5] = v;
-    __syncthreads();
+    if ((lane & 31) == 0) sm[lane >> 5] = v;
+    sync();
     double r = sm[0];
     for (int w = 1; w < LANES / 32; ++w) r = MAX ? dmaxv(r, sm[w]) : dminv(r, sm[w]);
-    __syncthreads();
+    sync();
     return r;
 }
-__device__ __forceinline__ double block_tree_max(double v, double *sm) { return block_extreme<true>(v, sm); }
-__device__ __forceinline__ double block_tree_min(double v, double *sm) { return block_extreme<false>(v, sm); }
+
+// ---- chunk kernels ----------------------------------------------------------
+// The kernels that compute per-row operands and reduce them run one chunk per
+// block of LANES * G threads: thread (g, lane) computes rows
+// lane + LANES m, m in [g RPL / G, (g + 1) RPL / G), the operands pass through
+// shared memory, and group j accumulates sum j lane by lane in the fixed
+// order.  A row costs several dependent loads, so a small system is bound by
+// the latency of the rows a thread walks in turn: with one group these
+// kernels took 19 us (k_kr_init), 38 (k_dc_resid), 40 (k_dc_step) and 61-72 us
+// (k_divergence) whatever the size, with eight 11, 17, 21 and 24 us.  Above
+// WIDE_CHUNKS_PER_SM chunks per SM the other blocks cover that latency and a
+// wide block only waits for its own reduction (10.5 M rows: k_dc_resid 426 us
+// with eight groups, 287 with two).
+constexpr int WIDE_CHUNKS_PER_SM = 2;
+constexpr int WIDE_G = 8, NARROW_G = 2;
+inline bool wide_chunks(int nchunks, int sms) { return nchunks <= WIDE_CHUNKS_PER_SM * sms; }
+
+// a lane's accumulation of sum a[q] b[q] over its rows of a chunk, from the
+// operands in shared memory (rows: rows of the chunk below the system's n)
+__device__ __forceinline__ double lane_dot(const double *a, const double *b, int lane, int rows) {
+    double acc = 0.0;
+#pragma unroll
+    for (int m = 0; m < RPL; ++m)
+        if (lane + m * LANES < rows) acc = __fma_rn(a[lane + m * LANES], b[lane + m * LANES], acc);
+    return acc;
+}
 
 // Final combination of `n` chunk partials (strided by `stride` doubles):
 // lane l sums partials l, l+LANES, ... in order, then the halving tree.
@@ -173,13 +184,6 @@ __device__ __forceinline__ void lanes_final_sum2(const double *part, int n, int 
             }
     }
     lanes_tree_sum2<double>(a, b, lane, sm, ra, rb, sync);
-}
-
-__device__ __forceinline__ double final_partials_sum(const double *part, int n, int stride, double *sm) {
-    return lanes_final_sum(part, n, stride, threadIdx.x, sm, BlockSync());
-}
-__device__ __forceinline__ void final_partials_sum2(const double *part, int n, double *sm, double &ra, double &rb) {
-    lanes_final_sum2(part, n, threadIdx.x, sm, ra, rb, BlockSync());
 }
 
 inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }

@@ -169,37 +169,46 @@ namespace ns3d {
         const int lc = c - S.chunk_begin;                                      \
         const int r0 = lc * CH + threadIdx.x;
 
-// ---- init: r = b - A x, r0 = r, |r|^2, |b|^2 ---------------------------------
-template <int CAP>
-__global__ void __launch_bounds__(LANES) k_kr_init(const __grid_constant__ KSetArgT<CAP> A) {
-    __shared__ double sm[LANES];
-    __shared__ int sh[2];
-    NS3D_CHUNK_LOOP
-        double arr = 0.0, abb = 0.0;
-        {
-            const Row4 ax = spmv4(S, r0, S.x);
-            const Row4 b = ld4(S.b + r0);
-            Row4 r;
+// r = b - A x into S.r and S.r0 for a chunk's rows, |r|^2 and (BB) |b|^2 of the
+// chunk into its partials.  sm: 2 CH operands, 8 for the trees (also of the
+// final sum, during which the other groups may already write the next chunk's
+// operands).
+template <int G, bool BB>
+__device__ __forceinline__ void chunk_residual(const KSys &S, int lc, double *sm) {
+    const int gi = threadIdx.x / LANES, lane = threadIdx.x % LANES;
+    double *const s_r = sm, *const s_b = sm + CH;
 #pragma unroll
-            for (int m = 0; m < RPL; ++m) {
-                r.v[m] = b.v[m] - ax.v[m];
-                if (r0 + m * LANES < S.n) {
-                    arr = __fma_rn(r.v[m], r.v[m], arr);
-                    abb = __fma_rn(b.v[m], b.v[m], abb);
-                }
-            }
-            st4(S.r + r0, r);
-            st4(S.r0 + r0, r);
-        }
-        double trr, tbb;
-        block_tree_sum2(arr, abb, sm, trr, tbb);
-        if (threadIdx.x == 0) {
-            S.part[2 * (size_t)lc + 0] = trr;
-            S.part[2 * (size_t)lc + 1] = tbb;
-        }
-        if (arrive_last(S.st, (unsigned)S.nchunks, sh)) {
+    for (int i = 0; i < RPL / G; ++i) {
+        const int q = lane + (gi * (RPL / G) + i) * LANES, row = lc * CH + q;
+        const double b = S.b[row];
+        const double r = b - spmv_row(S, row, S.x);
+        s_r[q] = r;
+        if (BB) s_b[q] = b;
+        S.r[row] = r;
+        S.r0[row] = r;
+    }
+    __syncthreads();
+    // sum j by group j (by group 0 in turn when it is the only one)
+    for (int j = gi; j < (BB ? 2 : 1); j += G) {
+        const double *v = j == 0 ? s_r : s_b;
+        const double t = lanes_tree_sum<double>(lane_dot(v, v, lane, min(CH, S.n - lc * CH)), lane, sm + 2 * CH + 4 * j,
+                                                GroupSync{gi + 1});
+        if (lane == 0) S.part[2 * (size_t)lc + j] = t;
+    }
+}
+
+// ---- init: r = b - A x, r0 = r, |r|^2, |b|^2 ---------------------------------
+template <int CAP, int G>
+__global__ void __launch_bounds__(LANES *G, 8 / G) k_kr_init(const __grid_constant__ KSetArgT<CAP> A) {
+    __shared__ double sm[2 * CH + 8];
+    __shared__ int sh[2];
+    for (int c = blockIdx.x; c < A.total_chunks; c += gridDim.x) {
+        const KSys &S = A.sys[sys_of_chunk(A, c)];
+        const int lc = c - S.chunk_begin;
+        chunk_residual<G, true>(S, lc, sm);
+        if (arrive_last(S.st, (unsigned)S.nchunks, sh) && threadIdx.x < LANES) {
             double rr, bb;
-            final_partials_sum2(S.part, S.nchunks, sm, rr, bb);
+            lanes_final_sum2(S.part, S.nchunks, threadIdx.x, sm + 2 * CH, rr, bb, GroupSync{1});
             if (threadIdx.x == 0) {
                 KState *st = S.st;
                 st->counter = 0;
@@ -540,27 +549,17 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
 }
 
 // restart of paused systems: r = b - A x, r0 = r, rho = |r0|^2
-template <int CAP>
-__global__ void __launch_bounds__(LANES) k_kr_restart(const __grid_constant__ KSetArgT<CAP> A) {
-    __shared__ double sm[LANES];
+template <int CAP, int G>
+__global__ void __launch_bounds__(LANES *G, 8 / G) k_kr_restart(const __grid_constant__ KSetArgT<CAP> A) {
+    __shared__ double sm[2 * CH + 8];
     __shared__ int sh[2];
-    NS3D_CHUNK_LOOP
+    for (int c = blockIdx.x; c < A.total_chunks; c += gridDim.x) {
+        const KSys &S = A.sys[sys_of_chunk(A, c)];
         if (!(__ldcg(&S.st->paused) != 0 && __ldcg(&S.st->done) == 0)) continue;
-        const Row4 ax = spmv4(S, r0, S.x);
-        const Row4 b = ld4(S.b + r0);
-        Row4 r;
-        double arr = 0.0;
-#pragma unroll
-        for (int m = 0; m < RPL; ++m) {
-            r.v[m] = b.v[m] - ax.v[m];
-            if (r0 + m * LANES < S.n) arr = __fma_rn(r.v[m], r.v[m], arr);
-        }
-        st4(S.r + r0, r);
-        st4(S.r0 + r0, r);
-        const double trr = block_tree_sum(arr, sm);
-        if (threadIdx.x == 0) S.part[2 * (size_t)lc] = trr;
-        if (arrive_last(S.st, (unsigned)S.nchunks, sh)) {
-            const double rr = final_partials_sum(S.part, S.nchunks, 2, sm);
+        const int lc = c - S.chunk_begin;
+        chunk_residual<G, false>(S, lc, sm);
+        if (arrive_last(S.st, (unsigned)S.nchunks, sh) && threadIdx.x < LANES) {
+            const double rr = lanes_final_sum(S.part, S.nchunks, 2, threadIdx.x, sm + 2 * CH, GroupSync{1});
             if (threadIdx.x == 0) {
                 KState *st = S.st;
                 st->counter = 0;
@@ -636,7 +635,10 @@ template <int CAP>
 void launch_krylov_init(const KSetArgT<CAP> &A, cudaStream_t st) {
     if (A.total_chunks <= 0) return;
     count_launches(2);
-    k_kr_init<CAP><<<kr_grid(A.total_chunks), LANES, 0, st>>>(A);
+    if (wide_chunks(A.total_chunks, device_sm_count()))
+        k_kr_init<CAP, WIDE_G><<<kr_grid(A.total_chunks), LANES * WIDE_G, 0, st>>>(A);
+    else
+        k_kr_init<CAP, NARROW_G><<<kr_grid(A.total_chunks), LANES * NARROW_G, 0, st>>>(A);
     k_kr_init2<CAP><<<kr_grid(A.total_chunks), LANES, 0, st>>>(A, A.total_chunks <= device_sm_count());
 }
 
@@ -717,7 +719,10 @@ template <int CAP>
 void launch_krylov_restart(const KSetArgT<CAP> &A, cudaStream_t st) {
     if (A.total_chunks <= 0) return;
     count_launches(1);
-    k_kr_restart<CAP><<<kr_grid(A.total_chunks), LANES, 0, st>>>(A);
+    if (wide_chunks(A.total_chunks, device_sm_count()))
+        k_kr_restart<CAP, WIDE_G><<<kr_grid(A.total_chunks), LANES * WIDE_G, 0, st>>>(A);
+    else
+        k_kr_restart<CAP, NARROW_G><<<kr_grid(A.total_chunks), LANES * NARROW_G, 0, st>>>(A);
 }
 
 template void launch_krylov_init<KMAX>(const KSetArg &, cudaStream_t);

@@ -26,21 +26,6 @@
 
 namespace ns3d {
 
-struct RowF4 {  // a thread's RPL rows
-    float v[RPL];
-};
-
-__device__ __forceinline__ RowF4 ldf4(const float *p) {
-    RowF4 r;
-#pragma unroll
-    for (int m = 0; m < RPL; ++m) r.v[m] = p[m * LANES];
-    return r;
-}
-__device__ __forceinline__ void stf4(float *p, const RowF4 &r) {
-#pragma unroll
-    for (int m = 0; m < RPL; ++m) p[m * LANES] = r.v[m];
-}
-
 // FP32 row product.  A missing entry has a zero coefficient; its gather
 // reads the row's own (finite) element, so all seven products are issued
 // without branches (FP32 issue is plentiful on GB300).
@@ -79,12 +64,28 @@ __device__ __forceinline__ float spmv_f32_fn(const MSys &S, int row, F xf) {
     return acc;
 }
 
-__device__ __forceinline__ double spmv_f64_row(const MSys &S, int row, const double *__restrict__ x) {
+// One row of A64 x, x given by a function of the column: every operand is
+// loaded before the chain of row_ordered (a missing neighbour takes the row's
+// own, unused), so the loads do not wait for each other.
+template <class F>
+__device__ __forceinline__ double spmv_f64_fn(const MSys &S, int row, F xf) {
     const size_t np = (size_t)S.npad;
     const int *nb = S.nbr + row;
     const double *cf = S.coef64 + row;
-    return row_ordered(row, nb[0 * np], nb[1 * np], nb[2 * np], nb[3 * np], nb[4 * np], nb[5 * np],
-                       [&](double acc, int s, int col) { return __fma_rn(cf[(size_t)s * np], x[col], acc); });
+    int col[6];
+    double c[7], x[7];
+#pragma unroll
+    for (int d = 0; d < 6; ++d) col[d] = ro(nb + d * np);
+#pragma unroll
+    for (int d = 0; d < 7; ++d) c[d] = ro(cf + d * np);
+    x[0] = xf(row);
+#pragma unroll
+    for (int d = 0; d < 6; ++d) x[d + 1] = xf(col[d] >= 0 ? col[d] : row);
+    return row_ordered(row, col[0], col[1], col[2], col[3], col[4], col[5],
+                       [&](double acc, int s, int) { return __fma_rn(c[s], x[s], acc); });
+}
+__device__ __forceinline__ double spmv_f64_row(const MSys &S, int row, const double *x) {
+    return spmv_f64_fn(S, row, [&](int c) { return x[c]; });
 }
 
 // system owning global chunk c (systems in chunk order, first begins at 0;
@@ -122,8 +123,7 @@ __device__ __forceinline__ bool m_active(const MSys &S, bool inner) {
     for (int c = blockIdx.x; c < A.total_chunks; c += gridDim.x) {           \
         const MSys &S = A.sys[msys_of_chunk(A, c)];                          \
         if (!m_active(S, INNER)) continue;                                    \
-        const int lc = c - S.chunk_begin;                                     \
-        const int r0 = lc * CH + threadIdx.x;
+        const int lc = c - S.chunk_begin;
 
 __device__ __forceinline__ bool m_arrive_last(unsigned int *counter, unsigned int total, int *sh) {
     __syncthreads();
@@ -141,32 +141,31 @@ __device__ __forceinline__ bool m_arrive_last(unsigned int *counter, unsigned in
 __device__ __forceinline__ bool finite(double x) { return isfinite(x); }
 
 // ---- FP64 residual and outer control -----------------------------------------
-template <int CAP>
-__global__ void __launch_bounds__(LANES) k_dc_resid(const __grid_constant__ MSetArgT<CAP> A, int first) {
-    __shared__ double sm[LANES];
+template <int CAP, int G>
+__global__ void __launch_bounds__(LANES *G, 8 / G) k_dc_resid(const __grid_constant__ MSetArgT<CAP> A, int first) {
+    __shared__ double sm[2 * CH + 8];  // r, b; the trees
     __shared__ int sh[4];
+    const int gi = threadIdx.x / LANES, lane = threadIdx.x % LANES;
     NS3D_MCHUNK_LOOP(false)
-        double arr = 0.0, abb = 0.0;
 #pragma unroll
-        for (int m = 0; m < RPL; ++m) {
-            const int row = r0 + m * LANES;
+        for (int i = 0; i < RPL / G; ++i) {
+            const int q = lane + (gi * (RPL / G) + i) * LANES, row = lc * CH + q;
             const double b = S.b64[row];
             const double r = b - spmv_f64_row(S, row, S.x64);
             S.r64[row] = r;
-            if (row < S.n) {
-                arr = __fma_rn(r, r, arr);
-                abb = __fma_rn(b, b, abb);
-            }
+            sm[q] = r;
+            sm[CH + q] = b;
         }
-        double trr, tbb;
-        block_tree_sum2(arr, abb, sm, trr, tbb);
-        if (threadIdx.x == 0) {
-            S.part[2 * (size_t)lc + 0] = trr;
-            S.part[2 * (size_t)lc + 1] = tbb;
+        __syncthreads();
+        for (int j = gi; j < 2; j += G) {
+            const double *v = sm + j * CH;
+            const double t = lanes_tree_sum<double>(lane_dot(v, v, lane, min(CH, S.n - lc * CH)), lane,
+                                                    sm + 2 * CH + 4 * j, GroupSync{gi + 1});
+            if (lane == 0) S.part[2 * (size_t)lc + j] = t;
         }
-        if (m_arrive_last(&S.dc->counter, (unsigned)S.nchunks, sh)) {
+        if (m_arrive_last(&S.dc->counter, (unsigned)S.nchunks, sh) && threadIdx.x < LANES) {
             double rr, bb;
-            final_partials_sum2(S.part, S.nchunks, sm, rr, bb);
+            lanes_final_sum2(S.part, S.nchunks, lane, sm + 2 * CH, rr, bb, GroupSync{1});
             if (threadIdx.x == 0) {
                 DCState *dc = S.dc;
                 KState *st = S.st;
@@ -220,32 +219,40 @@ __global__ void k_dc_zero(const __grid_constant__ MSetArgT<CAP> A) {
 }
 
 // ---- FP32 inner solve -------------------------------------------------------
-template <int CAP>
-__global__ void __launch_bounds__(LANES) k_m32_init(const __grid_constant__ MSetArgT<CAP> A) {
-    __shared__ double sm[LANES];
+template <int CAP, int G>
+__global__ void __launch_bounds__(LANES *G, 8 / G) k_m32_init(const __grid_constant__ MSetArgT<CAP> A) {
+    __shared__ float s_f[CH];
+    __shared__ double sm[8];
     __shared__ int sh[4];
+    const int gi = threadIdx.x / LANES, lane = threadIdx.x % LANES;
     NS3D_MCHUNK_LOOP(true)
         const double scale = __ldcg(&S.dc->scale);
-        float acc = 0.0f;
-        RowF4 f;
-        RowF4 zero;
+        double r[RPL / G];
 #pragma unroll
-        for (int m = 0; m < RPL; ++m) zero.v[m] = 0.0f;
+        for (int i = 0; i < RPL / G; ++i) r[i] = S.r64[lc * CH + lane + (gi * (RPL / G) + i) * LANES];
 #pragma unroll
-        for (int m = 0; m < RPL; ++m) {
-            const int row = r0 + m * LANES;
-            f.v[m] = (float)(S.r64[row] * scale);
-            if (row < S.n) acc = __fmaf_rn(f.v[m], f.v[m], acc);
+        for (int i = 0; i < RPL / G; ++i) {
+            const int q = lane + (gi * (RPL / G) + i) * LANES, row = lc * CH + q;
+            const float f = (float)(r[i] * scale);
+            s_f[q] = f;
+            S.r[row] = f;
+            S.r0[row] = f;
+            S.x[row] = 0.0f;
+            S.p[row] = 0.0f;
+            S.v[row] = 0.0f;
         }
-        stf4(S.r + r0, f);
-        stf4(S.r0 + r0, f);
-        stf4(S.x + r0, zero);
-        stf4(S.p + r0, zero);
-        stf4(S.v + r0, zero);
-        const double t = block_tree_sum((double)acc, sm);
-        if (threadIdx.x == 0) S.part[2 * (size_t)lc] = t;
-        if (m_arrive_last(&S.st->counter, (unsigned)S.nchunks, sh)) {
-            const double bb = final_partials_sum(S.part, S.nchunks, 2, sm);
+        __syncthreads();
+        if (gi == 0) {
+            float acc = 0.0f;
+            const int rows = min(CH, S.n - lc * CH);
+#pragma unroll
+            for (int m = 0; m < RPL; ++m)
+                if (lane + m * LANES < rows) acc = __fmaf_rn(s_f[lane + m * LANES], s_f[lane + m * LANES], acc);
+            const double t = lanes_tree_sum<double>((double)acc, lane, sm, GroupSync{1});
+            if (lane == 0) S.part[2 * (size_t)lc] = t;
+        }
+        if (m_arrive_last(&S.st->counter, (unsigned)S.nchunks, sh) && threadIdx.x < LANES) {
+            const double bb = lanes_final_sum(S.part, S.nchunks, 2, lane, sm, GroupSync{1});
             if (threadIdx.x == 0) {
                 KState *st = S.st;
                 st->counter = 0;
@@ -1014,6 +1021,22 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
             break;
         }
     }
+    // the correction in FP64, for k_dc_step and k_dc_update: one conversion and
+    // product per row here instead of one per operand there
+    __shared__ double s_inv[CAP];
+    if (threadIdx.x < A.nsys) s_inv[threadIdx.x] = 1.0 / A.sys[threadIdx.x].dc->scale;
+    __syncthreads();
+    for (int u = cbegin; u < total_units; u += gstride) {
+        const int si = msys_of_chunk(A, u / MSUB);
+        if (sdc[si] || sst[si].info != 0) continue;
+        const MSys &S = A.sys[si];
+        const int r0 = (u - S.chunk_begin * MSUB) * MUNIT + lane;
+        float x[MRPL];
+#pragma unroll
+        for (int m = 0; m < MRPL; ++m) x[m] = S.x[r0 + m * LANES];
+#pragma unroll
+        for (int m = 0; m < MRPL; ++m) S.d64[r0 + m * LANES] = (double)x[m] * s_inv[si];
+    }
     if (blockIdx.x == 0 && threadIdx.x < A.nsys) {
         KState k = sst[threadIdx.x];
         k.counter = 0;
@@ -1021,42 +1044,35 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
     }
 }
 
-// Step length of the round's correction delta = double(d) / scale:
+// Step length of the round's correction delta = double(d) / scale (S.d64):
 // theta = <r64, A64 delta> / <A64 delta, A64 delta> minimizes the FP64
 // residual along delta, so a correction from an inaccurate FP32 solve can
 // shrink the residual less but never grow it.  The last block to finish
 // sets dc->theta.
-template <int CAP>
-__global__ void __launch_bounds__(LANES) k_dc_step(const __grid_constant__ MSetArgT<CAP> A) {
-    __shared__ double sm[LANES];
+template <int CAP, int G>
+__global__ void __launch_bounds__(LANES *G, 8 / G) k_dc_step(const __grid_constant__ MSetArgT<CAP> A) {
+    __shared__ double s_q[CH], s_r[CH], sm[8];
     __shared__ int sh[4];
+    const int gi = threadIdx.x / LANES, lane = threadIdx.x % LANES;
     for (int c = blockIdx.x; c < A.total_chunks; c += gridDim.x) {
         const MSys &S = A.sys[msys_of_chunk(A, c)];
         if (!(__ldcg(&S.dc->done) == 0 && __ldcg(&S.st->info) == 0)) continue;
-        const double inv = 1.0 / __ldcg(&S.dc->scale);
         const int lc = c - S.chunk_begin;
-        const int r0 = lc * CH + threadIdx.x;
-        const size_t np = (size_t)S.npad;
-        double arq = 0.0, aqq = 0.0;
-        for (int m = 0; m < RPL; ++m) {
-            const int row = r0 + m * LANES;
-            const int *nb = S.nbr + row;
-            const double *cf = S.coef64 + row;
-            const double q = row_ordered(row, nb[0 * np], nb[1 * np], nb[2 * np], nb[3 * np], nb[4 * np], nb[5 * np],
-                                         [&](double acc, int sl, int col) {
-                                             return __fma_rn(cf[(size_t)sl * np], (double)S.x[col] * inv, acc);
-                                         });
-            if (row < S.n) {
-                arq = __fma_rn(S.r64[row], q, arq);
-                aqq = __fma_rn(q, q, aqq);
-            }
+#pragma unroll
+        for (int i = 0; i < RPL / G; ++i) {
+            const int q = lane + (gi * (RPL / G) + i) * LANES, row = lc * CH + q;
+            s_q[q] = spmv_f64_row(S, row, S.d64);
+            s_r[q] = S.r64[row];
         }
-        double trq, tqq;
-        block_tree_sum2(arq, aqq, sm, trq, tqq);
-        if (threadIdx.x == 0) reinterpret_cast<double2 *>(S.part)[lc] = make_double2(trq, tqq);
-        if (m_arrive_last(&S.dc->counter, (unsigned)S.nchunks, sh)) {
+        __syncthreads();
+        for (int j = gi; j < 2; j += G) {
+            const double t = lanes_tree_sum<double>(lane_dot(j == 0 ? s_r : s_q, s_q, lane, min(CH, S.n - lc * CH)), lane,
+                                                    sm + 4 * j, GroupSync{gi + 1});
+            if (lane == 0) S.part[2 * (size_t)lc + j] = t;
+        }
+        if (m_arrive_last(&S.dc->counter, (unsigned)S.nchunks, sh) && threadIdx.x < LANES) {
             double frq, fqq;
-            final_partials_sum2(S.part, S.nchunks, sm, frq, fqq);
+            lanes_final_sum2(S.part, S.nchunks, lane, sm, frq, fqq, GroupSync{1});
             if (threadIdx.x == 0) {
                 S.dc->counter = 0;
                 const double th = (fqq > 0.0) ? frq / fqq : 0.0;
@@ -1071,14 +1087,16 @@ __global__ void k_dc_update(const __grid_constant__ MSetArgT<CAP> A) {
     for (int c = blockIdx.x; c < A.total_chunks; c += gridDim.x) {
         const MSys &S = A.sys[msys_of_chunk(A, c)];
         if (!(__ldcg(&S.dc->done) == 0 && __ldcg(&S.st->info) == 0)) continue;
-        const double inv = 1.0 / __ldcg(&S.dc->scale);
         const double theta = __ldcg(&S.dc->theta);
         const int r0 = (c - S.chunk_begin) * CH + threadIdx.x;
+        double d[RPL], x[RPL];
 #pragma unroll
-        for (int m = 0; m < RPL; ++m) {
-            const int row = r0 + m * LANES;
-            S.x64[row] = __fma_rn(theta, (double)S.x[row] * inv, S.x64[row]);
+        for (int m = 0; m < RPL; ++m) {  // all loads before the first store
+            d[m] = S.d64[r0 + m * LANES];
+            x[m] = S.x64[r0 + m * LANES];
         }
+#pragma unroll
+        for (int m = 0; m < RPL; ++m) S.x64[r0 + m * LANES] = __fma_rn(theta, d[m], x[m]);
     }
 }
 
@@ -1095,13 +1113,18 @@ void launch_mg_galerkin(const MSys &S, cudaStream_t st) {
     }
 }
 
-// FP32 copy of a system's coefficients and inverse diagonal
-__global__ void k_to_f32(const double *__restrict__ coef, const double *__restrict__ invdiag, int npad,
-                         float *__restrict__ coef32, float *__restrict__ invdiag32) {
-    const long total = 8L * npad;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        if (i < 7L * npad) coef32[i] = (float)coef[i];
-        else invdiag32[i - 7L * npad] = (float)invdiag[i - 7L * npad];
+// FP32 copy of a system's coefficients and inverse diagonal (npad is a
+// multiple of 1024 and both arrays come from the pool, so pairs are aligned)
+__global__ void k_to_f32(const double2 *__restrict__ coef, const double2 *__restrict__ invdiag, int pairs,
+                         float2 *__restrict__ coef32, float2 *__restrict__ invdiag32) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pairs; i += gridDim.x * blockDim.x) {
+        double2 v[8];
+#pragma unroll
+        for (int s = 0; s < 7; ++s) v[s] = coef[(size_t)s * pairs + i];
+        v[7] = invdiag[i];
+#pragma unroll
+        for (int s = 0; s < 7; ++s) coef32[(size_t)s * pairs + i] = make_float2((float)v[s].x, (float)v[s].y);
+        invdiag32[i] = make_float2((float)v[7].x, (float)v[7].y);
     }
 }
 
@@ -1110,17 +1133,21 @@ static inline int m_grid(int total_chunks) { return std::max(1, std::min(total_c
 
 void launch_to_f32(const double *coef, const double *invdiag, int npad, float *coef32, float *invdiag32,
                    cudaStream_t st) {
-    const long total = 8L * npad;
+    const int pairs = npad / 2;
     count_launches(1);
-    k_to_f32<<<(int)std::min<long>((total + 255) / 256, 152L * 32), 256, 0, st>>>(coef, invdiag, npad, coef32,
-                                                                                invdiag32);
+    k_to_f32<<<std::min((pairs + 255) / 256, device_sm_count() * 32), 256, 0, st>>>(
+        reinterpret_cast<const double2 *>(coef), reinterpret_cast<const double2 *>(invdiag), pairs,
+        reinterpret_cast<float2 *>(coef32), reinterpret_cast<float2 *>(invdiag32));
 }
 
 template <int CAP>
 void launch_dc_resid(const MSetArgT<CAP> &A, int first, cudaStream_t st) {
     if (A.total_chunks <= 0) return;
     count_launches(1);
-    k_dc_resid<CAP><<<m_grid(A.total_chunks), LANES, 0, st>>>(A, first);
+    if (wide_chunks(A.total_chunks, device_sm_count()))
+        k_dc_resid<CAP, WIDE_G><<<m_grid(A.total_chunks), LANES * WIDE_G, 0, st>>>(A, first);
+    else
+        k_dc_resid<CAP, NARROW_G><<<m_grid(A.total_chunks), LANES * NARROW_G, 0, st>>>(A, first);
     if (first) {
         count_launches(1);
         k_dc_zero<CAP><<<m_grid(A.total_chunks), LANES, 0, st>>>(A);
@@ -1131,7 +1158,10 @@ template <int CAP>
 void launch_m32_init(const MSetArgT<CAP> &A, cudaStream_t st) {
     if (A.total_chunks <= 0) return;
     count_launches(1);
-    k_m32_init<CAP><<<m_grid(A.total_chunks), LANES, 0, st>>>(A);
+    if (wide_chunks(A.total_chunks, device_sm_count()))
+        k_m32_init<CAP, WIDE_G><<<m_grid(A.total_chunks), LANES * WIDE_G, 0, st>>>(A);
+    else
+        k_m32_init<CAP, 1><<<m_grid(A.total_chunks), LANES, 0, st>>>(A);  // bytes only: 74 us at 10.5 M rows, 101 with two groups
 }
 
 
@@ -1188,7 +1218,10 @@ template <int CAP>
 void launch_dc_update(const MSetArgT<CAP> &A, cudaStream_t st) {
     if (A.total_chunks <= 0) return;
     count_launches(2);
-    k_dc_step<CAP><<<m_grid(A.total_chunks), LANES, 0, st>>>(A);
+    if (wide_chunks(A.total_chunks, device_sm_count()))
+        k_dc_step<CAP, WIDE_G><<<m_grid(A.total_chunks), LANES * WIDE_G, 0, st>>>(A);
+    else
+        k_dc_step<CAP, NARROW_G><<<m_grid(A.total_chunks), LANES * NARROW_G, 0, st>>>(A);
     k_dc_update<CAP><<<m_grid(A.total_chunks), LANES, 0, st>>>(A);
 }
 

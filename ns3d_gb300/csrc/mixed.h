@@ -64,6 +64,7 @@ struct MSys {
     const double *b64;     // right-hand side
     double *x64;           // guess in, solution out
     double *r64;           // FP64 residual
+    double *d64;           // the round's correction double(x) / scale, written by the FP32 loop
     const float *coef32, *invdiag32;
     float *x, *r, *r0, *p, *v, *y, *s, *z, *t;  // FP32 inner vectors (x is the correction)
     float *p2, *v2;  // second buffers of p and v (the loop kernel alternates them)

@@ -57,6 +57,7 @@ void MixedSetT<CAP>::configure(const std::vector<SolveItem> &items, cudaStream_t
         m.b64 = items[i].b;
         m.x64 = items[i].x;
         m.r64 = S.r.p;
+        m.d64 = S.y.p;
         m.coef32 = S.coef32.p;
         m.invdiag32 = S.invdiag32.p;
         m.x = S.fx.p; m.r = S.fr.p; m.r0 = S.fr0.p; m.p = S.fp.p; m.v = S.fv.p;

@@ -649,73 +649,76 @@ __device__ __forceinline__ bool last_block_arrive(unsigned int *counter, unsigne
 }
 
 // ComputePermeability, src/NSBase.cxx:1886-1956: sums over the outlet u plane
-// (and, with a border, the inlet/outlet p planes), positions q = j*nz + k
-__global__ void k_permeability(Grid g, const double *__restrict__ u, const double *__restrict__ p, int border,
-                               double *__restrict__ part, DiagOut *out) {
-    __shared__ double sm[LANES];
+// (and, with a border, the inlet/outlet p planes), positions q = j*nz + k.
+// One plane position per thread, a position without a node adds +0 (which
+// changes no sum that starts at +0); group g accumulates sum g.
+__global__ void __launch_bounds__(CH) k_permeability(Grid g, const double *__restrict__ u, const double *__restrict__ p,
+                                                     int border, double *__restrict__ part, DiagOut *out) {
+    __shared__ double s_v[3][CH], sm[12];
     __shared__ bool last;
     const long plane = (long)g.ny * g.nz;
     const int nch = (int)((plane + CH - 1) / CH);
     const int iu = (border <= 0) ? g.nx : g.nx + 1 - border;
     const int io = g.nx - border, ii = border - 1;
+    const int gi = threadIdx.x / LANES, lane = threadIdx.x % LANES, sums = border > 0 ? 3 : 1;
     for (int c = blockIdx.x; c < nch; c += gridDim.x) {
-        double a = 0, so = 0, si = 0, co = 0, ci = 0;
-        for (int m = 0; m < RPL; ++m) {
-            long q = (long)c * CH + threadIdx.x + LANES * m;
-            if (q >= plane) break;
-            int r = g.umap[(long)iu * plane + q];
-            if (r > -1) a = a + u[r];
+        const long q = (long)c * CH + threadIdx.x;
+        int ro = -1, ri = -1;
+        if (q < plane) {
+            const int r = g.umap[(long)iu * plane + q];
             if (border > 0) {
-                int ro = g.pmap[(long)io * plane + q];
-                if (ro > -1) { so = so + p[ro]; co = co + 1.0; }
-                int ri = g.pmap[(long)ii * plane + q];
-                if (ri > -1) { si = si + p[ri]; ci = ci + 1.0; }
+                ro = g.pmap[(long)io * plane + q];
+                ri = g.pmap[(long)ii * plane + q];
             }
+            s_v[0][threadIdx.x] = r > -1 ? u[r] : 0.0;
+            s_v[1][threadIdx.x] = ro > -1 ? p[ro] : 0.0;
+            s_v[2][threadIdx.x] = ri > -1 ? p[ri] : 0.0;
         }
-        double ta = block_tree_sum(a, sm);
-        double tso = block_tree_sum(so, sm);
-        double tsi = block_tree_sum(si, sm);
-        double tco = block_tree_sum(co, sm);
-        double tci = block_tree_sum(ci, sm);
+        const int co = __syncthreads_count(ro > -1), ci = __syncthreads_count(ri > -1);
+        if (gi < sums) {
+            const int rows = (int)min((long)CH, plane - (long)c * CH);
+            double a = 0.0;
+#pragma unroll
+            for (int m = 0; m < RPL; ++m)
+                if (lane + m * LANES < rows) a = a + s_v[gi][lane + m * LANES];
+            const double t = lanes_tree_sum<double>(a, lane, sm + 4 * gi, GroupSync{gi + 1});
+            if (lane == 0) part[(size_t)c * 5 + gi] = t;
+        }
         if (threadIdx.x == 0) {
-            part[(size_t)c * 5 + 0] = ta;
-            part[(size_t)c * 5 + 1] = tso;
-            part[(size_t)c * 5 + 2] = tsi;
-            part[(size_t)c * 5 + 3] = tco;
-            part[(size_t)c * 5 + 4] = tci;
+            part[(size_t)c * 5 + 3] = (double)co;
+            part[(size_t)c * 5 + 4] = (double)ci;
         }
-        if (last_block_arrive(&out->counter[0], (unsigned)nch, &last)) {
-            double fa = final_partials_sum(part + 0, nch, 5, sm);
-            double fo = final_partials_sum(part + 1, nch, 5, sm);
-            double fi = final_partials_sum(part + 2, nch, 5, sm);
-            double fco = final_partials_sum(part + 3, nch, 5, sm);
-            double fci = final_partials_sum(part + 4, nch, 5, sm);
-            if (threadIdx.x == 0) {
-                out->v_sum = fa;
-                out->p_out_sum = fo;
-                out->p_in_sum = fi;
-                out->cnt_out = fco;
-                out->cnt_in = fci;
-                out->counter[0] = 0;
+        if (last_block_arrive(&out->counter[0], (unsigned)nch, &last) && gi < 3) {
+            const GroupSync sync{gi + 1};
+            const double t = gi < sums ? lanes_final_sum(part + gi, nch, 5, lane, sm + 4 * gi, sync) : 0.0;
+            if (lane == 0) (gi == 0 ? out->v_sum : gi == 1 ? out->p_out_sum : out->p_in_sum) = t;
+            if (border > 0 && gi > 0) {  // the node counts (whole numbers: exact in any order)
+                const double n = lanes_final_sum(part + 2 + gi, nch, 5, lane, sm + 4 * gi, sync);
+                if (lane == 0) (gi == 1 ? out->cnt_out : out->cnt_in) = n;
             }
+            if (threadIdx.x == 0) out->counter[0] = 0;
         }
     }
 }
 
 // ComputeDiv, src/NSBase.cxx:1958-2080
-__global__ void k_divergence(Grid g, Phys ph, SysView P, const double *__restrict__ u, const double *__restrict__ v,
-                             const double *__restrict__ w, double *__restrict__ part, DiagOut *out) {
-    __shared__ double sm[LANES];
+template <int G>
+__global__ void __launch_bounds__(LANES *G, 8 / G)
+    k_divergence(Grid g, Phys ph, SysView P, const double *__restrict__ u, const double *__restrict__ v,
+                 const double *__restrict__ w, double *__restrict__ part, DiagOut *out) {
+    __shared__ double s_div[CH], s_vel[CH], s_dv[CH], sm[16];
     __shared__ bool last;
     const int nx = g.nx, ny = g.ny, nz = g.nz;
     const double idx = ph.idx, idy = ph.idy, idz = ph.idz;
+    const int gi = threadIdx.x / LANES, lane = threadIdx.x % LANES;
     for (int c = blockIdx.x; c < P.nchunks; c += gridDim.x) {
-        double s2 = 0, sv = 0, mdv = 0, mdiv = 0;
-        for (int m = 0; m < RPL; ++m) {
-            int r = c * CH + threadIdx.x + LANES * m;
-            if (r >= P.n) break;
+        const int rows = min(CH, P.n - c * CH);
+#pragma unroll 1
+        for (int m = 0; m < RPL / G; ++m) {
+            const int q = lane + (gi * (RPL / G) + m) * LANES;
+            if (q >= rows) break;
             int i, j, k, f;
-            g.ijk(P.cell[r], i, j, k);
+            g.ijk(P.cell[c * CH + q], i, j, k);
             double div = 0, uu = 0, vv = 0, ww = 0, DV = 0;
             if (i > 0 && g.P(i - 1, j, k) > -1 && (f = g.U(i, j, k)) > -1) {
                 div += -u[f] * idx; DV += -u[f]; uu += u[f] * 0.5;
@@ -741,82 +744,113 @@ __global__ void k_divergence(Grid g, Phys ph, SysView P, const double *__restric
             if (i == nx - 1 && (f = g.U(i + 1, j, k)) > -1) {
                 div += u[f] * idx; DV += u[f]; uu += u[f] * 0.5;
             }
-            DV = fabs(DV);
-            div = fabs(div);
-            mdv = dmaxv(mdv, DV);
-            mdiv = dmaxv(mdiv, div);
-            s2 = __fma_rn(div, div, s2);
-            sv = sv + sqrt(uu * uu + vv * vv + ww * ww);
+            s_dv[q] = fabs(DV);
+            s_div[q] = fabs(div);
+            s_vel[q] = sqrt(uu * uu + vv * vv + ww * ww);
         }
-        double t2 = block_tree_sum(s2, sm);
-        double tv = block_tree_sum(sv, sm);
-        double tm1 = block_tree_max(mdv, sm);
-        double tm2 = block_tree_max(mdiv, sm);
-        if (threadIdx.x == 0) {
-            part[(size_t)c * 4 + 0] = t2;
-            part[(size_t)c * 4 + 1] = tv;
-            part[(size_t)c * 4 + 2] = tm1;
-            part[(size_t)c * 4 + 3] = tm2;
-        }
-        if (last_block_arrive(&out->counter[1], (unsigned)P.nchunks, &last)) {
-            double f2 = final_partials_sum(part + 0, P.nchunks, 4, sm);
-            double fv = final_partials_sum(part + 1, P.nchunks, 4, sm);
-            double m1 = 0, m2 = 0;
-            for (int q = threadIdx.x; q < P.nchunks; q += LANES) {
-                m1 = dmaxv(m1, __ldcg(part + (size_t)q * 4 + 2));
-                m2 = dmaxv(m2, __ldcg(part + (size_t)q * 4 + 3));
+        __syncthreads();
+        const GroupSync sync{gi + 1};
+        for (int j = gi; j < 2; j += G) {  // 0: sum of div^2 and its maximum, 1: sum of |u| and the maximum of DV
+            double acc = 0.0, mx = 0.0;
+            const double *val = j == 0 ? s_div : s_dv;
+#pragma unroll
+            for (int m = 0; m < RPL; ++m) {
+                const int q = lane + m * LANES;
+                if (q < rows) {
+                    acc = j == 0 ? __fma_rn(s_div[q], s_div[q], acc) : acc + s_vel[q];
+                    mx = dmaxv(mx, val[q]);
+                }
             }
-            m1 = block_tree_max(m1, sm);
-            m2 = block_tree_max(m2, sm);
-            if (threadIdx.x == 0) {
-                out->sumdiv2 = f2;
-                out->sumvel = fv;
-                out->maxdv = m1;
-                out->maxdiv = m2;
-                out->counter[1] = 0;
+            const double sum = lanes_tree_sum<double>(acc, lane, sm + 4 * j, sync);
+            const double ext = lanes_extreme<true>(mx, lane, sm + 8 + 4 * j, sync);
+            if (lane == 0) {
+                part[(size_t)c * 4 + j] = sum;
+                part[(size_t)c * 4 + 3 - j] = ext;
+            }
+        }
+        if (!last_block_arrive(&out->counter[1], (unsigned)P.nchunks, &last)) continue;
+        for (int j = gi; j < 2; j += G) {
+            const double sum = lanes_final_sum(part + j, P.nchunks, 4, lane, sm + 4 * j, sync);
+            double mx = 0.0;
+            for (int q = lane; q < P.nchunks; q += LANES) mx = dmaxv(mx, __ldcg(part + (size_t)q * 4 + 3 - j));
+            mx = lanes_extreme<true>(mx, lane, sm + 8 + 4 * j, sync);
+            if (lane == 0) {
+                if (j == 0) {
+                    out->sumdiv2 = sum;
+                    out->maxdiv = mx;
+                    out->counter[1] = 0;
+                } else {
+                    out->sumvel = sum;
+                    out->maxdv = mx;
+                }
             }
         }
     }
 }
 
 // CorrectPressureField, src/NSBase.cxx:2367-2380: max, min, |pc|^2, p += beta pc
-__global__ void k_correct_pressure(SysView P, const double *__restrict__ pc, double *__restrict__ p, double beta,
-                                   double *__restrict__ part, DiagOut *out) {
-    __shared__ double sm[LANES];
+template <int G>
+__global__ void __launch_bounds__(LANES *G, 8 / G)
+    k_correct_pressure(SysView P, const double *__restrict__ pc, double *__restrict__ p, double beta,
+                       double *__restrict__ part, DiagOut *out) {
+    __shared__ double s_x[CH], sm[12];
     __shared__ bool last;
+    const int gi = threadIdx.x / LANES, lane = threadIdx.x % LANES;
     for (int c = blockIdx.x; c < P.nchunks; c += gridDim.x) {
-        double mx = -HUGE_VAL, mn = HUGE_VAL, sq = 0;
-        for (int m = 0; m < RPL; ++m) {
-            int r = c * CH + threadIdx.x + LANES * m;
-            if (r >= P.n) break;
-            double x = pc[r];
-            mx = (x > mx) ? x : mx;
-            mn = (x < mn) ? x : mn;
-            sq = __fma_rn(x, x, sq);
-            p[r] = p[r] + beta * x;
-        }
-        double tmx = block_tree_max(mx, sm);
-        double tmn = block_tree_min(mn, sm);
-        double tsq = block_tree_sum(sq, sm);
-        if (threadIdx.x == 0) {
-            part[(size_t)c * 3 + 0] = tmx;
-            part[(size_t)c * 3 + 1] = tmn;
-            part[(size_t)c * 3 + 2] = tsq;
-        }
-        if (last_block_arrive(&out->counter[2], (unsigned)P.nchunks, &last)) {
-            double fsq = final_partials_sum(part + 2, P.nchunks, 3, sm);
-            double a = -HUGE_VAL, b = HUGE_VAL;
-            for (int q = threadIdx.x; q < P.nchunks; q += LANES) {
-                a = dmaxv(a, __ldcg(part + (size_t)q * 3 + 0));
-                b = dminv(b, __ldcg(part + (size_t)q * 3 + 1));
+        const int rows = min(CH, P.n - c * CH);
+#pragma unroll
+        for (int m = 0; m < RPL / G; ++m) {
+            const int q = lane + (gi * (RPL / G) + m) * LANES, r = c * CH + q;
+            if (q < rows) {
+                const double x = pc[r];
+                s_x[q] = x;
+                p[r] = p[r] + beta * x;
             }
-            a = block_tree_max(a, sm);
-            b = block_tree_min(b, sm);
-            if (threadIdx.x == 0) {
-                out->pcmax = a;
-                out->pcmin = b;
-                out->pcsq = fsq;
-                out->counter[2] = 0;
+        }
+        __syncthreads();
+        const GroupSync sync{gi + 1};
+        for (int j = gi; j < 2; j += G) {  // 0: sum of squares, 1: maximum and minimum
+            if (j == 0) {
+                const double sq = lanes_tree_sum<double>(lane_dot(s_x, s_x, lane, rows), lane, sm, sync);
+                if (lane == 0) part[(size_t)c * 3 + 2] = sq;
+            } else {
+                double mx = -HUGE_VAL, mn = HUGE_VAL;
+#pragma unroll
+                for (int m = 0; m < RPL; ++m) {
+                    const int q = lane + m * LANES;
+                    if (q < rows) {
+                        mx = dmaxv(mx, s_x[q]);
+                        mn = dminv(mn, s_x[q]);
+                    }
+                }
+                mx = lanes_extreme<true>(mx, lane, sm + 4, sync);
+                mn = lanes_extreme<false>(mn, lane, sm + 8, sync);
+                if (lane == 0) {
+                    part[(size_t)c * 3 + 0] = mx;
+                    part[(size_t)c * 3 + 1] = mn;
+                }
+            }
+        }
+        if (!last_block_arrive(&out->counter[2], (unsigned)P.nchunks, &last)) continue;
+        for (int j = gi; j < 2; j += G) {
+            if (j == 0) {
+                const double sq = lanes_final_sum(part + 2, P.nchunks, 3, lane, sm, sync);
+                if (lane == 0) {
+                    out->pcsq = sq;
+                    out->counter[2] = 0;
+                }
+            } else {
+                double a = -HUGE_VAL, b = HUGE_VAL;
+                for (int q = lane; q < P.nchunks; q += LANES) {
+                    a = dmaxv(a, __ldcg(part + (size_t)q * 3 + 0));
+                    b = dminv(b, __ldcg(part + (size_t)q * 3 + 1));
+                }
+                a = lanes_extreme<true>(a, lane, sm + 4, sync);
+                b = lanes_extreme<false>(b, lane, sm + 8, sync);
+                if (lane == 0) {
+                    out->pcmax = a;
+                    out->pcmin = b;
+                }
             }
         }
     }
@@ -962,7 +996,7 @@ void launch_permeability(const Grid &g, const double *u, const double *p, int bo
                          cudaStream_t st) {
     long plane = (long)g.ny * g.nz;
     int nch = (int)((plane + CH - 1) / CH);
-    count_launches(1); k_permeability<<<chunk_grid(nch), LANES, 0, st>>>(g, u, p, border, part, out);
+    count_launches(1); k_permeability<<<chunk_grid(nch), CH, 0, st>>>(g, u, p, border, part, out);
 }
 
 void launch_divergence(const Grid &g, const Phys &ph, const SysView &P, const double *u, const double *v,
@@ -971,13 +1005,21 @@ void launch_divergence(const Grid &g, const Phys &ph, const SysView &P, const do
         cudaMemsetAsync(&out->maxdv, 0, 4 * sizeof(double), st);
         return;
     }
-    count_launches(1); k_divergence<<<chunk_grid(P.nchunks), LANES, 0, st>>>(g, ph, P, u, v, w, part, out);
+    count_launches(1);
+    if (wide_chunks(P.nchunks, device_sm_count()))
+        k_divergence<WIDE_G><<<chunk_grid(P.nchunks), LANES * WIDE_G, 0, st>>>(g, ph, P, u, v, w, part, out);
+    else
+        k_divergence<NARROW_G><<<chunk_grid(P.nchunks), LANES * NARROW_G, 0, st>>>(g, ph, P, u, v, w, part, out);
 }
 
 void launch_correct_pressure(const SysView &P, const double *pc, double *p, double beta, double *part,
                              DiagOut *out, cudaStream_t st) {
     if (P.n <= 0) return;
-    count_launches(1); k_correct_pressure<<<chunk_grid(P.nchunks), LANES, 0, st>>>(P, pc, p, beta, part, out);
+    count_launches(1);
+    if (wide_chunks(P.nchunks, device_sm_count()))
+        k_correct_pressure<WIDE_G><<<chunk_grid(P.nchunks), LANES * WIDE_G, 0, st>>>(P, pc, p, beta, part, out);
+    else
+        k_correct_pressure<NARROW_G><<<chunk_grid(P.nchunks), LANES * NARROW_G, 0, st>>>(P, pc, p, beta, part, out);
 }
 
 void launch_default_pressure(const Grid &g, const SysView &P, double p0, double p1, double *p, cudaStream_t st) {
