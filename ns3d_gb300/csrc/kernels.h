@@ -82,6 +82,10 @@ void launch_face_average(const Grid &g, const double *u, const double *v, const 
 
 // krylov.cu: batched BiCGSTAB over a set of systems (instantiated for the
 // set capacities KMAX and KMAX_MERGED)
+// chooses the loop kernel of a solve of the set (kept until the solve ends:
+// the two keep different data in the work vectors); before the other launches
+template <int CAP>
+void plan_krylov(KSetArgT<CAP> &set, int share = 1);
 template <int CAP>
 void launch_krylov_init(const KSetArgT<CAP> &set, cudaStream_t st);
 // iterations until every system is done, one needs a restart, or max_iters

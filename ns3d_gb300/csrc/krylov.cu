@@ -100,6 +100,20 @@ __device__ __forceinline__ double spmv_row(const KSys &S, int row, const double 
     return spmv_row_nb(S, row, x, S.nbr + row, (size_t)S.npad);
 }
 
+// the same from a chunk's 16-bit distances (nb16[k * CH]: |column - row| of
+// slot k + 1, 0 = no entry): W, S and B columns lie before the row, E, N and
+// T columns after it
+__device__ __forceinline__ double spmv_row_16(const KSys &S, int row, const double *__restrict__ x,
+                                              const unsigned short *nb16) {
+    int nb[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        const int d = nb16[k * CH];
+        nb[k] = d == 0 ? -1 : row + ((k & 1) ? d : -d);
+    }
+    return spmv_row_nb(S, row, x, nb, 1);
+}
+
 // y = A x for the thread's rows (rows >= n give garbage that callers mask)
 __device__ __forceinline__ Row4 spmv4(const KSys &S, int r0, const double *__restrict__ x) {
     Row4 out;
@@ -246,22 +260,21 @@ __global__ void __launch_bounds__(LANES *G, 8 / G) k_kr_init(const __grid_consta
     }
 }
 
-// p = v = 0; x = 0 for a zero right-hand side; for the one-chunk-per-block
-// loop (`tags`) also the words it exchanges (krylov_chunk.cuh)
+// p = v = 0; x = 0 for a zero right-hand side; the words the loop kernels
+// exchange (krylov_chunk.cuh)
 template <int CAP>
-__global__ void k_kr_init2(const __grid_constant__ KSetArgT<CAP> A, bool tags) {
+__global__ void k_kr_init2(const __grid_constant__ KSetArgT<CAP> A) {
     NS3D_CHUNK_LOOP
         Row4 z;
 #pragma unroll
         for (int m = 0; m < RPL; ++m) z.v[m] = 0.0;
         st4(S.p + r0, z);
         st4(S.v + r0, z);
-        if (tags) {
+        if (A.one_per_block)
             for (double *q : {S.y, S.s, S.z, S.t}) st4(q + r0, z);
-            for (int k = threadIdx.x; k < TAG_KINDS * TAG_REPS; k += LANES) {
-                unsigned long long *slot = chunk_tag_words(S) + 2 * ((size_t)k * S.nchunks + lc);
-                slot[0] = slot[1] = 0;
-            }
+        for (int k = threadIdx.x; k < TAG_KINDS * TAG_REPS; k += LANES) {
+            unsigned long long *slot = chunk_tag_words(S) + 2 * ((size_t)k * S.nchunks + lc);
+            slot[0] = slot[1] = 0;
         }
         if (__ldcg(&S.st->zero_rhs)) st4(S.x + r0, z);
     }
@@ -272,47 +285,43 @@ __global__ void k_kr_init2(const __grid_constant__ KSetArgT<CAP> A, bool tags) {
 // LOOP_THREADS threads per block form LOOP_GROUPS groups of LANES threads; a
 // group processes whole chunks (its lanes own the rows of the fixed
 // reduction order) and reduces them with a named barrier.  Every block keeps
-// a copy of the per-system scalars in shared memory; after each grid-wide
-// barrier every block combines the chunk partials of each system in the
-// fixed order itself (group g for systems g, g + LOOP_GROUPS, ...), so all
-// copies stay bit-identical without a broadcast.  Partials of the three
-// reductions of an iteration go to separate regions of S.part, so a block
-// that runs ahead never overwrites partials another block is still
-// combining:
-//   [0, 2n)  <t,t>, <t,s> pairs     [2n, 4n)  <r0,r>, <r,r> pairs
-//   [4n, 5n) <r0,v>
+// a copy of the per-system scalars in shared memory.
+//
+// Two of the five phases read what other blocks wrote (y in K2, z in K4):
+// a grid barrier stands before them.  The three reductions need no grid
+// barrier: a thread's vectors are its own rows in every phase, so only the
+// chunk partials cross blocks, as words tagged with the system's iteration
+// (krylov_chunk.cuh), which every block polls and combines in the fixed order
+// itself; all scalar copies stay bit-identical without a broadcast.  A word
+// is rewritten only after the grid barrier of the next iteration.
 // The loop ends when every system is done, when a system needs a restart
 // (the host recomputes its residual and launches the loop again), after
-// `max_iters` iterations, or when a grid barrier gives up waiting.
+// `max_iters` iterations, or when a wait gives up.
+//
+// Loads come in batches before the first store of the batch: the vectors may
+// alias for the compiler, so a store between them would make every row wait
+// for its own loads (K1, K3 and K5 took 12.5, 11.5 and 17.0 us at 1.05 M rows
+// that way, 9.8, 7.0 and 16.1 in batches).
+constexpr int kSpmvUnroll = 2;  // rows in flight per thread in the SpMV phases (1: 1% slower, 4: 3%)
 
-// rows of a chunk in flight per thread in the SpMV phases (register budget)
-#ifndef NS3D_SPMV_UNROLL
-#define NS3D_SPMV_UNROLL 2
-#endif
-constexpr int kSpmvUnroll = NS3D_SPMV_UNROLL;
+// Resident neighbour tables (RES).  The matrix does not change during a
+// solve.  When no group has more than one chunk, each keeps its chunk's
+// columns in shared memory as 16-bit distances from the row (12 KB; 96 KB a
+// block): 48 B less traffic per row-iteration and no index load before the
+// gathers.  Columns further than 65535 rows away are read from memory, a
+// whole chunk at a time.  With more chunks per group the tables of one would
+// only take L1 from all: 32-bit tables of the first chunk (192 KB) made an
+// iteration of 3.55 M rows 291 us instead of 252.
+constexpr size_t kNbrSmemBytes = (size_t)LOOP_GROUPS * 6 * CH * sizeof(unsigned short);
 
-// Resident neighbour tables.  The matrix does not change during a solve, and
-// every group of the loop kernel processes the same chunks in every
-// iteration, so each group copies the six neighbour-column slabs of its
-// first chunk (6 x 1024 int32 = 24 KB) into shared memory once per launch
-// and both SpMV phases of every iteration gather through that copy: 48 B
-// per row-iteration less memory traffic, and the gathers of x no longer wait
-// for an index load from memory.  A group that owns more chunks (systems
-// above grid x LOOP_GROUPS chunks) reads the others' tables from memory.
-#ifndef NS3D_NBR_SMEM
-#define NS3D_NBR_SMEM 1
-#endif
-constexpr bool kNbrSmem = NS3D_NBR_SMEM != 0;
-constexpr size_t kNbrSmemBytes = kNbrSmem ? (size_t)LOOP_GROUPS * 6 * CH * sizeof(int) : 0;
-
-template <int CAP>
+template <int CAP, bool RES>
 __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
     k_kr_loop(const __grid_constant__ KSetArgT<CAP> A, GridBar *bar, LoopProf *prof, int max_iters) {
     static_assert(CAP <= LOOP_THREADS, "one thread copies each system's state");
     __shared__ KState sst[CAP];
     __shared__ double sm[LOOP_GROUPS][LANES];
     __shared__ int s_ok;
-    extern __shared__ int s_nbr_all[];  // [LOOP_GROUPS][6][CH] when kNbrSmem
+    extern __shared__ unsigned short s_nbr_all[];  // RES: [LOOP_GROUPS][6][CH]
     const int gi = threadIdx.x / LANES, lane = threadIdx.x % LANES;
     const GroupSync gsync{gi + 1};
     // chunk c belongs to block c % gridDim.x (group (c / gridDim.x) % LOOP_GROUPS):
@@ -320,14 +329,28 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
     const int gstride = gridDim.x * LOOP_GROUPS;
     const int cbegin = blockIdx.x + gridDim.x * gi;
     if (threadIdx.x < A.nsys) sst[threadIdx.x] = *A.sys[threadIdx.x].st;
-    if (kNbrSmem && cbegin < A.total_chunks) {  // this group's first chunk, for the whole launch
-        int *const s_nbr = s_nbr_all + (size_t)gi * 6 * CH;
+    bool far = false;  // RES: the chunk has a column beyond 16 bits
+    unsigned short *const s_nbr = s_nbr_all + (size_t)gi * 6 * CH + lane;
+    if (RES && cbegin < A.total_chunks) {  // this group's chunk, for the whole launch
         const KSys &S = A.sys[sys_of_chunk(A, cbegin)];
-        const int *src = S.nbr + (size_t)(cbegin - S.chunk_begin) * CH;
+        const int row0 = (cbegin - S.chunk_begin) * CH + lane;
 #pragma unroll
         for (int k = 0; k < 6; ++k)
 #pragma unroll
-            for (int m = 0; m < RPL; ++m) s_nbr[k * CH + lane + m * LANES] = src[(size_t)k * S.npad + lane + m * LANES];
+            for (int m = 0; m < RPL; ++m) {
+                const int row = row0 + m * LANES, c = ro(S.nbr + (size_t)k * S.npad + row);
+                const int d = c < 0 ? 0 : (k & 1) ? c - row : row - c;
+                far = far || d < 0 || d > 65535;
+                s_nbr[k * CH + m * LANES] = (unsigned short)d;
+            }
+        int any;  // over the group's 128 threads
+        asm volatile(
+            "{\n .reg .pred p, q;\n setp.ne.s32 p, %1, 0;\n barrier.cta.red.or.pred q, %2, %3, p;\n"
+            " selp.s32 %0, 1, 0, q;\n}"
+            : "=r"(any)
+            : "r"((int)far), "r"(gi + 1), "n"(LANES)
+            : "memory");
+        far = any != 0;
     }
     unsigned int target = grid_sync_start(bar);  // the counter is zeroed before every launch
     __syncthreads();           // the scalar copies in sst are complete
@@ -345,6 +368,10 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
             s_tp[5] = t;
         }
     };
+    auto row_product = [&](const KSys &S, int row, int m, const double *x) {
+        if (RES && !far) return spmv_row_16(S, row, x, s_nbr + m * LANES);
+        return spmv_row(S, row, x);
+    };
     int it = 0;
     bool ok = true;
     for (; it < max_iters; ++it) {
@@ -355,12 +382,24 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
             const KSys &S = A.sys[si];
             const int r0 = (c - S.chunk_begin) * CH + lane;
             const double beta = sst[si].beta, w = sst[si].w;
-#pragma unroll 4
-            for (int m = 0; m < RPL; ++m) {
-                const int row = r0 + m * LANES;
-                const double p = __fma_rn(beta, __fma_rn(-w, S.v[row], S.p[row]), S.r[row]);
-                S.p[row] = p;
-                S.y[row] = S.invdiag[row] * p;
+#pragma unroll
+            for (int m0 = 0; m0 < RPL; m0 += 4) {
+                double v[4], p[4], r[4], d[4];
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const int row = r0 + (m0 + m) * LANES;
+                    v[m] = S.v[row];
+                    p[m] = S.p[row];
+                    r[m] = S.r[row];
+                    d[m] = ro(S.invdiag + row);
+                }
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const int row = r0 + (m0 + m) * LANES;
+                    const double pn = __fma_rn(beta, __fma_rn(-w, v[m], p[m]), r[m]);
+                    S.p[row] = pn;
+                    S.y[row] = d[m] * pn;
+                }
             }
         }
         if (!(ok = grid_sync(bar, target, &s_ok))) break;
@@ -373,24 +412,12 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
             const int lc = c - S.chunk_begin;
             const int r0 = lc * CH + lane;
             double a = 0.0;
-            if (kNbrSmem && c == cbegin) {
-                // the resident copy: s_nbr_all[(gi * 6 + k) * CH + lane + m * LANES] for slot k, written
-                // from threadIdx.x = gi * LANES + lane so the offset stays one register
 #pragma unroll kSpmvUnroll
-                for (int m = 0; m < RPL; ++m) {
-                    const int row = r0 + m * LANES;
-                    const double v = spmv_row_nb(S, row, S.y, s_nbr_all + threadIdx.x + (gi * (6 * RPL - 1) + m) * LANES, CH);
-                    S.v[row] = v;
-                    if (row < S.n) a = __fma_rn(S.r0[row], v, a);
-                }
-            } else {
-#pragma unroll kSpmvUnroll
-                for (int m = 0; m < RPL; ++m) {
-                    const int row = r0 + m * LANES;
-                    const double v = spmv_row(S, row, S.y);
-                    S.v[row] = v;
-                    if (row < S.n) a = __fma_rn(S.r0[row], v, a);
-                }
+            for (int m = 0; m < RPL; ++m) {
+                const int row = r0 + m * LANES;
+                const double v = row_product(S, row, m, S.y);
+                S.v[row] = v;
+                if (row < S.n) a = __fma_rn(S.r0[row], v, a);
             }
             const double t = lanes_tree_sum(a, lane, sm[gi], gsync);
             if (lane == 0) S.part[4 * (size_t)S.nchunks + lc] = t;
@@ -411,12 +438,23 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
             const KSys &S = A.sys[si];
             const int r0 = (c - S.chunk_begin) * CH + lane;
             const double alpha = sst[si].alpha;
-#pragma unroll 4
-            for (int m = 0; m < RPL; ++m) {
-                const int row = r0 + m * LANES;
-                const double sv = __fma_rn(-alpha, S.v[row], S.r[row]);
-                S.s[row] = sv;
-                S.z[row] = S.invdiag[row] * sv;
+#pragma unroll
+            for (int m0 = 0; m0 < RPL; m0 += 4) {
+                double v[4], r[4], d[4];
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const int row = r0 + (m0 + m) * LANES;
+                    v[m] = S.v[row];
+                    r[m] = S.r[row];
+                    d[m] = ro(S.invdiag + row);
+                }
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const int row = r0 + (m0 + m) * LANES;
+                    const double sv = __fma_rn(-alpha, v[m], r[m]);
+                    S.s[row] = sv;
+                    S.z[row] = d[m] * sv;
+                }
             }
         }
         if (!(ok = grid_sync(bar, target, &s_ok))) break;
@@ -429,27 +467,14 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
             const int lc = c - S.chunk_begin;
             const int r0 = lc * CH + lane;
             double att = 0.0, ats = 0.0;
-            if (kNbrSmem && c == cbegin) {
 #pragma unroll kSpmvUnroll
-                for (int m = 0; m < RPL; ++m) {
-                    const int row = r0 + m * LANES;
-                    const double t = spmv_row_nb(S, row, S.z, s_nbr_all + threadIdx.x + (gi * (6 * RPL - 1) + m) * LANES, CH);
-                    S.t[row] = t;
-                    if (row < S.n) {
-                        att = __fma_rn(t, t, att);
-                        ats = __fma_rn(t, S.s[row], ats);
-                    }
-                }
-            } else {
-#pragma unroll kSpmvUnroll
-                for (int m = 0; m < RPL; ++m) {
-                    const int row = r0 + m * LANES;
-                    const double t = spmv_row(S, row, S.z);
-                    S.t[row] = t;
-                    if (row < S.n) {
-                        att = __fma_rn(t, t, att);
-                        ats = __fma_rn(t, S.s[row], ats);
-                    }
+            for (int m = 0; m < RPL; ++m) {
+                const int row = r0 + m * LANES;
+                const double t = row_product(S, row, m, S.z);
+                S.t[row] = t;
+                if (row < S.n) {
+                    att = __fma_rn(t, t, att);
+                    ats = __fma_rn(t, S.s[row], ats);
                 }
             }
             double tt, ts;
@@ -475,16 +500,30 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
             const int r0 = lc * CH + lane;
             const double alpha = sst[si].alpha, w = sst[si].w;
             double a0r = 0.0, arr = 0.0;
-#pragma unroll 4
-            for (int m = 0; m < RPL; ++m) {
-                const int row = r0 + m * LANES;
-                // rows >= n of x are padding; they receive values computed from zeros
-                S.x[row] = __fma_rn(w, S.z[row], __fma_rn(alpha, S.y[row], S.x[row]));
-                const double r = __fma_rn(-w, S.t[row], S.s[row]);
-                S.r[row] = r;
-                if (row < S.n) {
-                    a0r = __fma_rn(S.r0[row], r, a0r);
-                    arr = __fma_rn(r, r, arr);
+#pragma unroll
+            for (int m0 = 0; m0 < RPL; m0 += 2) {
+                double z[2], y[2], x[2], t[2], sv[2], q[2];
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    const int row = r0 + (m0 + m) * LANES;
+                    z[m] = S.z[row];
+                    y[m] = S.y[row];
+                    x[m] = S.x[row];
+                    t[m] = S.t[row];
+                    sv[m] = S.s[row];
+                    q[m] = S.r0[row];
+                }
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    const int row = r0 + (m0 + m) * LANES;
+                    // rows >= n of x are padding; they receive values computed from zeros
+                    S.x[row] = __fma_rn(w, z[m], __fma_rn(alpha, y[m], x[m]));
+                    const double r = __fma_rn(-w, t[m], sv[m]);
+                    S.r[row] = r;
+                    if (row < S.n) {
+                        a0r = __fma_rn(q[m], r, a0r);
+                        arr = __fma_rn(r, r, arr);
+                    }
                 }
             }
             double t0r, trr;
@@ -639,7 +678,7 @@ void launch_krylov_init(const KSetArgT<CAP> &A, cudaStream_t st) {
         k_kr_init<CAP, WIDE_G><<<kr_grid(A.total_chunks), LANES * WIDE_G, 0, st>>>(A);
     else
         k_kr_init<CAP, NARROW_G><<<kr_grid(A.total_chunks), LANES * NARROW_G, 0, st>>>(A);
-    k_kr_init2<CAP><<<kr_grid(A.total_chunks), LANES, 0, st>>>(A, A.total_chunks <= device_sm_count());
+    k_kr_init2<CAP><<<kr_grid(A.total_chunks), LANES, 0, st>>>(A);
 }
 
 // Blocks of a loop-kernel launch.  Every block must be resident at once
@@ -674,45 +713,47 @@ static int krylov_loop_grid(int total_chunks, int occ, int share) {
     return loop_grid(total_chunks, 1, occ);
 }
 
+// A set whose share of the SMs gives every chunk a block runs one chunk per
+// block (krylov_chunk.cuh), a larger one several chunks per block: a block has
+// one thread per row of its chunk, and the exchange needs every block
+// resident.  Measured, us per iteration, several per block -> one: 5 chunks
+// 35.4 -> 14.8, 44 chunks 38.4 -> 21.0, 141 chunks 39.9 -> 23.3.
+template <int CAP>
+void plan_krylov(KSetArgT<CAP> &A, int share) {
+    A.one_per_block = A.total_chunks <= device_sm_count() && krylov_loop_grid<CAP>(A.total_chunks, 1, share) >= A.total_chunks;
+}
+
 template <int CAP>
 cudaError_t launch_krylov_loop(const KSetArgT<CAP> &A, GridBar *bar, LoopProf *prof, int max_iters,
                                cudaStream_t st, int share) {
     if (A.total_chunks <= 0 || max_iters <= 0) return cudaSuccess;
-    static std::atomic<int> loop_occ{0};
-    int occ = loop_occ.load();
-    if (occ == 0) {
-        cudaError_t e = cudaSuccess;
-        if (kNbrSmemBytes > 0)
-            e = cudaFuncSetAttribute((const void *)k_kr_loop<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kNbrSmemBytes);
+    static std::atomic<bool> ready{false};
+    const void *one = (const void *)k_kr_chunk<CAP>, *res = (const void *)k_kr_loop<CAP, true>,
+               *many = (const void *)k_kr_loop<CAP, false>;
+    if (!ready.load()) {
+        cudaError_t e = cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChunkSmemBytes);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(res, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNbrSmemBytes);
         if (e != cudaSuccess) return e;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_kr_loop<CAP>, LOOP_THREADS, kNbrSmemBytes);
-        if (e != cudaSuccess) return e;
-        if (occ <= 0) return cudaErrorLaunchOutOfResources;
-        loop_occ = occ;
+        for (const void *fn : {one, res, many}) {  // one block of 1024 threads per SM
+            int occ = 0;
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, LOOP_THREADS,
+                                                              fn == one ? kChunkSmemBytes : fn == res ? kNbrSmemBytes : 0);
+            if (e != cudaSuccess) return e;
+            if (occ <= 0) return cudaErrorLaunchOutOfResources;
+        }
+        ready = true;
     }
-    const int grid = krylov_loop_grid<CAP>(A.total_chunks, occ, share);
     cudaError_t e = reset_grid_bar(bar, st);
     if (e != cudaSuccess) return e;
     KSetArgT<CAP> a = A;
     void *args[] = {&a, &bar, &prof, &max_iters};
     count_launches(1);
-    // A set whose share of the SMs gives every chunk a block runs one chunk
-    // per block (krylov_chunk.cuh), a larger one several chunks per block: a
-    // block has one thread per row of its chunk, and the exchange needs every
-    // block resident.  Measured, us per iteration, several per block -> one:
-    // 5 chunks 35.4 -> 14.8, 44 chunks 38.4 -> 21.0, 141 chunks 39.9 -> 23.3.
-    if (grid >= A.total_chunks && A.total_chunks <= device_sm_count()) {
-        static std::atomic<bool> ready{false};
-        if (!ready.load()) {
-            e = cudaFuncSetAttribute((const void *)k_kr_chunk<CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kChunkSmemBytes);
-            if (e != cudaSuccess) return e;
-            ready = true;
-        }
-        return cudaLaunchCooperativeKernel((const void *)k_kr_chunk<CAP>, A.total_chunks, CH, args, kChunkSmemBytes, st);
-    }
-    return cudaLaunchCooperativeKernel((const void *)k_kr_loop<CAP>, grid, LOOP_THREADS, args, kNbrSmemBytes, st);
+    if (A.one_per_block) return cudaLaunchCooperativeKernel(one, A.total_chunks, CH, args, kChunkSmemBytes, st);
+    const int grid = krylov_loop_grid<CAP>(A.total_chunks, 1, share);
+    if (A.total_chunks <= grid * LOOP_GROUPS)
+        return cudaLaunchCooperativeKernel(res, grid, LOOP_THREADS, args, kNbrSmemBytes, st);
+    return cudaLaunchCooperativeKernel(many, grid, LOOP_THREADS, args, 0, st);
 }
 
 template <int CAP>
@@ -725,6 +766,8 @@ void launch_krylov_restart(const KSetArgT<CAP> &A, cudaStream_t st) {
         k_kr_restart<CAP, NARROW_G><<<kr_grid(A.total_chunks), LANES * NARROW_G, 0, st>>>(A);
 }
 
+template void plan_krylov<KMAX>(KSetArg &, int);
+template void plan_krylov<KMAX_MERGED>(KSetArgMerged &, int);
 template void launch_krylov_init<KMAX>(const KSetArg &, cudaStream_t);
 template void launch_krylov_init<KMAX_MERGED>(const KSetArgMerged &, cudaStream_t);
 template cudaError_t launch_krylov_loop<KMAX>(const KSetArg &, GridBar *, LoopProf *, int, cudaStream_t, int);

@@ -141,6 +141,7 @@ extern "C" NS3D_API int ns3d_bicgstab_noalloc(const double *coef, const int32_t 
         return fail(NS3D_ERR_CUDA, "scratch set-up copy failed");
     k_noalloc_invdiag<<<std::max(1, std::min((n + 255) / 256, 1024)), 256, 0, st>>>(coef, n, invdiag);
     count_launches(1);
+    plan_krylov(set);
     launch_krylov_init(set, st);
     const long cap = 2L * maxit + 64;
     long issued = 0;

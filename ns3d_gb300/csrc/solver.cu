@@ -149,6 +149,7 @@ void KrylovSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st,
         maxit = std::max(maxit, items[i].maxit);
     }
     NS3D_CUDA_CHECK(cudaMemcpyAsync(st_.p, h_up_.p, ns * sizeof(KState), cudaMemcpyHostToDevice, st));
+    plan_krylov(set_, share);
     launch_krylov_init(set_, st);
     launches_ += 2;
     if (profiling) NS3D_CUDA_CHECK(cudaMemsetAsync(prof_.p, 0, sizeof(LoopProf), st));
@@ -162,7 +163,10 @@ void KrylovSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st,
     // merged sets: the grid of each loop launch comes from the autotuner,
     // which is told the launch's time per row-iteration
     const bool tune = CAP > KMAX;
-    const uint64_t tkey = tuner_key(0, total_chunks_, share);
+    // (a one-chunk-per-block set runs one grid whatever the candidate: its
+    // times stay out of the class of the larger sets that share its size
+    // bucket, 128 to 255 chunks)
+    const uint64_t tkey = tuner_key(0, set_.one_per_block ? std::min(total_chunks_, 127) : total_chunks_, share);
     int cand = 0;
     while (true) {
         NS3D_CUDA_CHECK(cudaMemcpyAsync(h_st_.p, st_.p, ns * sizeof(KState), cudaMemcpyDeviceToHost, st));
