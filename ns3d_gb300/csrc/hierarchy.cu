@@ -199,7 +199,7 @@ void build_hierarchy(DevSys &S, cudaStream_t st) {
         k_hb_members<<<hb_grid(nf), 256, 0, st>>>(cell, nf, box, mask.p, index.p, L.mstart.p, L.agg.p, L.members.p);
         k_hb_nbr<<<hb_grid(L.npad), 256, 0, st>>>(ccell.p, nc, L.npad, cbox, index.p, L.nbr.p);
         L.coef.alloc_zero((size_t)7 * L.npad, st);
-        for (DBuf<float> *b : {&L.invdiag, &L.x, &L.b, &L.t, &L.t2}) b->alloc_zero((size_t)L.npad, st);
+        for (DBuf<float> *b : {&L.invdiag, &L.x, &L.b, &L.t, &L.xo}) b->alloc_zero((size_t)L.npad, st);
         cell = ccell.p;
         box = cbox;
         nf = nc;

@@ -280,11 +280,11 @@ struct MGView {
     int n, npad;
     const int *nbr;
     const float *coef, *invdiag;
-    float *x, *b, *t, *t2;
+    float *x, *b, *t, *xo;  // Jacobi start, right-hand side, residual, result
 };
 
-// level k of the hierarchy of S (level 0: the FP32 system, solution x0 of
-// right-hand side b0, scratch S.t and S.p2)
+// level k of the hierarchy of S (level 0: the FP32 system, right-hand side b0,
+// Jacobi start S.p2, result x0, scratch S.t)
 __device__ __forceinline__ MGView mg_level(const MSys &S, int k, const float *b0, float *x0) {
     MGView L;
     if (k == 0) {
@@ -293,10 +293,10 @@ __device__ __forceinline__ MGView mg_level(const MSys &S, int k, const float *b0
         L.nbr = S.nbr;
         L.coef = S.coef32;
         L.invdiag = S.invdiag32;
-        L.x = x0;
+        L.x = S.p2;
         L.b = const_cast<float *>(b0);
         L.t = S.t;
-        L.t2 = S.p2;
+        L.xo = x0;
     } else {
         const MGLevel &G = S.mg.lev[k];
         L.n = G.n;
@@ -307,7 +307,7 @@ __device__ __forceinline__ MGView mg_level(const MSys &S, int k, const float *b0
         L.x = G.x;
         L.b = G.b;
         L.t = G.t;
-        L.t2 = G.t2;
+        L.xo = G.xo;
     }
     return L;
 }
@@ -334,8 +334,8 @@ __device__ __forceinline__ float mg_spmv(const MGView &L, int row, const float *
 
 // The passes of a V-cycle, one row each.  Down: the residual t of the
 // level's Jacobi start x, then the restriction of t with the next level's
-// Jacobi start.  Up: the residual t2 of x with the coarse correction cx
-// added on the fly, then x with correction and one damped Jacobi sweep.
+// Jacobi start.  Up: x with the coarse correction cx added on the fly and one
+// damped Jacobi sweep, into xo (the neighbours still read x).
 __device__ __forceinline__ void mg_down(const MGView &L, int r) { L.t[r] = L.b[r] - mg_spmv(L, r, L.x); }
 __device__ __forceinline__ void mg_restrict(const MGLevel &C, const float *t, float w, int I) {
     float acc = 0.0f;
@@ -343,12 +343,10 @@ __device__ __forceinline__ void mg_restrict(const MGLevel &C, const float *t, fl
     C.b[I] = acc;
     C.x[I] = w * C.invdiag[I] * acc;
 }
-__device__ __forceinline__ void mg_up(const MGView &L, const int *agg, const float *cx, int r) {
-    L.t2[r] = L.b[r] - mg_spmv_fn(L, r, [&](int c) { return L.x[c] + cx[ro(agg + c)]; });
-}
-__device__ __forceinline__ void mg_finish(const MGView &L, const int *agg, const float *cx, float w, int r) {
+__device__ __forceinline__ void mg_up(const MGView &L, const int *agg, const float *cx, float w, int r) {
     const float x = L.x[r] + cx[ro(agg + r)];
-    L.x[r] = x + w * L.invdiag[r] * L.t2[r];
+    const float t = L.b[r] - mg_spmv_fn(L, r, [&](int c) { return c == r ? x : L.x[c] + cx[ro(agg + c)]; });
+    L.xo[r] = x + w * L.invdiag[r] * t;
 }
 
 // Jacobi sweeps on the coarsest level by the calling block: x = w D^-1 b,
@@ -437,8 +435,8 @@ __device__ __forceinline__ float tail_spmv(const TailLevel &L, int r, F xf) {
 }
 
 // One V-cycle of the tail by the calling block, right-hand side restricted
-// from the residual t of the level above; the result is T[G.tail].x.
-__device__ void mg_tail(const MGSet &G, TailLevels &T, const float *t) {
+// from the residual t of the level above; returns the result.
+__device__ const float *mg_tail(const MGSet &G, TailLevels &T, const float *t) {
     const int K = G.nlev, tid = threadIdx.x, nth = blockDim.x;
     const float w = G.omega;
     for (int k = G.tail; k <= K; ++k) {
@@ -503,17 +501,19 @@ __device__ void mg_tail(const MGSet &G, TailLevels &T, const float *t) {
             __syncthreads();
         }
     }
+    const float *cx = T[K].x;
     for (int k = K - 1; k >= G.tail; --k) {
-        const TailLevel &L = T[k], &C = T[k + 1];
-        for (int r = tid; r < L.n; r += nth)
-            L.t[r] = L.b[r] - tail_spmv(L, r, [&](int c) { return L.x[c] + C.x[C.agg[c]]; });
-        __syncthreads();
+        const TailLevel &L = T[k];
+        const int *agg = T[k + 1].agg;
         for (int r = tid; r < L.n; r += nth) {
-            const float x = L.x[r] + C.x[C.agg[r]];
-            L.x[r] = x + w * L.invdiag[r] * L.t[r];
+            const float x = L.x[r] + cx[agg[r]];
+            const float t = L.b[r] - tail_spmv(L, r, [&](int c) { return L.x[c] + cx[agg[c]]; });
+            L.x2[r] = x + w * L.invdiag[r] * t;
         }
         __syncthreads();
+        cx = L.x2;
     }
+    return cx;
 }
 
 // x0 = M^-1 b0: one V-cycle -- a damped Jacobi sweep from zero, the residual
@@ -523,27 +523,27 @@ __device__ void mg_tail(const MGSet &G, TailLevels &T, const float *t) {
 // barriers between the passes); false when a barrier failed.  The fine
 // level's Jacobi start x0 = w D^-1 b0 is already written by the loop phase
 // that computed b0 (p or s), so the V-cycle starts with the fine residual.
-// Two passes down and two up per level: the restriction writes the next
-// level's Jacobi start, and the correction is added where x is read (a pass
-// that adds it first costs a grid barrier and 12 bytes a row more).  The up
-// pass writes its residual to t2, because other blocks may still read t for
-// their tail.  (Fusing residual and restriction too, one pass per coarse row,
-// measured 3-8% slower: it walks the fine rows out of order.)
+// Two passes down and one up per level: the restriction writes the next
+// level's Jacobi start; the way up adds the correction where x is read and
+// writes its result to another vector, so it needs no barrier between the
+// residual and the sweep.  (Fusing residual and restriction too, one pass per
+// coarse row, measured 3-8% slower: it walks the fine rows out of order.)
 // With the tail in shared memory an iteration of a 205 K-row system (five
-// levels) has 27 grid barriers instead of 53: six IDEAL outer iterations
-// 112.6 -> 83.1 ms; 3.6 M rows, six SIMPLEC outer iterations, 289 -> 271 ms.
+// levels) has 21 grid barriers instead of 53 with three passes each way and
+// every level in the grid.
 __device__ bool mg_apply(const MSys &S, const float *b0, float *x0, TailLevels &T, GridBar *bar, unsigned int &target,
                          int *s_ok) {
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int gth = gridDim.x * blockDim.x;
     const int K = S.mg.nlev, tail = S.mg.tail;
     const float w = S.mg.omega;
+    const float *cx = S.mg.lev[K].x;  // the coarse correction: the coarsest level's x, the other levels' xo
     for (int k = 0; k < K; ++k) {
         const MGView L = mg_level(S, k, b0, x0);
         for (int r = gtid; r < L.n; r += gth) mg_down(L, r);
         if (!grid_sync(bar, target, s_ok)) return false;
         if (k + 1 == tail) {
-            mg_tail(S.mg, T, L.t);
+            cx = mg_tail(S.mg, T, L.t);
             break;
         }
         const MGLevel &C = S.mg.lev[k + 1];
@@ -557,11 +557,9 @@ __device__ bool mg_apply(const MSys &S, const float *b0, float *x0, TailLevels &
     for (int k = min(K, tail) - 1; k >= 0; --k) {
         const MGView L = mg_level(S, k, b0, x0);
         const int *agg = S.mg.lev[k + 1].agg;
-        const float *cx = k + 1 == tail ? T[tail].x : S.mg.lev[k + 1].x;
-        for (int r = gtid; r < L.n; r += gth) mg_up(L, agg, cx, r);
+        for (int r = gtid; r < L.n; r += gth) mg_up(L, agg, cx, w, r);
         if (!grid_sync(bar, target, s_ok)) return false;
-        for (int r = gtid; r < L.n; r += gth) mg_finish(L, agg, cx, w, r);
-        if (!grid_sync(bar, target, s_ok)) return false;
+        cx = L.xo;
     }
     return true;
 }
@@ -628,12 +626,7 @@ __device__ bool mg_apply_set(const MSetArgT<CAP> &A, const KState *sst, const in
         auto rows = [&](int q) { return k == 0 ? A.sys[q].n : A.sys[q].mg.lev[k].n; };
         mg_rows(A, part, rows, [&](int q, int r) {
             const MGLevel &C = A.sys[q].mg.lev[k + 1];
-            mg_up(lvl(q, k), C.agg, C.x, r);
-        });
-        if (!grid_sync(bar, target, s_ok)) return false;
-        mg_rows(A, part, rows, [&](int q, int r) {
-            const MGLevel &C = A.sys[q].mg.lev[k + 1];
-            mg_finish(lvl(q, k), C.agg, C.x, A.sys[q].mg.omega, r);
+            mg_up(lvl(q, k), C.agg, k + 1 == A.sys[q].mg.nlev ? C.x : C.xo, A.sys[q].mg.omega, r);
         });
         if (!grid_sync(bar, target, s_ok)) return false;
     }
@@ -877,7 +870,8 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
                     const float p = __fmaf_rn(beta, __fmaf_rn(-w, S.v[row], S.p[row]), S.r[row]);
                     S.p[row] = p;
                     // a system with a hierarchy: the V-cycle's start w D^-1 p
-                    S.y[row] = S.mg.nlev > 0 ? S.mg.omega * S.invdiag32[row] * p : S.invdiag32[row] * p;
+                    if (S.mg.nlev > 0) S.p2[row] = S.mg.omega * S.invdiag32[row] * p;
+                    else S.y[row] = S.invdiag32[row] * p;
                 }
             }
             if (!grid_sync(bar, target, &s_ok)) break;
@@ -921,7 +915,8 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
                     const int row = r0 + m * LANES;
                     const float sv = __fmaf_rn(-alpha, S.v[row], S.r[row]);
                     S.s[row] = sv;
-                    S.z[row] = S.mg.nlev > 0 ? S.mg.omega * S.invdiag32[row] * sv : S.invdiag32[row] * sv;
+                    if (S.mg.nlev > 0) S.p2[row] = S.mg.omega * S.invdiag32[row] * sv;
+                    else S.z[row] = S.invdiag32[row] * sv;
                 }
             }
             if (!grid_sync(bar, target, &s_ok)) break;

@@ -34,7 +34,7 @@ struct MGLevel {
     const int *agg;       // [rows of level k-1]: the row of this level each belongs to
     const int *mstart;    // [n + 1]: offsets into members
     const int *members;   // rows of level k-1 of each row, ascending
-    float *x, *b, *t, *t2;  // V-cycle vectors [npad]
+    float *x, *b, *t, *xo;  // V-cycle vectors [npad]: Jacobi start, right-hand side, residual, result
 };
 struct MGSet {
     int nlev;             // coarse levels (0: Jacobi preconditioning)

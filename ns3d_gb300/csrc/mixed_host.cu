@@ -89,7 +89,7 @@ void MixedSetT<CAP>::configure(const std::vector<SolveItem> &items, cudaStream_t
                 G.x = H.x.p;
                 G.b = H.b.p;
                 G.t = H.t.p;
-                G.t2 = H.t2.p;
+                G.xo = H.xo.p;
             }
             // the tail: the levels that fit in a block's shared memory (a
             // merged set has no shared memory of its own per system)

@@ -100,7 +100,7 @@ inline int pad_rows(int n) { return ((n + CH - 1) / CH) * CH; }
 struct MGHostLevel {
     int n = 0, npad = 0;
     DBuf<int> nbr, agg, mstart, members;
-    DBuf<float> coef, invdiag, x, b, t, t2;
+    DBuf<float> coef, invdiag, x, b, t, xo;
 };
 struct MGHost {
     int nlev = 0;
