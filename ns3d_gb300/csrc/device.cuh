@@ -113,13 +113,16 @@ struct KSys {  // one system of a solve set (device array)
     const double *invdiag;
     const double *b;
     double *x, *r, *r0, *p, *v, *y, *s, *z, *t;
-    double *part;  // [PART_PER_CHUNK * nchunks]: reduction partials (layout in krylov.cu)
+    double *part;  // [part_doubles(nchunks)]: reduction partials (layout in krylov.cu, tags.cuh)
     KState *st;
 };
 
-// doubles held per chunk for reduction partials (the FP64 loop uses 5, the
-// FP32 loop 5 per quarter chunk, the one-chunk-per-block FP64 loop 84)
-constexpr int PART_PER_CHUNK = 84;
+// doubles held per chunk for reduction partials (plain ones: the FP64 loop
+// uses 5, the FP32 loop 5 per quarter chunk; tagged ones behind them: the
+// loops with resident chunks use 10 and 20), and per system (tags.cuh)
+constexpr int PART_PER_CHUNK = 40;
+constexpr int PART_FIXED = 96;
+inline __host__ __device__ size_t part_doubles(int nchunks) { return (size_t)PART_PER_CHUNK * nchunks + PART_FIXED; }
 
 // A solve set as a kernel argument (passed by value, read from constant
 // memory): the systems in chunk order, sys[0].chunk_begin == 0.  A solver

@@ -260,8 +260,8 @@ __global__ void __launch_bounds__(LANES *G, 8 / G) k_kr_init(const __grid_consta
     }
 }
 
-// p = v = 0; x = 0 for a zero right-hand side; the words the loop kernels
-// exchange (krylov_chunk.cuh)
+// p = v = 0; x = 0 for a zero right-hand side; what the one-chunk-per-block
+// loop exchanges (krylov_chunk.cuh)
 template <int CAP>
 __global__ void k_kr_init2(const __grid_constant__ KSetArgT<CAP> A) {
     NS3D_CHUNK_LOOP
@@ -270,11 +270,13 @@ __global__ void k_kr_init2(const __grid_constant__ KSetArgT<CAP> A) {
         for (int m = 0; m < RPL; ++m) z.v[m] = 0.0;
         st4(S.p + r0, z);
         st4(S.v + r0, z);
-        if (A.one_per_block)
+        if (A.one_per_block) {
             for (double *q : {S.y, S.s, S.z, S.t}) st4(q + r0, z);
-        for (int k = threadIdx.x; k < TAG_KINDS * TAG_REPS; k += LANES) {
-            unsigned long long *slot = chunk_tag_words(S) + 2 * ((size_t)k * S.nchunks + lc);
-            slot[0] = slot[1] = 0;
+            if (threadIdx.x < TAG_KINDS) {
+                unsigned long long *slot = chunk_tag_words(S) + 2 * ((size_t)threadIdx.x * S.nchunks + lc);
+                slot[0] = slot[1] = 0;
+                if (lc == 0) *tag_counter(S.part, S.nchunks, threadIdx.x) = 0;
+            }
         }
         if (__ldcg(&S.st->zero_rhs)) st4(S.x + r0, z);
     }
@@ -717,7 +719,7 @@ static int krylov_loop_grid(int total_chunks, int occ, int share) {
 // block (krylov_chunk.cuh), a larger one several chunks per block: a block has
 // one thread per row of its chunk, and the exchange needs every block
 // resident.  Measured, us per iteration, several per block -> one: 5 chunks
-// 35.4 -> 14.8, 44 chunks 38.4 -> 21.0, 141 chunks 39.9 -> 23.3.
+// 35.4 -> 15.0, 44 chunks 38.4 -> 17.5, 141 chunks 39.9 -> 19.2.
 template <int CAP>
 void plan_krylov(KSetArgT<CAP> &A, int share) {
     A.one_per_block = A.total_chunks <= device_sm_count() && krylov_loop_grid<CAP>(A.total_chunks, 1, share) >= A.total_chunks;

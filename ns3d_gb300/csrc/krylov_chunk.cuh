@@ -12,7 +12,7 @@
 //     two 8-byte words that each hold 32 bits of it and the 32-bit epoch
 //     (iteration number) it belongs to; a reader polls the words it needs
 //     until both carry the epoch.  A word is valid by itself, so no fence is
-//     needed: an all-reduce over the chunk partials takes 0.5-0.8 us instead
+//     needed: an all-reduce over the chunk partials takes 1.1-1.6 us instead
 //     of barrier, fence and load (2.1 us), y and z reach a neighbouring block
 //     in 1.3 us instead of 2.2 us;
 //   - neighbours inside the chunk are read from shared memory;
@@ -36,68 +36,18 @@
 // y and z.
 #pragma once
 
+#include "tags.cuh"
+
 namespace ns3d {
 
-// Copies of each chunk partial: block b polls copy b % TAG_REPS, because one
-// copy polled by 152 blocks takes 2.9 us where 44 blocks take 0.8 us.
-constexpr int TAG_REPS = 8;
-constexpr int TAG_KINDS = 5;  // <r0,v>, <t,t>, <t,s>, <r0,r>, <r,r>
 // S.part of a system: [0, 4 n) the plain partials of k_kr_init and
-// k_kr_restart, then 2 words per kind, copy and chunk
+// k_kr_restart, then 2 words per kind and chunk
 __device__ __forceinline__ unsigned long long *chunk_tag_words(const KSys &S) {
     return reinterpret_cast<unsigned long long *>(S.part + 4 * (size_t)S.nchunks);
 }
-static_assert(PART_PER_CHUNK >= 4 + 2 * TAG_KINDS * TAG_REPS, "tagged partials");
+static_assert(PART_PER_CHUNK >= 4 + 2 * TAG_KINDS, "tagged partials");
 
 constexpr size_t kChunkSmemBytes = (size_t)(7 + 10) * CH * sizeof(double) + (size_t)6 * CH * sizeof(int);
-
-__device__ __forceinline__ unsigned long long tag_lo(double v, unsigned int ep) {
-    return ((unsigned long long)ep << 32) | (unsigned int)__double2loint(v);
-}
-__device__ __forceinline__ unsigned long long tag_hi(double v, unsigned int ep) {
-    return ((unsigned long long)ep << 32) | (unsigned int)__double2hiint(v);
-}
-__device__ __forceinline__ double tag_value(unsigned long long lo, unsigned long long hi) {
-    return __hiloint2double((int)(unsigned int)hi, (int)(unsigned int)lo);
-}
-__device__ __forceinline__ bool tag_ok(unsigned long long lo, unsigned long long hi, unsigned int ep) {
-    return (unsigned int)(lo >> 32) == ep && (unsigned int)(hi >> 32) == ep;
-}
-__device__ __forceinline__ unsigned long long ld_word(const void *p) {
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_word(void *p, unsigned long long v) {
-    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ void ld_words(const void *p, unsigned long long &a, unsigned long long &b) {
-    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
-}
-__device__ __forceinline__ void st_words(void *p, unsigned long long a, unsigned long long b) {
-    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
-}
-
-// Bounded polling: false when the wait has run out (the same limit as the
-// grid barrier's), after setting bar->err and the thread's flag; the block
-// stops at its next barrier, which combines the flags.
-struct PollLimit {
-    GridBar *bar;
-    int &bad;
-    unsigned int polls = 0;
-    unsigned long long t0 = 0;
-    __device__ PollLimit(GridBar *b, int &f) : bar(b), bad(f) {}
-    __device__ __forceinline__ bool again() {
-        if ((++polls & 255u) != 0) return true;
-        const unsigned long long now = global_ns();
-        if (polls == 256u) t0 = now;
-        const unsigned long long lim = bar->limit_ns ? bar->limit_ns : kBarrierLimitNs;
-        if (now - t0 <= lim && polls <= 0x7fffffffu) return true;
-        atomicExch(&bar->err, 1);
-        bad = 1;
-        return false;
-    }
-};
 
 // The column values of the thread's row, slots W, E, S, N, B, T: neighbours
 // in the chunk from `own` (shared), the others from their tagged words; a
@@ -143,57 +93,35 @@ __device__ __forceinline__ void gather_tagged(const int *s_col, int base, int t,
     }
 }
 
-// The tree sum of lanes_tree_sum over the 128 threads of one group, of which
-// only the first `n` hold a value and the others +0: a level that would only
-// add those zeros is left out (v + 0 = v; no value here is -0).  FP64 adds
-// have a latency of 68 cycles, a level with its shuffle 94.  Valid in the
-// group's first thread; with n <= 32 only its first warp takes part.
-__device__ __forceinline__ double group_tree(double v, int n, int lane, double *red, GroupSync sync) {
-#pragma unroll
-    for (int off = 16; off >= 1; off >>= 1)
-        if (off < n) v = v + __shfl_down_sync(0xffffffffu, v, off);
-    if (n <= 32) return v;
-    if ((lane & 31) == 0) red[lane >> 5] = v;
-    sync();
-    double r = 0.0;
-    if (lane < 32) {
-        r = lane < LANES / 32 ? red[lane] : 0.0;
-        if (n > 64) r = r + __shfl_down_sync(0xffffffffu, r, 2);
-        r = r + __shfl_down_sync(0xffffffffu, r, 1);
-    }
-    return r;
-}
-
 // One dot product of a system over all its chunks, by one group of 128
-// threads: the chunk's partial from the operands in shared memory, published
-// in TAG_REPS copies, and the sum of all chunks' partials in the fixed order.
-// Valid in the group's first thread.  Every thread of the group calls
-// `published` once its part in publishing is done.
+// threads: the chunk's partial from the operands in shared memory, published,
+// and the sum of all chunks' partials in the fixed order.  Valid in the
+// group's first thread.  Every thread of the group calls `published` once its
+// part in publishing is done.
 template <class Published>
 __device__ __forceinline__ double dot_all(const KSys &S, int lc, int kind, const double *a, const double *b, int lane,
                                           unsigned int ep, unsigned int want, double *red, GroupSync sync,
                                           GridBar *bar, int &bad, Published published) {
     const int n = S.nchunks;
-    double acc = 0.0;
-    const int rows = min(CH, S.n - lc * CH);
-#pragma unroll
-    for (int m = 0; m < RPL; ++m)
-        if (lane + m * LANES < rows) acc = __fma_rn(a[lane + m * LANES], b[lane + m * LANES], acc);
-    double part = group_tree(acc, LANES, lane, red, sync);
-    unsigned long long *slots = chunk_tag_words(S) + 2 * (size_t)(kind * TAG_REPS) * n;
-    if (lane < 32) {
-        part = __shfl_sync(0xffffffffu, part, 0);
-        if (lane < TAG_REPS) st_words(slots + 2 * ((size_t)lane * n + lc), tag_lo(part, ep), tag_hi(part, ep));
+    const double part = group_tree(lane_dot(a, b, lane, min(CH, S.n - lc * CH)), LANES, lane, red, sync);
+    unsigned long long *slots = chunk_tag_words(S) + 2 * (size_t)kind * n;
+    unsigned int *counter = tag_counter(S.part, n, kind);
+    if (lane == 0) {
+        st_words(slots + 2 * (size_t)lc, tag_lo(part, ep), tag_hi(part, ep));
+        if (n > 32) count_arrival(counter);
     }
     published();
     if (n <= 32 && lane >= 32) return 0.0;  // the first warp alone combines them
-    const unsigned long long *mine = slots + 2 * (size_t)(blockIdx.x % TAG_REPS) * n;
     PollLimit limit(bar, bad);
+    if (n > 32) {  // fewer words are polled directly: one round trip less, and one warp only
+        if (lane == 0) wait_arrivals(counter, ep * (unsigned int)n, limit);
+        sync();
+    }
     double sum = 0.0;
     for (int i = lane; i < n; i += LANES) {
         unsigned long long lo, hi;
         while (true) {
-            ld_words(mine + 2 * (size_t)i, lo, hi);
+            ld_words(slots + 2 * (size_t)i, lo, hi);
             if (tag_ok(lo, hi, want) || !limit.again()) break;
         }
         sum = sum + tag_value(lo, hi);

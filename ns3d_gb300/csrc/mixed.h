@@ -68,6 +68,7 @@ struct MSys {
     const float *coef32, *invdiag32;
     float *x, *r, *r0, *p, *v, *y, *s, *z, *t;  // FP32 inner vectors (x is the correction)
     float *p2, *v2;  // second buffers of p and v (the loop kernel alternates them)
+    unsigned long long *wy, *wz;  // words of y and z exchanged by the loop with resident chunks (mixed_chunk.cuh)
     double *part;
     KState *st;  // inner BiCGSTAB state (scalars in FP64)
     DCState *dc;
@@ -81,6 +82,7 @@ constexpr int KMAX_MERGED_M = 32;
 template <int CAP>
 struct MSetArgT {
     int nsys, total_chunks;
+    int resident, pad_;  // chunks per block of the loop with resident chunks; 0: the other loops (plan_mixed)
     MSys sys[CAP];
 };
 using MSetArg = MSetArgT<KMAX>;
@@ -92,6 +94,10 @@ void launch_mg_galerkin(const MSys &sys, cudaStream_t st);
 void launch_to_f32(const double *coef, const double *invdiag, int npad, float *coef32, float *invdiag32,
                    cudaStream_t st);
 // (the set launchers are instantiated for CAP = KMAX and KMAX_MERGED_M)
+// chooses the FP32 loop of a solve of the set (kept for all its rounds);
+// before the other launches
+template <int CAP>
+void plan_mixed(MSetArgT<CAP> &set, int variant, int share);
 template <int CAP>
 void launch_dc_resid(const MSetArgT<CAP> &set, int first, cudaStream_t st);
 template <int CAP>

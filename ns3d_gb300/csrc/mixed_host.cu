@@ -58,6 +58,8 @@ void MixedSetT<CAP>::configure(const std::vector<SolveItem> &items, cudaStream_t
         m.x64 = items[i].x;
         m.r64 = S.r.p;
         m.d64 = S.y.p;
+        m.wy = reinterpret_cast<unsigned long long *>(S.p.p);
+        m.wz = reinterpret_cast<unsigned long long *>(S.v.p);
         m.coef32 = S.coef32.p;
         m.invdiag32 = S.invdiag32.p;
         m.x = S.fx.p; m.r = S.fr.p; m.r0 = S.fr0.p; m.p = S.fp.p; m.v = S.fv.p;
@@ -152,6 +154,7 @@ void MixedSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st, s
     }
     NS3D_CUDA_CHECK(cudaMemcpyAsync(dc_.p, h_dc_.p, ns * sizeof(DCState), cudaMemcpyHostToDevice, st));
     NS3D_CUDA_CHECK(cudaMemcpyAsync(st_.p, h_st_.p, ns * sizeof(KState), cudaMemcpyHostToDevice, st));
+    plan_mixed(set_, variant, share);
     launch_dc_resid(set_, 1, st);
     // Every round runs at least one inner iteration per unfinished system, so
     // maxit + 2 rounds bound the loop; each round's inner loop is bounded by
@@ -164,7 +167,7 @@ void MixedSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st, s
     if (tune) {
         bool mg = false;
         for (int i = 0; i < ns; ++i) mg = mg || set_.sys[i].mg.nlev > 0;
-        kind = mg ? 3 : (variant == 1 ? 2 : 1);
+        kind = mg ? 3 : set_.resident ? 4 : (variant == 1 ? 2 : 1);
         if (!ev_[0])
             for (cudaEvent_t &e : ev_) NS3D_CUDA_CHECK(cudaEventCreate(&e));
     }

@@ -34,7 +34,7 @@ constexpr int kScratchRows = 1 << 16;
 constexpr int kScratchChunks = kScratchRows / CH;
 constexpr int kVectors = 9;  // r, r0, p, v, y, s, z, t, invdiag
 constexpr size_t kVecBytes = (size_t)kVectors * kScratchRows * sizeof(double);
-constexpr size_t kPartBytes = (size_t)PART_PER_CHUNK * kScratchChunks * sizeof(double);
+constexpr size_t kPartBytes = ((size_t)PART_PER_CHUNK * kScratchChunks + PART_FIXED) * sizeof(double);
 constexpr size_t kStateOffset = kVecBytes + kPartBytes;
 constexpr size_t kBarOffset = kStateOffset + 256;
 constexpr size_t kScratchBytes = kBarOffset + 512;

@@ -42,7 +42,7 @@ void DevSys::allocate(int rows, int first_extent, cudaStream_t st) {
     invdiag.alloc_zero(npad, st);
     DBuf<double> *ws[] = {&r, &r0, &p, &v, &y, &s, &z, &t};
     for (auto *b : ws) b->alloc_zero(npad, st);
-    part.alloc_zero((size_t)PART_PER_CHUNK * std::max(nchunks, 1), st);
+    part.alloc_zero(part_doubles(std::max(nchunks, 1)), st);
 }
 
 size_t DevSys::device_bytes() const {

@@ -49,7 +49,8 @@ class GridTuner {
 GridTuner &grid_tuner();
 
 // class of a merged set: kind (0 FP64; 1 mixed five-phase; 2 mixed fused;
-// 3 mixed with multilevel systems), work units (power-of-two bucket) and the
+// 3 mixed with multilevel systems; 4 mixed with resident chunks, whose grid
+// does not depend on the candidate), work units (power-of-two bucket) and the
 // lanes sharing the SMs
 inline uint64_t tuner_key(int kind, long units, int share) {
     int bucket = 0;
