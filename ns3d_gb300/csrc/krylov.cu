@@ -285,61 +285,73 @@ __global__ void k_kr_init2(const __grid_constant__ KSetArgT<CAP> A) {
 // ---- the BiCGSTAB iteration loop: one persistent cooperative kernel ----------
 //
 // LOOP_THREADS threads per block form LOOP_GROUPS groups of LANES threads; a
-// group processes whole chunks (its lanes own the rows of the fixed
-// reduction order) and reduces them with a named barrier.  Every block keeps
-// a copy of the per-system scalars in shared memory.
-//
-// Two of the five phases read what other blocks wrote (y in K2, z in K4):
-// a grid barrier stands before them.  The three reductions need no grid
-// barrier: a thread's vectors are its own rows in every phase, so only the
-// chunk partials cross blocks, as words tagged with the system's iteration
-// (krylov_chunk.cuh), which every block polls and combines in the fixed order
-// itself; all scalar copies stay bit-identical without a broadcast.  A word
-// is rewritten only after the grid barrier of the next iteration.
+// chunk is worked on by GPC groups (the lanes own the rows of the fixed
+// reduction order) and reduced with a named barrier.  Every block keeps a copy
+// of the per-system scalars in shared memory; after each grid-wide barrier
+// every block combines the chunk partials of each system in the fixed order
+// itself (group g for systems g, g + LOOP_GROUPS, ...), so all copies stay
+// bit-identical without a broadcast.  Partials of the three reductions of an
+// iteration go to separate regions of S.part, so a block that runs ahead never
+// overwrites partials another block is still combining:
+//   [0, 2n)  <t,t>, <t,s> pairs     [2n, 4n)  <r0,r>, <r,r> pairs
+//   [4n, 5n) <r0,v>
 // The loop ends when every system is done, when a system needs a restart
 // (the host recomputes its residual and launches the loop again), after
-// `max_iters` iterations, or when a wait gives up.
+// `max_iters` iterations, or when a grid barrier gives up waiting.
+//
+// GPC 0: any number of chunks per group (group g of the grid takes chunks
+// g, g + groups, ...).  GPC 1, 2, 4: one chunk per GPC groups and no more, so
+// a set of 1.2 to 4 chunks per SM does not leave half of the groups idle: a
+// chunk's rows are split over its groups (group p takes the lanes' rows
+// p RPL / GPC ...), and the lanes' sums pass from group to group through
+// shared memory, in row order (eight images in lockstep, pressure sets of
+// about 480 chunks: 185 -> 168 ms).
 //
 // Loads come in batches before the first store of the batch: the vectors may
 // alias for the compiler, so a store between them would make every row wait
 // for its own loads (K1, K3 and K5 took 12.5, 11.5 and 17.0 us at 1.05 M rows
-// that way, 9.8, 7.0 and 16.1 in batches).
+// that way, 9.8, 7.0 and 16.1 in batches).  x is updated between the two
+// halves of the last barrier, in time the block would spend waiting.
 constexpr int kSpmvUnroll = 2;  // rows in flight per thread in the SpMV phases (1: 1% slower, 4: 3%)
 
-// Resident neighbour tables (RES).  The matrix does not change during a
-// solve.  When no group has more than one chunk, each keeps its chunk's
-// columns in shared memory as 16-bit distances from the row (12 KB; 96 KB a
-// block): 48 B less traffic per row-iteration and no index load before the
-// gathers.  Columns further than 65535 rows away are read from memory, a
-// whole chunk at a time.  With more chunks per group the tables of one would
-// only take L1 from all: 32-bit tables of the first chunk (192 KB) made an
-// iteration of 3.55 M rows 291 us instead of 252.
-constexpr size_t kNbrSmemBytes = (size_t)LOOP_GROUPS * 6 * CH * sizeof(unsigned short);
+// Resident neighbour tables (GPC > 0).  The matrix does not change during a
+// solve, so the block keeps its chunks' columns in shared memory as 16-bit
+// distances from the row (12 KB a chunk): 48 B less traffic per row-iteration
+// and no index load before the gathers.  Columns further than 65535 rows away
+// are read from memory, a group's rows at a time.  With GPC 0 the tables of
+// one chunk would only take L1 from all: 32-bit tables of the first chunk
+// (192 KB) made an iteration of 3.55 M rows 291 us instead of 252.
+template <int GPC>
+constexpr size_t kNbrSmemBytes = GPC ? (size_t)(LOOP_GROUPS / (GPC ? GPC : 1)) * 6 * CH * sizeof(unsigned short) : 0;
 
-template <int CAP, bool RES>
+template <int CAP, int GPC>
 __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
     k_kr_loop(const __grid_constant__ KSetArgT<CAP> A, GridBar *bar, LoopProf *prof, int max_iters) {
     static_assert(CAP <= LOOP_THREADS, "one thread copies each system's state");
+    constexpr bool RES = GPC > 0;
+    constexpr int PARTS = RES ? GPC : 1, RP = RPL / PARTS, BATCH = RP < 4 ? RP : 4;
     __shared__ KState sst[CAP];
-    __shared__ double sm[LOOP_GROUPS][LANES];
+    __shared__ double sm[LOOP_GROUPS][16];
+    __shared__ double s_acc[PARTS > 1 ? LOOP_GROUPS : 1][2][LANES];  // the lanes' sums on their way
     __shared__ int s_ok;
-    extern __shared__ unsigned short s_nbr_all[];  // RES: [LOOP_GROUPS][6][CH]
-    const int gi = threadIdx.x / LANES, lane = threadIdx.x % LANES;
+    extern __shared__ unsigned short s_nbr_all[];  // RES: [LOOP_GROUPS / GPC][6][CH]
+    const int gi = threadIdx.x / LANES, lane = threadIdx.x % LANES, part = gi % PARTS;
     const GroupSync gsync{gi + 1};
-    // chunk c belongs to block c % gridDim.x (group (c / gridDim.x) % LOOP_GROUPS):
-    // every block, hence every SM, gets the same number of chunks to within one
+    // chunk c belongs to block c % gridDim.x: every block, hence every SM,
+    // gets the same number of chunks to within one
     const int gstride = gridDim.x * LOOP_GROUPS;
-    const int cbegin = blockIdx.x + gridDim.x * gi;
+    const int cbegin = blockIdx.x + gridDim.x * (gi / PARTS);
+    const int lane0 = part * RP * LANES + lane;  // the thread's first row in a chunk
     if (threadIdx.x < A.nsys) sst[threadIdx.x] = *A.sys[threadIdx.x].st;
-    bool far = false;  // RES: the chunk has a column beyond 16 bits
-    unsigned short *const s_nbr = s_nbr_all + (size_t)gi * 6 * CH + lane;
-    if (RES && cbegin < A.total_chunks) {  // this group's chunk, for the whole launch
+    bool far = false;  // RES: a row of the group has a column beyond 16 bits
+    unsigned short *const s_nbr = s_nbr_all + (size_t)(gi / PARTS) * 6 * CH + lane0;
+    if (RES && cbegin < A.total_chunks) {  // the group's rows, for the whole launch
         const KSys &S = A.sys[sys_of_chunk(A, cbegin)];
-        const int row0 = (cbegin - S.chunk_begin) * CH + lane;
+        const int row0 = (cbegin - S.chunk_begin) * CH + lane0;
 #pragma unroll
         for (int k = 0; k < 6; ++k)
 #pragma unroll
-            for (int m = 0; m < RPL; ++m) {
+            for (int m = 0; m < RP; ++m) {
                 const int row = row0 + m * LANES, c = ro(S.nbr + (size_t)k * S.npad + row);
                 const int d = c < 0 ? 0 : (k & 1) ? c - row : row - c;
                 far = far || d < 0 || d > 65535;
@@ -355,7 +367,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
         far = any != 0;
     }
     unsigned int target = grid_sync_start(bar);  // the counter is zeroed before every launch
-    __syncthreads();           // the scalar copies in sst are complete
+    __syncthreads();  // the scalar copies in sst are complete
     // phase times of block 0 (thread 0), kept in shared memory
     __shared__ unsigned long long s_tp[6];
     const bool timing = prof != nullptr && blockIdx.x == 0 && threadIdx.x == 0;
@@ -374,6 +386,25 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
         if (RES && !far) return spmv_row_16(S, row, x, s_nbr + m * LANES);
         return spmv_row(S, row, x);
     };
+    // before a group adds to its chunk's lane sums: take them from the group
+    // before it (named barrier 8 + gi: that group arrives, this one waits)
+    auto take = [&](double &a, double &b) {
+        if (PARTS > 1 && part > 0) {
+            asm volatile("bar.sync %0, %1;" ::"r"(8 + gi), "n"(2 * LANES) : "memory");
+            a = s_acc[gi - 1][0][lane];
+            b = s_acc[gi - 1][1][lane];
+        }
+    };
+    // afterwards: pass them on; true for the chunk's last group, which reduces them
+    auto pass = [&](double a, double b) {
+        if (PARTS > 1 && part < PARTS - 1) {
+            s_acc[gi][0][lane] = a;
+            s_acc[gi][1][lane] = b;
+            asm volatile("bar.arrive %0, %1;" ::"r"(9 + gi), "n"(2 * LANES) : "memory");
+            return false;
+        }
+        return true;
+    };
     int it = 0;
     bool ok = true;
     for (; it < max_iters; ++it) {
@@ -382,13 +413,13 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
             const int si = sys_of_chunk(A, c);
             if (!state_active(sst[si])) continue;
             const KSys &S = A.sys[si];
-            const int r0 = (c - S.chunk_begin) * CH + lane;
+            const int r0 = (c - S.chunk_begin) * CH + lane0;
             const double beta = sst[si].beta, w = sst[si].w;
 #pragma unroll
-            for (int m0 = 0; m0 < RPL; m0 += 4) {
-                double v[4], p[4], r[4], d[4];
+            for (int m0 = 0; m0 < RP; m0 += BATCH) {
+                double v[BATCH], p[BATCH], r[BATCH], d[BATCH];
 #pragma unroll
-                for (int m = 0; m < 4; ++m) {
+                for (int m = 0; m < BATCH; ++m) {
                     const int row = r0 + (m0 + m) * LANES;
                     v[m] = S.v[row];
                     p[m] = S.p[row];
@@ -396,13 +427,14 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
                     d[m] = ro(S.invdiag + row);
                 }
 #pragma unroll
-                for (int m = 0; m < 4; ++m) {
+                for (int m = 0; m < BATCH; ++m) {
                     const int row = r0 + (m0 + m) * LANES;
                     const double pn = __fma_rn(beta, __fma_rn(-w, v[m], p[m]), r[m]);
                     S.p[row] = pn;
                     S.y[row] = d[m] * pn;
                 }
             }
+            if (RES) break;
         }
         if (!(ok = grid_sync(bar, target, &s_ok))) break;
         mark(0);
@@ -411,18 +443,36 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
             const int si = sys_of_chunk(A, c);
             if (!state_active(sst[si])) continue;
             const KSys &S = A.sys[si];
-            const int lc = c - S.chunk_begin;
-            const int r0 = lc * CH + lane;
-            double a = 0.0;
+            const int lc = c - S.chunk_begin, r0 = lc * CH + lane0;
+            double a = 0.0, none = 0.0;
+            if constexpr (PARTS > 1) {
+                double v[RP], q[RP];
+#pragma unroll
+                for (int m = 0; m < RP; ++m) {
+                    const int row = r0 + m * LANES;
+                    v[m] = row_product(S, row, m, S.y);
+                    q[m] = S.r0[row];
+                }
+                take(a, none);
+#pragma unroll
+                for (int m = 0; m < RP; ++m) {
+                    S.v[r0 + m * LANES] = v[m];
+                    if (r0 + m * LANES < S.n) a = __fma_rn(q[m], v[m], a);
+                }
+            } else {
 #pragma unroll kSpmvUnroll
-            for (int m = 0; m < RPL; ++m) {
-                const int row = r0 + m * LANES;
-                const double v = row_product(S, row, m, S.y);
-                S.v[row] = v;
-                if (row < S.n) a = __fma_rn(S.r0[row], v, a);
+                for (int m = 0; m < RP; ++m) {
+                    const int row = r0 + m * LANES;
+                    const double v = row_product(S, row, m, S.y);
+                    S.v[row] = v;
+                    if (row < S.n) a = __fma_rn(S.r0[row], v, a);
+                }
             }
-            const double t = lanes_tree_sum(a, lane, sm[gi], gsync);
-            if (lane == 0) S.part[4 * (size_t)S.nchunks + lc] = t;
+            if (pass(a, none)) {
+                const double t = lanes_tree_sum(a, lane, sm[gi], gsync);
+                if (lane == 0) S.part[4 * (size_t)S.nchunks + lc] = t;
+            }
+            if (RES) break;
         }
         if (!(ok = grid_sync(bar, target, &s_ok))) break;
         for (int q = gi; q < A.nsys; q += LOOP_GROUPS) {
@@ -438,26 +488,27 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
             const int si = sys_of_chunk(A, c);
             if (!state_active(sst[si])) continue;
             const KSys &S = A.sys[si];
-            const int r0 = (c - S.chunk_begin) * CH + lane;
+            const int r0 = (c - S.chunk_begin) * CH + lane0;
             const double alpha = sst[si].alpha;
 #pragma unroll
-            for (int m0 = 0; m0 < RPL; m0 += 4) {
-                double v[4], r[4], d[4];
+            for (int m0 = 0; m0 < RP; m0 += BATCH) {
+                double v[BATCH], r[BATCH], d[BATCH];
 #pragma unroll
-                for (int m = 0; m < 4; ++m) {
+                for (int m = 0; m < BATCH; ++m) {
                     const int row = r0 + (m0 + m) * LANES;
                     v[m] = S.v[row];
                     r[m] = S.r[row];
                     d[m] = ro(S.invdiag + row);
                 }
 #pragma unroll
-                for (int m = 0; m < 4; ++m) {
+                for (int m = 0; m < BATCH; ++m) {
                     const int row = r0 + (m0 + m) * LANES;
                     const double sv = __fma_rn(-alpha, v[m], r[m]);
                     S.s[row] = sv;
                     S.z[row] = d[m] * sv;
                 }
             }
+            if (RES) break;
         }
         if (!(ok = grid_sync(bar, target, &s_ok))) break;
         mark(2);
@@ -466,22 +517,43 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
             const int si = sys_of_chunk(A, c);
             if (!state_active(sst[si])) continue;
             const KSys &S = A.sys[si];
-            const int lc = c - S.chunk_begin;
-            const int r0 = lc * CH + lane;
+            const int lc = c - S.chunk_begin, r0 = lc * CH + lane0;
             double att = 0.0, ats = 0.0;
+            if constexpr (PARTS > 1) {
+                double t[RP], q[RP];
+#pragma unroll
+                for (int m = 0; m < RP; ++m) {
+                    const int row = r0 + m * LANES;
+                    t[m] = row_product(S, row, m, S.z);
+                    q[m] = S.s[row];
+                }
+                take(att, ats);
+#pragma unroll
+                for (int m = 0; m < RP; ++m) {
+                    S.t[r0 + m * LANES] = t[m];
+                    if (r0 + m * LANES < S.n) {
+                        att = __fma_rn(t[m], t[m], att);
+                        ats = __fma_rn(t[m], q[m], ats);
+                    }
+                }
+            } else {
 #pragma unroll kSpmvUnroll
-            for (int m = 0; m < RPL; ++m) {
-                const int row = r0 + m * LANES;
-                const double t = row_product(S, row, m, S.z);
-                S.t[row] = t;
-                if (row < S.n) {
-                    att = __fma_rn(t, t, att);
-                    ats = __fma_rn(t, S.s[row], ats);
+                for (int m = 0; m < RP; ++m) {
+                    const int row = r0 + m * LANES;
+                    const double t = row_product(S, row, m, S.z);
+                    S.t[row] = t;
+                    if (row < S.n) {
+                        att = __fma_rn(t, t, att);
+                        ats = __fma_rn(t, S.s[row], ats);
+                    }
                 }
             }
-            double tt, ts;
-            lanes_tree_sum2(att, ats, lane, sm[gi], tt, ts, gsync);
-            if (lane == 0) reinterpret_cast<double2 *>(S.part)[lc] = make_double2(tt, ts);
+            if (pass(att, ats)) {
+                double tt, ts;
+                lanes_tree_sum2(att, ats, lane, sm[gi], tt, ts, gsync);
+                if (lane == 0) reinterpret_cast<double2 *>(S.part)[lc] = make_double2(tt, ts);
+            }
+            if (RES) break;
         }
         if (!(ok = grid_sync(bar, target, &s_ok))) break;
         for (int q = gi; q < A.nsys; q += LOOP_GROUPS) {
@@ -493,33 +565,28 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
         }
         __syncthreads();
         mark(3);
-        // K5: x += alpha y + w z; r = s - w t; <r0, r>, <r, r>
+        // K5: r = s - w t; <r0, r>, <r, r>
         for (int c = cbegin; c < A.total_chunks; c += gstride) {
             const int si = sys_of_chunk(A, c);
             if (!state_active(sst[si])) continue;
             const KSys &S = A.sys[si];
-            const int lc = c - S.chunk_begin;
-            const int r0 = lc * CH + lane;
-            const double alpha = sst[si].alpha, w = sst[si].w;
+            const int lc = c - S.chunk_begin, r0 = lc * CH + lane0;
+            const double w = sst[si].w;
             double a0r = 0.0, arr = 0.0;
 #pragma unroll
-            for (int m0 = 0; m0 < RPL; m0 += 2) {
-                double z[2], y[2], x[2], t[2], sv[2], q[2];
+            for (int m0 = 0; m0 < RP; m0 += BATCH) {
+                double t[BATCH], sv[BATCH], q[BATCH];
 #pragma unroll
-                for (int m = 0; m < 2; ++m) {
+                for (int m = 0; m < BATCH; ++m) {
                     const int row = r0 + (m0 + m) * LANES;
-                    z[m] = S.z[row];
-                    y[m] = S.y[row];
-                    x[m] = S.x[row];
                     t[m] = S.t[row];
                     sv[m] = S.s[row];
                     q[m] = S.r0[row];
                 }
+                if (m0 == 0) take(a0r, arr);
 #pragma unroll
-                for (int m = 0; m < 2; ++m) {
+                for (int m = 0; m < BATCH; ++m) {
                     const int row = r0 + (m0 + m) * LANES;
-                    // rows >= n of x are padding; they receive values computed from zeros
-                    S.x[row] = __fma_rn(w, z[m], __fma_rn(alpha, y[m], x[m]));
                     const double r = __fma_rn(-w, t[m], sv[m]);
                     S.r[row] = r;
                     if (row < S.n) {
@@ -528,11 +595,38 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
                     }
                 }
             }
-            double t0r, trr;
-            lanes_tree_sum2(a0r, arr, lane, sm[gi], t0r, trr, gsync);
-            if (lane == 0) reinterpret_cast<double2 *>(S.part + 2 * (size_t)S.nchunks)[lc] = make_double2(t0r, trr);
+            if (pass(a0r, arr)) {
+                double t0r, trr;
+                lanes_tree_sum2(a0r, arr, lane, sm[gi], t0r, trr, gsync);
+                if (lane == 0) reinterpret_cast<double2 *>(S.part + 2 * (size_t)S.nchunks)[lc] = make_double2(t0r, trr);
+            }
+            if (RES) break;
         }
-        if (!(ok = grid_sync(bar, target, &s_ok))) break;
+        grid_arrive(bar, target);
+        // x += alpha y + w z (no other block reads x)
+        for (int c = cbegin; c < A.total_chunks; c += gstride) {
+            const int si = sys_of_chunk(A, c);
+            if (!state_active(sst[si])) continue;
+            const KSys &S = A.sys[si];
+            const int r0 = (c - S.chunk_begin) * CH + lane0;
+            const double alpha = sst[si].alpha, w = sst[si].w;
+#pragma unroll
+            for (int m0 = 0; m0 < RP; m0 += BATCH) {
+                double z[BATCH], y[BATCH], x[BATCH];
+#pragma unroll
+                for (int m = 0; m < BATCH; ++m) {
+                    const int row = r0 + (m0 + m) * LANES;
+                    z[m] = S.z[row];
+                    y[m] = S.y[row];
+                    x[m] = S.x[row];
+                }
+#pragma unroll
+                for (int m = 0; m < BATCH; ++m)  // rows >= n of x are padding; they receive values computed from zeros
+                    S.x[r0 + (m0 + m) * LANES] = __fma_rn(w, z[m], __fma_rn(alpha, y[m], x[m]));
+            }
+            if (RES) break;
+        }
+        if (!(ok = grid_wait(bar, target, &s_ok))) break;
         for (int q = gi; q < A.nsys; q += LOOP_GROUPS) {
             if (!state_active(sst[q])) continue;
             const KSys &S = A.sys[q];
@@ -729,33 +823,40 @@ template <int CAP>
 cudaError_t launch_krylov_loop(const KSetArgT<CAP> &A, GridBar *bar, LoopProf *prof, int max_iters,
                                cudaStream_t st, int share) {
     if (A.total_chunks <= 0 || max_iters <= 0) return cudaSuccess;
+    // the kernels in the order of their chunks per block; one block of 1024
+    // threads per SM each
+    struct Kernel {
+        const void *fn;
+        size_t smem;
+        int chunks_per_block;  // at most (0: any number)
+    };
+    static const Kernel kernels[] = {{(const void *)k_kr_chunk<CAP>, kChunkSmemBytes, 1},
+                                     {(const void *)k_kr_loop<CAP, 4>, kNbrSmemBytes<4>, LOOP_GROUPS / 4},
+                                     {(const void *)k_kr_loop<CAP, 2>, kNbrSmemBytes<2>, LOOP_GROUPS / 2},
+                                     {(const void *)k_kr_loop<CAP, 1>, kNbrSmemBytes<1>, LOOP_GROUPS},
+                                     {(const void *)k_kr_loop<CAP, 0>, 0, 0}};
     static std::atomic<bool> ready{false};
-    const void *one = (const void *)k_kr_chunk<CAP>, *res = (const void *)k_kr_loop<CAP, true>,
-               *many = (const void *)k_kr_loop<CAP, false>;
+    cudaError_t e = cudaSuccess;
     if (!ready.load()) {
-        cudaError_t e = cudaFuncSetAttribute(one, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChunkSmemBytes);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(res, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kNbrSmemBytes);
-        if (e != cudaSuccess) return e;
-        for (const void *fn : {one, res, many}) {  // one block of 1024 threads per SM
+        for (const Kernel &k : kernels) {
+            if (k.smem) e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
+            if (e != cudaSuccess) return e;
             int occ = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, LOOP_THREADS,
-                                                              fn == one ? kChunkSmemBytes : fn == res ? kNbrSmemBytes : 0);
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k.fn, LOOP_THREADS, k.smem);
             if (e != cudaSuccess) return e;
             if (occ <= 0) return cudaErrorLaunchOutOfResources;
         }
         ready = true;
     }
-    cudaError_t e = reset_grid_bar(bar, st);
+    e = reset_grid_bar(bar, st);
     if (e != cudaSuccess) return e;
     KSetArgT<CAP> a = A;
     void *args[] = {&a, &bar, &prof, &max_iters};
     count_launches(1);
-    if (A.one_per_block) return cudaLaunchCooperativeKernel(one, A.total_chunks, CH, args, kChunkSmemBytes, st);
-    const int grid = krylov_loop_grid<CAP>(A.total_chunks, 1, share);
-    if (A.total_chunks <= grid * LOOP_GROUPS)
-        return cudaLaunchCooperativeKernel(res, grid, LOOP_THREADS, args, kNbrSmemBytes, st);
-    return cudaLaunchCooperativeKernel(many, grid, LOOP_THREADS, args, 0, st);
+    const int grid = A.one_per_block ? A.total_chunks : krylov_loop_grid<CAP>(A.total_chunks, 1, share);
+    int k = A.one_per_block ? 0 : 1;
+    while (!A.one_per_block && kernels[k].chunks_per_block && A.total_chunks > grid * kernels[k].chunks_per_block) ++k;
+    return cudaLaunchCooperativeKernel(kernels[k].fn, grid, LOOP_THREADS, args, kernels[k].smem, st);
 }
 
 template <int CAP>

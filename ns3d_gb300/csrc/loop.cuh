@@ -34,12 +34,20 @@ __device__ __forceinline__ void red_release_add(unsigned int *p, unsigned int v)
 // The block barrier orders every thread's writes before thread 0's release
 // arrival; thread 0's acquire poll plus the closing block barrier order the
 // block's later reads after every other block's arrival.
-__device__ __forceinline__ bool grid_sync(GridBar *bar, unsigned int &target, int *s_ok) {
+// the first half of the barrier: every thread of the block has arrived
+__device__ __forceinline__ void grid_arrive(GridBar *bar, unsigned int &target) {
     __syncthreads();
     if (threadIdx.x == 0) {
-        int ok = 1;
         target += gridDim.x;
         red_release_add(&bar->count, 1u);
+    }
+}
+
+// The second half.  Between the two a block may work on what no other block
+// reads or writes.
+__device__ __forceinline__ bool grid_wait(GridBar *bar, unsigned int target, int *s_ok) {
+    if (threadIdx.x == 0) {
+        int ok = 1;
         if ((int)(ld_acquire(&bar->count) - target) < 0) {
             const unsigned long long t0 = global_ns();
             const unsigned long long lim = bar->limit_ns ? bar->limit_ns : kBarrierLimitNs;
@@ -56,6 +64,11 @@ __device__ __forceinline__ bool grid_sync(GridBar *bar, unsigned int &target, in
     }
     __syncthreads();
     return *s_ok != 0;
+}
+
+__device__ __forceinline__ bool grid_sync(GridBar *bar, unsigned int &target, int *s_ok) {
+    grid_arrive(bar, target);
+    return grid_wait(bar, target, s_ok);
 }
 
 // The arrival target a launch starts from (thread 0 keeps it): 0, or the

@@ -1,5 +1,5 @@
-"""The one-chunk-per-block BiCGSTAB loop at the edges of its range, bit for bit
-against the CPU oracle: one row over a chunk, the chunk counts at which its
+"""The FP64 BiCGSTAB loops at the edges of their ranges, bit for bit
+against the CPU oracle.  One chunk per block: one row over a chunk, the chunk counts at which its
 reduction trees lose or gain a level (32/33, 64/65, 128/129 chunks), the
 largest set it takes on a 152-SM GPU and the first one it leaves to the
 several-chunks-per-block loop, rows whose west or east entry directly precedes
@@ -38,7 +38,13 @@ def _systems(lib, img, sys):
     return x, (info.iterations, info.info, info.error), (coef, nbr)
 
 
-@pytest.mark.parametrize("shape", BOXES)
+# the largest set and the first one beyond it of the loops with several chunks
+# per block: two chunks (four groups each), four, eight, any number on 152 SMs;
+# and columns more than 65535 rows away
+SEVERAL = [(304, 32, 32), (305, 32, 32), (608, 32, 32), (609, 32, 32), (1216, 32, 32), (1217, 32, 32), (3, 264, 256)]
+
+
+@pytest.mark.parametrize("shape", BOXES + SEVERAL)
 def test_boxes_bitwise(gpulib, oracle, shape):
     img = np.zeros(shape, np.uint8)
     for sys in (capi.SYS_P, capi.SYS_U):
