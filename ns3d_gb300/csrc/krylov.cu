@@ -35,6 +35,77 @@
 
 namespace ns3d {
 
+// ---- tensor memory as a resident store --------------------------------------
+// The 256 KB of tensor memory of an SM lie idle in this solver.  The loop
+// kernel keeps matrix coefficients there for a launch: a warp reaches the 32
+// lanes of its rank in the warpgroup, a group of 128 threads has 64 of the 512
+// columns, so a thread owns 64 words, and reads back what it wrote itself.
+// A row's first NT coefficients take 2 NT words, padded to TMEM_ROW<NT>.
+// With four of seven coefficients there a row's data outside the SM shrink
+// from 136 to 104 bytes, and 1.05 M rows fit the L2: 79.5 -> 72.8 us per
+// iteration (0.73 M rows 58.1 -> 55.8).  With several chunks per group only
+// the first could live there: 3.55 M rows 250 -> 253 us, so not used.
+constexpr int TMEM_COLUMNS = 512;
+template <int NT>
+constexpr int TMEM_ROW = NT > 4 ? 16 : 8;
+
+// one warp of the block; *base (shared) receives the address
+__device__ __forceinline__ void tmem_alloc(unsigned int *base) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     (unsigned int)__cvta_generic_to_shared(base)),
+                 "n"(TMEM_COLUMNS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+// the same warp, after every other warp's last access
+__device__ __forceinline__ void tmem_free(unsigned int base) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "n"(TMEM_COLUMNS) : "memory");
+}
+// NT doubles to / from the words at taddr (whole warps)
+template <int NT>
+__device__ __forceinline__ void tmem_store(unsigned int taddr, const double *c) {
+    unsigned int w[16];
+    __syncwarp();  // .aligned: the whole warp issues the instruction
+#pragma unroll
+    for (int d = 0; d < 8; ++d) {
+        w[2 * d] = d < NT ? (unsigned int)__double2loint(c[d < NT ? d : 0]) : 0u;
+        w[2 * d + 1] = d < NT ? (unsigned int)__double2hiint(c[d < NT ? d : 0]) : 0u;
+    }
+    if constexpr (NT > 4)
+        asm volatile(
+            "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+            "%14, %15, %16};" ::"r"(taddr),
+            "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]),
+            "r"(w[9]), "r"(w[10]), "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15])
+            : "memory");
+    else if constexpr (NT > 0)
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
+                     "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                     : "memory");
+}
+template <int NT>
+__device__ __forceinline__ void tmem_load(unsigned int taddr, double *c) {
+    unsigned int w[16];
+    if (NT > 0) __syncwarp();
+    if constexpr (NT > 4)
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+            "%15}, [%16];\n tcgen05.wait::ld.sync.aligned;"
+            : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]),
+              "=r"(w[8]), "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15])
+            : "r"(taddr)
+            : "memory");
+    else if constexpr (NT > 0)
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+            " tcgen05.wait::ld.sync.aligned;"
+            : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+            : "r"(taddr)
+            : "memory");
+#pragma unroll
+    for (int d = 0; d < NT; ++d) c[d] = __hiloint2double((int)w[2 * d + 1], (int)w[2 * d]);
+}
+
 struct Row4 {  // a thread's RPL rows
     double v[RPL];
 };
@@ -58,10 +129,12 @@ __device__ __forceinline__ void st4(double *p, const Row4 &r) {
 // two rare orders (W directly before the row, E directly after it) are taken
 // only by warps that contain such a row.
 // The neighbour columns come from `nb` (nb[k * stride], k = slot - 1): the
-// system's table in global memory, or a chunk's copy in shared memory.
-template <class Stride>
+// system's table in global memory, or a chunk's copy in shared memory.  The
+// first NT coefficients (slots P, W, E, ...) come from the tensor memory of
+// the SM (taddr; tmem_row below), the others from memory.
+template <int NT, class Stride>
 __device__ __forceinline__ double spmv_row_nb(const KSys &S, int row, const double *__restrict__ x, const int *nb,
-                                              Stride stride) {
+                                              Stride stride, unsigned int taddr = 0) {
     const size_t np = (size_t)S.npad;
     const double *cf = S.coef + row;
     const int nW = nb[0 * stride], nE = nb[1 * stride], nS = nb[2 * stride], nN = nb[3 * stride],
@@ -69,8 +142,11 @@ __device__ __forceinline__ double spmv_row_nb(const KSys &S, int row, const doub
     const double xP = x[row];
     const double xW = x[nW >= 0 ? nW : row], xE = x[nE >= 0 ? nE : row], xS = x[nS >= 0 ? nS : row];
     const double xN = x[nN >= 0 ? nN : row], xB = x[nB >= 0 ? nB : row], xT = x[nT >= 0 ? nT : row];
-    const double cP = ro(cf), cW = ro(cf + 1 * np), cE = ro(cf + 2 * np), cS = ro(cf + 3 * np),
-                 cN = ro(cf + 4 * np), cB = ro(cf + 5 * np), cT = ro(cf + 6 * np);
+    double cc[7];
+#pragma unroll
+    for (int d = NT; d < 7; ++d) cc[d] = ro(cf + d * np);
+    tmem_load<NT>(taddr, cc);
+    const double cP = cc[0], cW = cc[1], cE = cc[2], cS = cc[3], cN = cc[4], cB = cc[5], cT = cc[6];
     const bool wlate = nW >= 0 && nW == row - 1;
     const bool eearly = nE >= 0 && nE == row + 1;
     double acc = 0.0;
@@ -97,21 +173,22 @@ __device__ __forceinline__ double spmv_row_nb(const KSys &S, int row, const doub
 }
 
 __device__ __forceinline__ double spmv_row(const KSys &S, int row, const double *__restrict__ x) {
-    return spmv_row_nb(S, row, x, S.nbr + row, (size_t)S.npad);
+    return spmv_row_nb<0>(S, row, x, S.nbr + row, (size_t)S.npad);
 }
 
 // the same from a chunk's 16-bit distances (nb16[k * CH]: |column - row| of
 // slot k + 1, 0 = no entry): W, S and B columns lie before the row, E, N and
 // T columns after it
+template <int NT>
 __device__ __forceinline__ double spmv_row_16(const KSys &S, int row, const double *__restrict__ x,
-                                              const unsigned short *nb16) {
+                                              const unsigned short *nb16, unsigned int taddr) {
     int nb[6];
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
         const int d = nb16[k * CH];
         nb[k] = d == 0 ? -1 : row + ((k & 1) ? d : -d);
     }
-    return spmv_row_nb(S, row, x, nb, 1);
+    return spmv_row_nb<NT>(S, row, x, nb, 1, taddr);
 }
 
 // y = A x for the thread's rows (rows >= n give garbage that callers mask)
@@ -330,10 +407,14 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
     static_assert(CAP <= LOOP_THREADS, "one thread copies each system's state");
     constexpr bool RES = GPC > 0;
     constexpr int PARTS = RES ? GPC : 1, RP = RPL / PARTS, BATCH = RP < 4 ? RP : 4;
+    // a row's coefficients in tensor memory: a thread's 64 words hold RP rows
+    constexpr int NT = RES ? (RP < 8 ? 7 : 4) : 0;
+    static_assert(!RES || RP * TMEM_ROW<NT> <= TMEM_COLUMNS / LOOP_GROUPS, "a thread's words");
     __shared__ KState sst[CAP];
     __shared__ double sm[LOOP_GROUPS][16];
     __shared__ double s_acc[PARTS > 1 ? LOOP_GROUPS : 1][2][LANES];  // the lanes' sums on their way
     __shared__ int s_ok;
+    __shared__ unsigned int s_tmem;
     extern __shared__ unsigned short s_nbr_all[];  // RES: [LOOP_GROUPS / GPC][6][CH]
     const int gi = threadIdx.x / LANES, lane = threadIdx.x % LANES, part = gi % PARTS;
     const GroupSync gsync{gi + 1};
@@ -367,7 +448,24 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
         far = any != 0;
     }
     unsigned int target = grid_sync_start(bar);  // the counter is zeroed before every launch
-    __syncthreads();  // the scalar copies in sst are complete
+    if (RES && threadIdx.x < 32) tmem_alloc(&s_tmem);
+    if (RES) asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();  // the scalar copies in sst are complete, the tensor memory is allocated
+    if (RES) asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // the words of the thread's rows
+    const unsigned int taddr = RES ? s_tmem + ((unsigned int)(lane & ~31) << 16) + gi * (TMEM_COLUMNS / LOOP_GROUPS) : 0;
+    if (RES && cbegin < A.total_chunks) {
+        const KSys &S = A.sys[sys_of_chunk(A, cbegin)];
+        const int row0 = (cbegin - S.chunk_begin) * CH + lane0;
+#pragma unroll 1
+        for (int m = 0; m < RP; ++m) {
+            double c[7];
+#pragma unroll
+            for (int d = 0; d < NT; ++d) c[d] = ro(S.coef + (size_t)d * S.npad + row0 + m * LANES);
+            tmem_store<NT>(taddr + m * TMEM_ROW<NT>, c);
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    }
     // phase times of block 0 (thread 0), kept in shared memory
     __shared__ unsigned long long s_tp[6];
     const bool timing = prof != nullptr && blockIdx.x == 0 && threadIdx.x == 0;
@@ -382,9 +480,10 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
             s_tp[5] = t;
         }
     };
+    // row m of the thread
     auto row_product = [&](const KSys &S, int row, int m, const double *x) {
-        if (RES && !far) return spmv_row_16(S, row, x, s_nbr + m * LANES);
-        return spmv_row(S, row, x);
+        if (RES && !far) return spmv_row_16<NT>(S, row, x, s_nbr + m * LANES, taddr + m * TMEM_ROW<NT>);
+        return spmv_row_nb<NT>(S, row, x, S.nbr + row, (size_t)S.npad, taddr + m * TMEM_ROW<NT>);
     };
     // before a group adds to its chunk's lane sums: take them from the group
     // before it (named barrier 8 + gi: that group arrives, this one waits)
@@ -669,6 +768,14 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
         if (!any_active || any_paused) {
             ++it;
             break;
+        }
+    }
+    if (RES) {
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            tmem_free(s_tmem);
         }
     }
     if (blockIdx.x == 0 && threadIdx.x < A.nsys) {
