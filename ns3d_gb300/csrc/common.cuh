@@ -147,19 +147,19 @@ __device__ __forceinline__ double lane_dot(const double *a, const double *b, int
 // instead of one per partial.
 constexpr int FINAL_BATCH = 8;
 
-template <class Sync>
+template <int BATCH = FINAL_BATCH, class Sync>
 __device__ __forceinline__ double lanes_final_sum(const double *part, int n, int stride, int lane, double *sm,
                                                   Sync sync) {
     double a = 0.0;
-    for (int base = lane; base < n; base += FINAL_BATCH * LANES) {
-        double v[FINAL_BATCH];
+    for (int base = lane; base < n; base += BATCH * LANES) {
+        double v[BATCH];
 #pragma unroll
-        for (int k = 0; k < FINAL_BATCH; ++k) {
+        for (int k = 0; k < BATCH; ++k) {
             const int i = base + k * LANES;
             v[k] = (i < n) ? __ldcg(part + (size_t)i * stride) : 0.0;
         }
 #pragma unroll
-        for (int k = 0; k < FINAL_BATCH; ++k)
+        for (int k = 0; k < BATCH; ++k)
             if (base + k * LANES < n) a = a + v[k];
     }
     return lanes_tree_sum<double>(a, lane, sm, sync);

@@ -130,13 +130,14 @@ __global__ void __launch_bounds__(HB_THREADS)
 }
 
 __global__ void k_hb_members(const int *__restrict__ cell, int n, CellBox f, const unsigned int *__restrict__ mask,
-                             const int *__restrict__ index, const int *__restrict__ mstart, int *__restrict__ agg,
+                             const int *__restrict__ index, const int *__restrict__ mstart, int *__restrict__ pos,
                              int *__restrict__ members) {
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
         int oct;
         const int b = block_of(cell[r], f, oct), I = index[b];
-        agg[r] = I;
-        members[mstart[I] + __popc(mask[b] & ((1u << oct) - 1u))] = r;
+        const int rank = __popc(mask[b] & ((1u << oct) - 1u));
+        pos[r] = 8 * I + rank;
+        members[mstart[I] + rank] = r;
     }
 }
 
@@ -189,16 +190,17 @@ void build_hierarchy(DevSys &S, cudaStream_t st) {
         L.n = nc;
         L.npad = (nc + 255) / 256 * 256;
         L.nbr.alloc((size_t)6 * L.npad, st);
-        L.agg.alloc((size_t)nf, st);
+        L.pos.alloc((size_t)nf, st);
         L.mstart.alloc((size_t)nc + 1, st);
         L.members.alloc((size_t)nf, st);
         DBuf<int> &ccell = cells[flip];
         ccell.alloc((size_t)nc, st);
         count_launches(3);
         k_hb_number<<<ntiles, HB_THREADS, 0, st>>>(mask.p, nb, tiles.p, ntiles, index.p, ccell.p, L.mstart.p);
-        k_hb_members<<<hb_grid(nf), 256, 0, st>>>(cell, nf, box, mask.p, index.p, L.mstart.p, L.agg.p, L.members.p);
+        k_hb_members<<<hb_grid(nf), 256, 0, st>>>(cell, nf, box, mask.p, index.p, L.mstart.p, L.pos.p, L.members.p);
         k_hb_nbr<<<hb_grid(L.npad), 256, 0, st>>>(ccell.p, nc, L.npad, cbox, index.p, L.nbr.p);
         L.coef.alloc_zero((size_t)7 * L.npad, st);
+        L.t8.alloc_zero((size_t)8 * L.npad, st);
         for (DBuf<float> *b : {&L.invdiag, &L.x, &L.b, &L.t, &L.xo}) b->alloc_zero((size_t)L.npad, st);
         cell = ccell.p;
         box = cbox;

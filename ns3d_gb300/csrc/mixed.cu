@@ -18,6 +18,7 @@
 // from the new FP64 residual.  iterations() reports the inner iterations.
 #include <atomic>
 #include <cfloat>
+#include <type_traits>
 
 #include "device.cuh"
 #include "kernels.h"
@@ -316,7 +317,7 @@ struct MGView {
 };
 
 // level k of the hierarchy of S (level 0: the FP32 system, right-hand side b0,
-// Jacobi start S.p2, result x0, scratch S.t)
+// Jacobi start S.p2, result x0)
 __device__ __forceinline__ MGView mg_level(const MSys &S, int k, const float *b0, float *x0) {
     MGView L;
     if (k == 0) {
@@ -364,21 +365,47 @@ __device__ __forceinline__ float mg_spmv(const MGView &L, int row, const float *
     return mg_spmv_fn(L, row, [&](int c) { return x[c]; });
 }
 
-// The passes of a V-cycle, one row each.  Down: the residual t of the
-// level's Jacobi start x, then the restriction of t with the next level's
-// Jacobi start.  Up: x with the coarse correction cx added on the fly and one
-// damped Jacobi sweep, into xo (the neighbours still read x).
-__device__ __forceinline__ void mg_down(const MGView &L, int r) { L.t[r] = L.b[r] - mg_spmv(L, r, L.x); }
-__device__ __forceinline__ void mg_restrict(const MGLevel &C, const float *t, float w, int I) {
+// The passes of a V-cycle, one row each.  Down: the residual of the level's
+// Jacobi start x, stored at its place among the coarse row's up to eight
+// members (C.t8, so that the restriction reads 32 contiguous bytes instead of
+// a member list and scattered residuals), then the restriction with the next
+// level's Jacobi start.  Up: x with the coarse correction cx added on the fly
+// and one damped Jacobi sweep, into xo (the neighbours still read x).
+__device__ __forceinline__ float mg_down(const MGView &L, int r) { return L.b[r] - mg_spmv(L, r, L.x); }
+// sum over a coarse row's members in ascending order; the unused places add +0
+// to a sum that starts at +0, which changes nothing
+__device__ __forceinline__ float mg_sum8(const float *t8, int I) {
+    const float4 a = __ldcg(reinterpret_cast<const float4 *>(t8) + 2 * I),
+                 b = __ldcg(reinterpret_cast<const float4 *>(t8) + 2 * I + 1);
     float acc = 0.0f;
-    for (int q = C.mstart[I]; q < C.mstart[I + 1]; ++q) acc += t[C.members[q]];
+    for (float v : {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w}) acc += v;
+    return acc;
+}
+__device__ __forceinline__ void mg_restrict(const MGLevel &C, float w, int I) {
+    const float acc = mg_sum8(C.t8, I);
     C.b[I] = acc;
     C.x[I] = w * C.invdiag[I] * acc;
 }
-__device__ __forceinline__ void mg_up(const MGView &L, const int *agg, const float *cx, float w, int r) {
-    const float x = L.x[r] + cx[ro(agg + r)];
-    const float t = L.b[r] - mg_spmv_fn(L, r, [&](int c) { return c == r ? x : L.x[c] + cx[ro(agg + c)]; });
-    L.xo[r] = x + w * L.invdiag[r] * t;
+__device__ __forceinline__ float mg_up(const MGView &L, const int *pos, const float *cx, float w, int r) {
+    const float x = L.x[r] + cx[ro(pos + r) >> 3];
+    const float t = L.b[r] - mg_spmv_fn(L, r, [&](int c) { return c == r ? x : L.x[c] + cx[ro(pos + c) >> 3]; });
+    return x + w * L.invdiag[r] * t;
+}
+// store(r, value(r)) for the rows r < n of the calling thread, two at a time
+// when it has that many (the loads of both in flight)
+template <class Value, class Store>
+__device__ __forceinline__ void mg_pass(int n, int gtid, int gth, Value value, Store store) {
+    if (n <= gth) {
+        if (gtid < n) store(gtid, value(gtid));
+        return;
+    }
+    for (int r = gtid; r < n; r += 2 * gth) {
+        const bool two = n - r > gth;
+        const int q = two ? r + gth : r;
+        const float a = value(r), b = value(q);
+        store(r, a);
+        if (two) store(q, b);
+    }
 }
 
 // Jacobi sweeps on the coarsest level by the calling block: x = w D^-1 b,
@@ -451,7 +478,7 @@ __device__ void mg_tail_load(const MGSet &G, float *mem, TailLevels &T) {
             for (int r = threadIdx.x; r <= L.n; r += blockDim.x) L.mstart[r] = ro(C.mstart + r);
             for (int r = threadIdx.x; r < nf; r += blockDim.x) {
                 L.members[r] = ro(C.members + r);
-                L.agg[r] = ro(C.agg + r);
+                L.agg[r] = ro(C.pos + r) >> 3;
             }
         }
     }
@@ -467,19 +494,20 @@ __device__ __forceinline__ float tail_spmv(const TailLevel &L, int r, F xf) {
 }
 
 // One V-cycle of the tail by the calling block, right-hand side restricted
-// from the residual t of the level above; returns the result.
-__device__ const float *mg_tail(const MGSet &G, TailLevels &T, const float *t) {
+// from the residual of the level above; returns the result.
+__device__ const float *mg_tail(const MGSet &G, TailLevels &T) {
     const int K = G.nlev, tid = threadIdx.x, nth = blockDim.x;
     const float w = G.omega;
     for (int k = G.tail; k <= K; ++k) {
         const TailLevel &L = T[k];
-        const MGLevel &C = G.lev[k];
-        const bool first = k == G.tail;
-        const int *mstart = first ? C.mstart : L.mstart, *members = first ? C.members : L.members;
-        const float *src = first ? t : T[k - 1].t;
         for (int I = tid; I < L.n; I += nth) {
             float acc = 0.0f;
-            for (int q = mstart[I]; q < mstart[I + 1]; ++q) acc += first ? __ldcg(src + members[q]) : src[members[q]];
+            if (k == G.tail) {
+                acc = mg_sum8(G.lev[k].t8, I);
+            } else {
+                const float *src = T[k - 1].t;
+                for (int q = L.mstart[I]; q < L.mstart[I + 1]; ++q) acc += src[L.members[q]];
+            }
             L.b[I] = acc;
             L.x[I] = w * L.invdiag[I] * acc;
         }
@@ -562,7 +590,7 @@ __device__ const float *mg_tail(const MGSet &G, TailLevels &T, const float *t) {
 // coarse row, measured 3-8% slower: it walks the fine rows out of order.)
 // With the tail in shared memory an iteration of a 205 K-row system (five
 // levels) has 21 grid barriers instead of 53 with three passes each way and
-// every level in the grid.
+// every level in the grid: 117 -> 78 us.
 __device__ bool mg_apply(const MSys &S, const float *b0, float *x0, TailLevels &T, GridBar *bar, unsigned int &target,
                          int *s_ok) {
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -572,14 +600,14 @@ __device__ bool mg_apply(const MSys &S, const float *b0, float *x0, TailLevels &
     const float *cx = S.mg.lev[K].x;  // the coarse correction: the coarsest level's x, the other levels' xo
     for (int k = 0; k < K; ++k) {
         const MGView L = mg_level(S, k, b0, x0);
-        for (int r = gtid; r < L.n; r += gth) mg_down(L, r);
+        const MGLevel &C = S.mg.lev[k + 1];
+        mg_pass(L.n, gtid, gth, [&](int r) { return mg_down(L, r); }, [&](int r, float v) { C.t8[ro(C.pos + r)] = v; });
         if (!grid_sync(bar, target, s_ok)) return false;
         if (k + 1 == tail) {
-            cx = mg_tail(S.mg, T, L.t);
+            cx = mg_tail(S.mg, T);
             break;
         }
-        const MGLevel &C = S.mg.lev[k + 1];
-        for (int I = gtid; I < C.n; I += gth) mg_restrict(C, L.t, w, I);
+        for (int I = gtid; I < C.n; I += gth) mg_restrict(C, w, I);
         if (!grid_sync(bar, target, s_ok)) return false;
     }
     if (tail > K) {
@@ -588,8 +616,8 @@ __device__ bool mg_apply(const MSys &S, const float *b0, float *x0, TailLevels &
     }
     for (int k = min(K, tail) - 1; k >= 0; --k) {
         const MGView L = mg_level(S, k, b0, x0);
-        const int *agg = S.mg.lev[k + 1].agg;
-        for (int r = gtid; r < L.n; r += gth) mg_up(L, agg, cx, w, r);
+        const int *pos = S.mg.lev[k + 1].pos;
+        mg_pass(L.n, gtid, gth, [&](int r) { return mg_up(L, pos, cx, w, r); }, [&](int r, float v) { L.xo[r] = v; });
         if (!grid_sync(bar, target, s_ok)) return false;
         cx = L.xo;
     }
@@ -638,10 +666,13 @@ __device__ bool mg_apply_set(const MSetArgT<CAP> &A, const KState *sst, const in
     for (int k = 0; k < kmax; ++k) {
         auto part = [&](int q) { return on(q) && k < A.sys[q].mg.nlev; };
         mg_rows(A, part, [&](int q) { return k == 0 ? A.sys[q].n : A.sys[q].mg.lev[k].n; },
-                [&](int q, int r) { mg_down(lvl(q, k), r); });
+                [&](int q, int r) {
+                    const MGLevel &C = A.sys[q].mg.lev[k + 1];
+                    C.t8[ro(C.pos + r)] = mg_down(lvl(q, k), r);
+                });
         if (!grid_sync(bar, target, s_ok)) return false;
         mg_rows(A, part, [&](int q) { return A.sys[q].mg.lev[k + 1].n; },
-                [&](int q, int I) { mg_restrict(A.sys[q].mg.lev[k + 1], lvl(q, k).t, A.sys[q].mg.omega, I); });
+                [&](int q, int I) { mg_restrict(A.sys[q].mg.lev[k + 1], A.sys[q].mg.omega, I); });
         if (!grid_sync(bar, target, s_ok)) return false;
     }
     {
@@ -658,7 +689,8 @@ __device__ bool mg_apply_set(const MSetArgT<CAP> &A, const KState *sst, const in
         auto rows = [&](int q) { return k == 0 ? A.sys[q].n : A.sys[q].mg.lev[k].n; };
         mg_rows(A, part, rows, [&](int q, int r) {
             const MGLevel &C = A.sys[q].mg.lev[k + 1];
-            mg_up(lvl(q, k), C.agg, k + 1 == A.sys[q].mg.nlev ? C.x : C.xo, A.sys[q].mg.omega, r);
+            const MGView L = lvl(q, k);
+            L.xo[r] = mg_up(L, C.pos, k + 1 == A.sys[q].mg.nlev ? C.x : C.xo, A.sys[q].mg.omega, r);
         });
         if (!grid_sync(bar, target, s_ok)) return false;
     }
@@ -701,7 +733,7 @@ __global__ void k_mg_galerkin(int npad_f, const int *__restrict__ nbr_f, const f
                 const int col = nbr_f[(size_t)dir * npad_f + m];
                 if (col < 0) continue;
                 const float a = coef_f[(size_t)(dir + 1) * npad_f + m];
-                if (C.agg[col] == I) d += a;
+                if (C.pos[col] >> 3 == I) d += a;
                 else off[dir] += a;
             }
         }
@@ -728,6 +760,38 @@ __global__ void k_mg_galerkin(int npad_f, const int *__restrict__ nbr_f, const f
 // block keeps a copy of the inner state; the kernel ends when every inner
 // solve of the round is done or after `max_iters` iterations.
 
+struct Pair4 {  // four elements of one or two result vectors
+    float *pa, *pb;
+    float4 a, b;
+};
+__device__ __forceinline__ float4 at4(const float *p, int i) { return reinterpret_cast<const float4 *>(p)[i]; }
+template <class F>
+__device__ __forceinline__ float4 each4(F f, float4 a, float4 b, float4 c) {
+    return make_float4(f(a.x, b.x, c.x), f(a.y, b.y, c.y), f(a.z, b.z, c.z), f(a.w, b.w, c.w));
+}
+
+// H work units of a group, taken together so that the loads of all are in
+// flight: one beyond the end (or an inactive one) falls back to rows whose
+// results are then not stored.
+template <int CAP, int H>
+struct UnitPair {
+    int si[H], lc[H];
+    bool on[H];
+    __device__ __forceinline__ UnitPair(const MSetArgT<CAP> &A, const KState *sst, const int *sdc, int u, int gstride,
+                                        int total_units) {
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+            const int v = u + h * gstride;
+            on[h] = v < total_units;
+            si[h] = msys_of_chunk(A, (on[h] ? v : u) / MSUB);
+            lc[h] = (on[h] ? v : u) - A.sys[si[h]].chunk_begin * MSUB;
+            on[h] = on[h] && inner_active(sst[si[h]], sdc[si[h]]);
+        }
+    }
+    __device__ __forceinline__ bool none() const { return !on[0] && !on[H - 1]; }
+    __device__ __forceinline__ const MSys &S(const MSetArgT<CAP> &A, int h) const { return A.sys[si[h]]; }
+};
+
 template <bool FUSED, int CAP>
 __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
     k_m32_loop(const __grid_constant__ MSetArgT<CAP> A, GridBar *bar, int max_iters) {
@@ -751,6 +815,44 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
         if (A.sys[0].mg.nlev > 0 && A.sys[0].mg.tail <= A.sys[0].mg.nlev) mg_tail_load(A.sys[0].mg, tail_mem, s_tail);
     unsigned int target = grid_sync_start(bar);
     __syncthreads();
+    __shared__ double s_sum[CAP][2];
+    // two reductions (pairs at 2 n x of the partials) of every active system
+    // into s_sum, one group each
+    auto two_sums = [&](int region) {
+#pragma unroll 1
+        for (int task = gi; task < 2 * A.nsys; task += LOOP_GROUPS) {
+            const int q = task >> 1, j = task & 1;
+            if (!inner_active(sst[q], sdc[q])) continue;
+            const MSys &S = A.sys[q];
+            const double t = lanes_final_sum<16>(S.part + region * (size_t)S.nchunks * MSUB + j, S.nchunks * MSUB, 2, lane,
+                                                 sm[gi], gsync);
+            if (lane == 0) s_sum[q][j] = t;
+        }
+        __syncthreads();
+    };
+    // An element-wise phase: op(system index, system, i) computes elements
+    // 4 i .. 4 i + 3 of one or two result vectors.  A group takes whole chunks,
+    // a lane two float4 of each vector at once: with one row in flight per
+    // thread K1, K3 and K5 took 30, 28 and 58 us at 3.6 M rows, now 11, 9 and 32.
+    auto stream_chunks = [&](auto op) {
+        for (int c = cbegin; c < A.total_chunks; c += gstride) {
+            const int si = msys_of_chunk(A, c);
+            if (!inner_active(sst[si], sdc[si])) continue;
+            const MSys &S = A.sys[si];
+            const int i = (c - S.chunk_begin) * (CH / 4) + lane;
+            const Pair4 e0 = op(si, S, i), e1 = op(si, S, i + LANES);
+            reinterpret_cast<float4 *>(e0.pa)[i] = e0.a;
+            if (e0.pb) reinterpret_cast<float4 *>(e0.pb)[i] = e0.b;
+            reinterpret_cast<float4 *>(e1.pa)[i + LANES] = e1.a;
+            if (e1.pb) reinterpret_cast<float4 *>(e1.pb)[i + LANES] = e1.b;
+        }
+    };
+    static_assert(CH == 8 * LANES, "two float4 a lane");
+    // a phase over work units, two at a time when a group has that many
+    auto unit_phase = [&](auto run) {
+        if (total_units > gstride) run(std::integral_constant<int, 2>());
+        else run(std::integral_constant<int, 1>());
+    };
     int it = 0;
     for (; it < max_iters; ++it) {
         if constexpr (FUSED) {
@@ -873,133 +975,169 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
                     mg_on = mg_on || (A.sys[q].mg.nlev > 0 && inner_active(sst[q], sdc[q]));
             }
             // p = r + beta (p - w v); y = D^-1 p
-            for (int u = cbegin; u < total_units; u += gstride) {
-                const int si = msys_of_chunk(A, u / MSUB);
-                if (!inner_active(sst[si], sdc[si])) continue;
-                const MSys &S = A.sys[si];
-                const int r0 = (u - S.chunk_begin * MSUB) * MUNIT + lane;
+            stream_chunks([&](int si, const MSys &S, int i) {
                 const float beta = (float)sst[si].beta, w = (float)sst[si].w;
-    #pragma unroll
-                for (int m = 0; m < MRPL; ++m) {
-                    const int row = r0 + m * LANES;
-                    const float p = __fmaf_rn(beta, __fmaf_rn(-w, S.v[row], S.p[row]), S.r[row]);
-                    S.p[row] = p;
-                    // a system with a hierarchy: the V-cycle's start w D^-1 p
-                    if (S.mg.nlev > 0) S.p2[row] = S.mg.omega * S.invdiag32[row] * p;
-                    else S.y[row] = S.invdiag32[row] * p;
-                }
-            }
+                float4 p = at4(S.p, i);
+                const float4 v = at4(S.v, i), r = at4(S.r, i), d = at4(S.invdiag32, i);
+                // a system with a hierarchy: the V-cycle's start w D^-1 p
+                float *const out = S.mg.nlev > 0 ? S.p2 : S.y;
+                const float om = S.mg.omega;
+                const bool mg = S.mg.nlev > 0;
+                p = each4([&](float p1, float v1, float r1) { return __fmaf_rn(beta, __fmaf_rn(-w, v1, p1), r1); }, p, v, r);
+                const float4 y = each4([&](float d1, float p1, float) { return mg ? om * d1 * p1 : d1 * p1; }, d, p, p);
+                return Pair4{S.p, out, p, y};
+            });
             if (!grid_sync(bar, target, &s_ok)) break;
             // multilevel preconditioning: y = M^-1 p (replaces the Jacobi y)
             if (mg_on && !mg_precondition(A, sst, sdc, 0, s_tail, bar, target, &s_ok)) break;
             // v = A y, <r0, v>
-            for (int u = cbegin; u < total_units; u += gstride) {
-                const int si = msys_of_chunk(A, u / MSUB);
-                if (!inner_active(sst[si], sdc[si])) continue;
-                const MSys &S = A.sys[si];
-                const int lc = u - S.chunk_begin * MSUB;
-                const int r0 = lc * MUNIT + lane;
-                float a = 0.0f;
-    #pragma unroll
-                for (int m = 0; m < MRPL; ++m) {
-                    const int row = r0 + m * LANES;
-                    const float v = spmv_f32_row(S, row, S.y);
-                    S.v[row] = v;
-                    if (row < S.n) a = __fmaf_rn(S.r0[row], v, a);
+            unit_phase([&](auto units) {
+                constexpr int H = decltype(units)::value;
+                for (int u = cbegin; u < total_units; u += H * gstride) {
+                    const UnitPair<CAP, H> U(A, sst, sdc, u, gstride, total_units);
+                    if (U.none()) continue;
+                    float v[H][MRPL], q[H][MRPL], a[2] = {0.0f, 0.0f};
+#pragma unroll
+                    for (int h = 0; h < H; ++h)
+#pragma unroll
+                        for (int m = 0; m < MRPL; ++m) {
+                            const int row = U.lc[h] * MUNIT + lane + m * LANES;
+                            v[h][m] = spmv_f32_row(U.S(A, h), row, U.S(A, h).y);
+                            q[h][m] = U.S(A, h).r0[row];
+                        }
+#pragma unroll
+                    for (int h = 0; h < H; ++h)
+                        if (U.on[h])
+#pragma unroll
+                            for (int m = 0; m < MRPL; ++m) {
+                                const int row = U.lc[h] * MUNIT + lane + m * LANES;
+                                U.S(A, h).v[row] = v[h][m];
+                                if (row < U.S(A, h).n) a[h] = __fmaf_rn(q[h][m], v[h][m], a[h]);
+                            }
+                    float t[2];
+                    lanes_tree_sum2<float>(a[0], a[1], lane, reinterpret_cast<float *>(sm[gi]), t[0], t[1], gsync);
+                    if (lane == 0)
+#pragma unroll
+                        for (int h = 0; h < H; ++h)
+                            if (U.on[h]) U.S(A, h).part[4 * (size_t)U.S(A, h).nchunks * MSUB + U.lc[h]] = (double)t[h];
                 }
-                const float t = lanes_tree_sum<float>(a, lane, reinterpret_cast<float *>(sm[gi]), gsync);
-                if (lane == 0) S.part[4 * (size_t)S.nchunks * MSUB + lc] = (double)t;
-            }
+            });
             if (!grid_sync(bar, target, &s_ok)) break;
             for (int q = gi; q < A.nsys; q += LOOP_GROUPS) {
                 if (!inner_active(sst[q], sdc[q])) continue;
                 const MSys &S = A.sys[q];
-                const double d = lanes_final_sum(S.part + 4 * (size_t)S.nchunks * MSUB, S.nchunks * MSUB, 1, lane, sm[gi], gsync);
+                const double d = lanes_final_sum<16>(S.part + 4 * (size_t)S.nchunks * MSUB, S.nchunks * MSUB, 1, lane, sm[gi], gsync);
                 if (lane == 0) sst[q].alpha = sst[q].rho / d;
             }
             __syncthreads();
             // s = r - alpha v; z = D^-1 s
-            for (int u = cbegin; u < total_units; u += gstride) {
-                const int si = msys_of_chunk(A, u / MSUB);
-                if (!inner_active(sst[si], sdc[si])) continue;
-                const MSys &S = A.sys[si];
-                const int r0 = (u - S.chunk_begin * MSUB) * MUNIT + lane;
+            stream_chunks([&](int si, const MSys &S, int i) {
                 const float alpha = (float)sst[si].alpha;
-    #pragma unroll
-                for (int m = 0; m < MRPL; ++m) {
-                    const int row = r0 + m * LANES;
-                    const float sv = __fmaf_rn(-alpha, S.v[row], S.r[row]);
-                    S.s[row] = sv;
-                    if (S.mg.nlev > 0) S.p2[row] = S.mg.omega * S.invdiag32[row] * sv;
-                    else S.z[row] = S.invdiag32[row] * sv;
-                }
-            }
+                const float4 v = at4(S.v, i), r = at4(S.r, i), d = at4(S.invdiag32, i);
+                float *const out = S.mg.nlev > 0 ? S.p2 : S.z;
+                const float om = S.mg.omega;
+                const bool mg = S.mg.nlev > 0;
+                const float4 sv = each4([&](float v1, float r1, float) { return __fmaf_rn(-alpha, v1, r1); }, v, r, r);
+                const float4 z = each4([&](float d1, float s1, float) { return mg ? om * d1 * s1 : d1 * s1; }, d, sv, sv);
+                return Pair4{S.s, out, sv, z};
+            });
             if (!grid_sync(bar, target, &s_ok)) break;
             if (mg_on && !mg_precondition(A, sst, sdc, 1, s_tail, bar, target, &s_ok)) break;
             // t = A z, <t, t>, <t, s>
-            for (int u = cbegin; u < total_units; u += gstride) {
-                const int si = msys_of_chunk(A, u / MSUB);
-                if (!inner_active(sst[si], sdc[si])) continue;
-                const MSys &S = A.sys[si];
-                const int lc = u - S.chunk_begin * MSUB;
-                const int r0 = lc * MUNIT + lane;
-                float att = 0.0f, ats = 0.0f;
-    #pragma unroll
-                for (int m = 0; m < MRPL; ++m) {
-                    const int row = r0 + m * LANES;
-                    const float t = spmv_f32_row(S, row, S.z);
-                    S.t[row] = t;
-                    if (row < S.n) {
-                        att = __fmaf_rn(t, t, att);
-                        ats = __fmaf_rn(t, S.s[row], ats);
+            unit_phase([&](auto units) {
+                constexpr int H = decltype(units)::value;
+                for (int u = cbegin; u < total_units; u += H * gstride) {
+                    const UnitPair<CAP, H> U(A, sst, sdc, u, gstride, total_units);
+                    if (U.none()) continue;
+                    float t[H][MRPL], q[H][MRPL], att[H] = {}, ats[H] = {};
+#pragma unroll
+                    for (int h = 0; h < H; ++h)
+#pragma unroll
+                        for (int m = 0; m < MRPL; ++m) {
+                            const int row = U.lc[h] * MUNIT + lane + m * LANES;
+                            t[h][m] = spmv_f32_row(U.S(A, h), row, U.S(A, h).z);
+                            q[h][m] = U.S(A, h).s[row];
+                        }
+#pragma unroll
+                    for (int h = 0; h < H; ++h)
+                        if (U.on[h])
+#pragma unroll
+                            for (int m = 0; m < MRPL; ++m) {
+                                const int row = U.lc[h] * MUNIT + lane + m * LANES;
+                                U.S(A, h).t[row] = t[h][m];
+                                if (row < U.S(A, h).n) {
+                                    att[h] = __fmaf_rn(t[h][m], t[h][m], att[h]);
+                                    ats[h] = __fmaf_rn(t[h][m], q[h][m], ats[h]);
+                                }
+                            }
+#pragma unroll
+                    for (int h = 0; h < H; ++h) {
+                        if (!U.on[h]) continue;
+                        float tt, ts;
+                        lanes_tree_sum2<float>(att[h], ats[h], lane, reinterpret_cast<float *>(sm[gi]), tt, ts, gsync);
+                        if (lane == 0) reinterpret_cast<double2 *>(U.S(A, h).part)[U.lc[h]] = make_double2(tt, ts);
                     }
                 }
-                float tt, ts;
-                lanes_tree_sum2<float>(att, ats, lane, reinterpret_cast<float *>(sm[gi]), tt, ts, gsync);
-                if (lane == 0) reinterpret_cast<double2 *>(S.part)[lc] = make_double2(tt, ts);
-            }
+            });
             if (!grid_sync(bar, target, &s_ok)) break;
-            for (int q = gi; q < A.nsys; q += LOOP_GROUPS) {
-                if (!inner_active(sst[q], sdc[q])) continue;
-                const MSys &S = A.sys[q];
-                double ftt, fts;
-                lanes_final_sum2(S.part, S.nchunks * MSUB, lane, sm[gi], ftt, fts, gsync);
-                if (lane == 0) sst[q].w = (ftt > 0.0) ? fts / ftt : 0.0;
+            two_sums(0);
+            if (threadIdx.x < A.nsys && inner_active(sst[threadIdx.x], sdc[threadIdx.x])) {
+                const double ftt = s_sum[threadIdx.x][0];
+                sst[threadIdx.x].w = (ftt > 0.0) ? s_sum[threadIdx.x][1] / ftt : 0.0;
             }
             __syncthreads();
-            // x += alpha y + w z; r = s - w t; <r0, r>, <r, r>
-            for (int u = cbegin; u < total_units; u += gstride) {
-                const int si = msys_of_chunk(A, u / MSUB);
-                if (!inner_active(sst[si], sdc[si])) continue;
-                const MSys &S = A.sys[si];
-                const int lc = u - S.chunk_begin * MSUB;
-                const int r0 = lc * MUNIT + lane;
-                const float alpha = (float)sst[si].alpha, w = (float)sst[si].w;
-                float a0r = 0.0f, arr = 0.0f;
-    #pragma unroll
-                for (int m = 0; m < MRPL; ++m) {
-                    const int row = r0 + m * LANES;
-                    S.x[row] = __fmaf_rn(w, S.z[row], __fmaf_rn(alpha, S.y[row], S.x[row]));
-                    const float r = __fmaf_rn(-w, S.t[row], S.s[row]);
-                    S.r[row] = r;
-                    if (row < S.n) {
-                        a0r = __fmaf_rn(S.r0[row], r, a0r);
-                        arr = __fmaf_rn(r, r, arr);
+            // r = s - w t; <r0, r>, <r, r>
+            unit_phase([&](auto units) {
+                constexpr int H = decltype(units)::value;
+                for (int u = cbegin; u < total_units; u += H * gstride) {
+                    const UnitPair<CAP, H> U(A, sst, sdc, u, gstride, total_units);
+                    if (U.none()) continue;
+                    float t[H][MRPL], sv[H][MRPL], q[H][MRPL];
+#pragma unroll
+                    for (int h = 0; h < H; ++h)
+#pragma unroll
+                        for (int m = 0; m < MRPL; ++m) {
+                            const int row = U.lc[h] * MUNIT + lane + m * LANES;
+                            t[h][m] = U.S(A, h).t[row];
+                            sv[h][m] = U.S(A, h).s[row];
+                            q[h][m] = U.S(A, h).r0[row];
+                        }
+#pragma unroll
+                    for (int h = 0; h < H; ++h) {
+                        if (!U.on[h]) continue;
+                        const float w = (float)sst[U.si[h]].w;
+                        float a0r = 0.0f, arr = 0.0f;
+#pragma unroll
+                        for (int m = 0; m < MRPL; ++m) {
+                            const int row = U.lc[h] * MUNIT + lane + m * LANES;
+                            const float r = __fmaf_rn(-w, t[h][m], sv[h][m]);
+                            U.S(A, h).r[row] = r;
+                            if (row < U.S(A, h).n) {
+                                a0r = __fmaf_rn(q[h][m], r, a0r);
+                                arr = __fmaf_rn(r, r, arr);
+                            }
+                        }
+                        float t0r, trr;
+                        lanes_tree_sum2<float>(a0r, arr, lane, reinterpret_cast<float *>(sm[gi]), t0r, trr, gsync);
+                        if (lane == 0)
+                            reinterpret_cast<double2 *>(U.S(A, h).part + 2 * (size_t)U.S(A, h).nchunks * MSUB)[U.lc[h]] =
+                                make_double2(t0r, trr);
                     }
                 }
-                float t0r, trr;
-                lanes_tree_sum2<float>(a0r, arr, lane, reinterpret_cast<float *>(sm[gi]), t0r, trr, gsync);
-                if (lane == 0)
-                    reinterpret_cast<double2 *>(S.part + 2 * (size_t)S.nchunks * MSUB)[lc] = make_double2(t0r, trr);
-            }
-            if (!grid_sync(bar, target, &s_ok)) break;
-            for (int q = gi; q < A.nsys; q += LOOP_GROUPS) {
-                if (!inner_active(sst[q], sdc[q])) continue;
-                const MSys &S = A.sys[q];
-                double f0r, frr;
-                lanes_final_sum2(S.part + 2 * (size_t)S.nchunks * MSUB, S.nchunks * MSUB, lane, sm[gi], f0r, frr, gsync);
-                if (lane == 0) m32_end_iteration(sst[q], f0r, frr);
-            }
+            });
+            grid_arrive(bar, target);
+            // x += alpha y + w z, while the other blocks arrive
+            stream_chunks([&](int si, const MSys &S, int i) {
+                const float alpha = (float)sst[si].alpha, w = (float)sst[si].w;
+                const float4 x = at4(S.x, i), y = at4(S.y, i), z = at4(S.z, i);
+                const float4 xn = each4(
+                    [&](float x1, float y1, float z1) { return __fmaf_rn(w, z1, __fmaf_rn(alpha, y1, x1)); }, x, y, z);
+                return Pair4{S.x, nullptr, xn, xn};
+            });
+            if (!grid_wait(bar, target, &s_ok)) break;
+            two_sums(2);
+            if (threadIdx.x < A.nsys && inner_active(sst[threadIdx.x], sdc[threadIdx.x]))
+                m32_end_iteration(sst[threadIdx.x], s_sum[threadIdx.x][0], s_sum[threadIdx.x][1]);
             __syncthreads();
         }
         bool any = false;

@@ -31,10 +31,11 @@ struct MGLevel {
     const int *nbr;       // [6][npad], -1 none
     float *coef;          // [7][npad]
     float *invdiag;       // [npad]
-    const int *agg;       // [rows of level k-1]: the row of this level each belongs to
+    const int *pos;       // [rows of level k-1]: 8 x the row of this level each belongs to + its rank there
     const int *mstart;    // [n + 1]: offsets into members
     const int *members;   // rows of level k-1 of each row, ascending
-    float *x, *b, *t, *xo;  // V-cycle vectors [npad]: Jacobi start, right-hand side, residual, result
+    float *x, *b, *t, *xo;  // V-cycle vectors [npad]: Jacobi start, right-hand side, scratch, result
+    float *t8;            // [8 npad]: the residual of level k-1 at `pos`, +0 in the unused places
 };
 struct MGSet {
     int nlev;             // coarse levels (0: Jacobi preconditioning)

@@ -85,13 +85,14 @@ void MixedSetT<CAP>::configure(const std::vector<SolveItem> &items, cudaStream_t
                 G.nbr = H.nbr.p;
                 G.coef = H.coef.p;
                 G.invdiag = H.invdiag.p;
-                G.agg = H.agg.p;
+                G.pos = H.pos.p;
                 G.mstart = H.mstart.p;
                 G.members = H.members.p;
                 G.x = H.x.p;
                 G.b = H.b.p;
                 G.t = H.t.p;
                 G.xo = H.xo.p;
+                G.t8 = H.t8.p;
             }
             // the tail: the levels that fit in a block's shared memory (a
             // merged set has no shared memory of its own per system)

@@ -99,8 +99,8 @@ inline int pad_rows(int n) { return ((n + CH - 1) / CH) * CH; }
 // Device arrays of the multilevel hierarchy of one system (MIXED_MG)
 struct MGHostLevel {
     int n = 0, npad = 0;
-    DBuf<int> nbr, agg, mstart, members;
-    DBuf<float> coef, invdiag, x, b, t, xo;
+    DBuf<int> nbr, pos, mstart, members;
+    DBuf<float> coef, invdiag, x, b, t, xo, t8;
 };
 struct MGHost {
     int nlev = 0;
