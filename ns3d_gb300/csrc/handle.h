@@ -136,17 +136,20 @@ struct ns3d_handle {
     std::vector<ns3d::SolveItem> pressure_correction_begin();
     void pressure_correction_end(const std::vector<ns3d::SolveOutcome> &out);
     void correct_pressure_launch();
-    void correct_pressure_read();
+    void diag_fetch();  // the reductions' results to the host
+    void correct_pressure_read();  // fetch and take one result; *_result: after a fetch
+    void correct_pressure_result();
     void permeability_launch();
     void permeability_read(ns3d::Scalars &s);
+    void permeability_result(ns3d::Scalars &s);
     void divergence_launch();
     void divergence_read(ns3d::Scalars &s);
+    void divergence_result(ns3d::Scalars &s);
     void diagnostics_end(ns3d::Scalars &s);
     void log_solve(const char *comp, const ns3d::SolveOutcome &o);
     void log_pressure_status(const ns3d::SolveOutcome &o);
     void compute_pressure_correction();
     void compute_pressure_field();
-    void correct_pressure_field();
     void permeability(ns3d::Scalars &s);
     void divergence(ns3d::Scalars &s);
     void diagnostics(ns3d::Scalars &s);

@@ -504,6 +504,9 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
         }
         return true;
     };
+    bool any = false;  // a launch that finds every system done returns at once
+    for (int q = 0; q < A.nsys; ++q) any = any || state_active(sst[q]);
+    if (!any) max_iters = 0;
     int it = 0;
     bool ok = true;
     for (; it < max_iters; ++it) {

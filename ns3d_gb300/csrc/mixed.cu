@@ -848,6 +848,11 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
         }
     };
     static_assert(CH == 8 * LANES, "two float4 a lane");
+    {  // a launch that finds every system done returns at once
+        bool any = false;
+        for (int q = 0; q < A.nsys; ++q) any = any || inner_active(sst[q], sdc[q]);
+        if (!any) max_iters = 0;
+    }
     // a phase over work units, two at a time when a group has that many
     auto unit_phase = [&](auto run) {
         if (total_units > gstride) run(std::integral_constant<int, 2>());

@@ -30,17 +30,13 @@ void MixedSetT<CAP>::configure(const std::vector<SolveItem> &items, cudaStream_t
     if (ns > CAP) throw ApiError(NS3D_ERR_ARG, "too many systems in one solve set");
     std::vector<MSys> ms(ns);
     int chunk = 0;
-    if (!bar_.n) {
-        bar_.alloc_zero(1, st);
-        h_err_.alloc(1);
-    }
-    if ((int)st_.n < ns) {
-        st_.alloc_zero(ns, st);
+    if (cap_ < ns) {
+        cap_ = ns;
+        const size_t lines = (state_bytes() + sizeof(GridBar) - 1) / sizeof(GridBar);
+        bar_.alloc_zero(lines, st);
+        h_bar_.alloc(lines);
         out_st_.alloc_zero(ns, st);
-        dc_.alloc_zero(ns, st);
-        h_st_.alloc(ns);
         h_out_.alloc(ns);
-        h_dc_.alloc(ns);
     }
     for (int i = 0; i < ns; ++i) {
         DevSys &S = *items[i].sys;
@@ -66,8 +62,8 @@ void MixedSetT<CAP>::configure(const std::vector<SolveItem> &items, cudaStream_t
         m.p2 = S.fp2.p; m.v2 = S.fv2.p;
         m.y = S.fy.p; m.s = S.fs.p; m.z = S.fz.p; m.t = S.ft.p;
         m.part = S.part.p;
-        m.st = st_.p + i;
-        m.dc = dc_.p + i;
+        m.st = st_of(bar_.p) + i;
+        m.dc = dc_of(bar_.p) + i;
         // a solver instance's own set: the multilevel preconditioner for a
         // single system; a merged set: what each system's own set chose
         const bool mg = CAP > KMAX ? (items[i].mg && S.mg)
@@ -108,7 +104,6 @@ void MixedSetT<CAP>::configure(const std::vector<SolveItem> &items, cudaStream_t
     set_.nsys = ns;
     set_.total_chunks = chunk;
     for (int i = 0; i < ns; ++i) set_.sys[i] = ms[i];
-    NS3D_CUDA_CHECK(cudaStreamSynchronize(st));  // FP32 buffers allocated above
     key_ = key;
     nsys_ = ns;
     total_chunks_ = chunk;
@@ -131,6 +126,9 @@ void MixedSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st, s
     configure(items, st);
     const int ns = nsys_;
     int maxit = 0;
+    DCState *const h_dc = dc_of(h_bar_.p);
+    KState *const h_st = st_of(h_bar_.p);
+    std::memset(h_bar_.p, 0, state_bytes());
     for (int i = 0; i < ns; ++i) {
         DevSys &S = *items[i].sys;
         launch_to_f32(S.coef.p, S.invdiag.p, S.npad, S.coef32.p, S.invdiag32.p, st);
@@ -147,14 +145,10 @@ void MixedSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st, s
             d.total_iter = d.maxit;
             d.error = d.tol;
         }
-        h_dc_.p[i] = d;
-        KState k;
-        std::memset(&k, 0, sizeof k);
-        h_st_.p[i] = k;
+        h_dc[i] = d;
         maxit = std::max(maxit, items[i].maxit);
     }
-    NS3D_CUDA_CHECK(cudaMemcpyAsync(dc_.p, h_dc_.p, ns * sizeof(DCState), cudaMemcpyHostToDevice, st));
-    NS3D_CUDA_CHECK(cudaMemcpyAsync(st_.p, h_st_.p, ns * sizeof(KState), cudaMemcpyHostToDevice, st));
+    NS3D_CUDA_CHECK(cudaMemcpyAsync(bar_.p, h_bar_.p, state_bytes(), cudaMemcpyHostToDevice, st));
     plan_mixed(set_, variant, share);
     launch_dc_resid(set_, 1, st);
     // Every round runs at least one inner iteration per unfinished system, so
@@ -176,25 +170,28 @@ void MixedSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st, s
     std::vector<int> iters_before(ns, 0);
     // One round = FP32 init, the FP32 loop kernel (it ends when every inner
     // solve of the round is done: each is capped by the remaining iteration
-    // budget), the FP64 update and residual; the host reads the outer state
-    // once per round.
+    // budget), the FP64 update and residual; the host reads barrier and states
+    // once per round.  The first round follows the first residual unseen: its
+    // kernels skip the systems that are done already.
     while (true) {
-        NS3D_CUDA_CHECK(cudaMemcpyAsync(h_dc_.p, dc_.p, ns * sizeof(DCState), cudaMemcpyDeviceToHost, st));
-        NS3D_CUDA_CHECK(cudaMemcpyAsync(h_err_.p, &bar_.p->err, sizeof(int), cudaMemcpyDeviceToHost, st));
-        NS3D_CUDA_CHECK(cudaStreamSynchronize(st));
-        if (rounds > 0 && h_err_.p[0])
-            throw ApiError(NS3D_ERR_TIMEOUT, "FP32 BiCGSTAB loop kernel: a grid barrier timed out");
-        if (tune && rounds > 0) {  // inner iterations of the round, from the FP64 states
-            double rows = 0;
-            for (int i = 0; i < ns; ++i) rows += (double)set_.sys[i].n * (h_dc_.p[i].total_iter - iters_before[i]);
-            float ms = 0;
-            NS3D_CUDA_CHECK(cudaEventElapsedTime(&ms, ev_[0], ev_[1]));
-            grid_tuner().report(tkey, cand, ms, rows);
+        if (rounds > 0) {
+            NS3D_CUDA_CHECK(cudaMemcpyAsync(h_bar_.p, bar_.p, state_bytes(), cudaMemcpyDeviceToHost, st));
+            NS3D_CUDA_CHECK(cudaStreamSynchronize(st));
+            if (total_chunks_ > 0 && h_bar_.p->err)
+                throw ApiError(NS3D_ERR_TIMEOUT, "FP32 BiCGSTAB loop kernel: a grid barrier timed out");
+            if (tune) {  // inner iterations of the round, from the FP64 states
+                double rows = 0;
+                for (int i = 0; i < ns; ++i)
+                    if (!h_dc[i].zero_rhs) rows += (double)set_.sys[i].n * (h_dc[i].total_iter - iters_before[i]);
+                float ms = 0;
+                NS3D_CUDA_CHECK(cudaEventElapsedTime(&ms, ev_[0], ev_[1]));
+                grid_tuner().report(tkey, cand, ms, rows);
+            }
+            for (int i = 0; i < ns; ++i) iters_before[i] = h_dc[i].total_iter;
+            bool all_done = true;
+            for (int i = 0; i < ns; ++i) all_done = all_done && h_dc[i].done;
+            if (all_done) break;
         }
-        for (int i = 0; i < ns; ++i) iters_before[i] = h_dc_.p[i].total_iter;
-        bool all_done = true;
-        for (int i = 0; i < ns; ++i) all_done = all_done && h_dc_.p[i].done;
-        if (all_done) break;
         if (++rounds > maxit + 2L) throw ApiError(NS3D_ERR_TIMEOUT, "defect correction exceeded its round bound");
         launch_m32_init(set_, st);
         if (tune) {
@@ -206,15 +203,13 @@ void MixedSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st, s
         launch_dc_update(set_, st);
         launch_dc_resid(set_, 0, st);
     }
-    NS3D_CUDA_CHECK(cudaMemcpyAsync(h_st_.p, st_.p, ns * sizeof(KState), cudaMemcpyDeviceToHost, st));
-    NS3D_CUDA_CHECK(cudaStreamSynchronize(st));
     out.assign(ns, SolveOutcome());
     for (int i = 0; i < ns; ++i) {
-        const DCState &d = h_dc_.p[i];
+        const DCState &d = h_dc[i];
         out[i].iters = d.total_iter;
         out[i].info = d.info;
         out[i].error = d.error;
-        out[i].work = h_st_.p[i].work;
+        out[i].work = h_st[i].work;
         out[i].valid = true;
         KState k;
         std::memset(&k, 0, sizeof k);

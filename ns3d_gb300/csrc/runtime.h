@@ -178,11 +178,11 @@ template <int CAP>
 class KrylovSetT {
   public:
     void run(const std::vector<SolveItem> &items, cudaStream_t st, std::vector<SolveOutcome> &out);
-    const KState *device_state(int i) const { return st_.p + i; }
+    const KState *device_state(int i) const { return reinterpret_cast<const KState *>(bar_.p + 1) + i; }
     // allocates the per-system state of `items` (and records them) without
     // solving: a merged run copies the final states here
     void prepare(const std::vector<SolveItem> &items, cudaStream_t st) { configure(items, st); }
-    KState *state_buffer() { return st_.p; }
+    KState *state_buffer() { return reinterpret_cast<KState *>(bar_.p + 1); }
     long launches() const { return launches_; }
     void reset_launch_count() { launches_ = 0; }
 
@@ -203,19 +203,18 @@ class KrylovSetT {
     void configure(const std::vector<SolveItem> &items, cudaStream_t st);
     cudaEvent_t ev_[2] = {nullptr, nullptr};
     KSetArgT<CAP> set_;  // passed to every kernel by value
-    DBuf<KState> st_;
-    HBuf<KState> h_st_, h_up_;
+    // the loop kernel's barrier and behind it the cap_ systems' states: one copy reads both back
     DBuf<GridBar> bar_;
+    HBuf<GridBar> h_bar_;
+    HBuf<KState> h_up_;
+    int cap_ = 0;
     DBuf<LoopProf> prof_;
-    HBuf<int> h_err_;
     int nsys_ = 0, total_chunks_ = 0;
     long launches_ = 0;
 };
 using KrylovSet = KrylovSetT<KMAX>;
 using KrylovSetMerged = KrylovSetT<KMAX_MERGED>;
 
-
-struct DCState;
 
 #ifndef NS3D_MIXED_INNER_TOL
 #define NS3D_MIXED_INNER_TOL 1e-4
@@ -235,7 +234,6 @@ class MixedSetT {
     // variant: -1 from the set's own rows, 0 five-phase, 1 fused FP32 loop
     void run(const std::vector<SolveItem> &items, cudaStream_t st, std::vector<SolveOutcome> &out,
              int variant = -1);
-    const KState *inner_state(int i) const { return st_.p + i; }
     // FP64 outcome of system i, mirrored into a KState (iter, info) for the
     // velocity post-processing kernel
     const KState *device_state(int i) const { return out_st_.p + i; }
@@ -254,14 +252,18 @@ class MixedSetT {
   private:
     void configure(const std::vector<SolveItem> &items, cudaStream_t st);
     cudaEvent_t ev_[2] = {nullptr, nullptr};  // around the FP32 loop launch (merged sets: autotuner timing)
-    DBuf<KState> st_, out_st_;
-    DBuf<DCState> dc_;
-    HBuf<KState> h_st_, h_out_;
-    HBuf<DCState> h_dc_;
+    // the loop kernel's barrier, the outer and the inner states of cap_
+    // systems in one buffer: one copy reads or writes them all
+    DBuf<GridBar> bar_;
+    HBuf<GridBar> h_bar_;
+    int cap_ = 0;
+    static DCState *dc_of(GridBar *b) { return reinterpret_cast<DCState *>(b + 1); }
+    KState *st_of(GridBar *b) const { return reinterpret_cast<KState *>(dc_of(b) + cap_); }
+    size_t state_bytes() const { return sizeof(GridBar) + cap_ * (sizeof(DCState) + sizeof(KState)); }
+    DBuf<KState> out_st_;
+    HBuf<KState> h_out_;
     std::vector<const double *> key_;
     MSetArgT<CAP> set_;  // passed to every kernel by value
-    DBuf<GridBar> bar_;
-    HBuf<int> h_err_;
     int nsys_ = 0, total_chunks_ = 0;
 };
 using MixedSet = MixedSetT<KMAX>;

@@ -105,22 +105,22 @@ void KrylovSetT<CAP>::configure(const std::vector<SolveItem> &items, cudaStream_
     }
     const int ns = (int)ks.size();
     if (ns > CAP) throw ApiError(NS3D_ERR_ARG, "too many systems in one solve set");
-    if ((int)st_.n < ns) {
-        st_.alloc_zero(ns, st);
-        h_st_.alloc(ns);
+    if (cap_ < ns) {
+        cap_ = ns;
+        const size_t lines = 1 + (ns * sizeof(KState) + sizeof(GridBar) - 1) / sizeof(GridBar);
+        bar_.alloc_zero(lines, st);
+        h_bar_.alloc(lines);
         h_up_.alloc(ns);
     }
-    if (!bar_.n) {
-        bar_.alloc_zero(1, st);
+    if (!prof_.n) {
         prof_.alloc_zero(1, st);
-        h_err_.alloc(1);
         for (cudaEvent_t &e : ev_) NS3D_CUDA_CHECK(cudaEventCreate(&e));
     }
     std::memset(&set_, 0, sizeof set_);
     set_.nsys = ns;
     set_.total_chunks = chunk;
     for (int i = 0; i < ns; ++i) {
-        ks[i].st = st_.p + i;
+        ks[i].st = state_buffer() + i;
         set_.sys[i] = ks[i];
     }
     nsys_ = ns;
@@ -148,7 +148,7 @@ void KrylovSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st,
         h_up_.p[i] = z;
         maxit = std::max(maxit, items[i].maxit);
     }
-    NS3D_CUDA_CHECK(cudaMemcpyAsync(st_.p, h_up_.p, ns * sizeof(KState), cudaMemcpyHostToDevice, st));
+    NS3D_CUDA_CHECK(cudaMemcpyAsync(state_buffer(), h_up_.p, ns * sizeof(KState), cudaMemcpyHostToDevice, st));
     plan_krylov(set_, share);
     launch_krylov_init(set_, st);
     launches_ += 2;
@@ -168,46 +168,48 @@ void KrylovSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st,
     // bucket, 128 to 255 chunks)
     const uint64_t tkey = tuner_key(0, set_.one_per_block ? std::min(total_chunks_, 127) : total_chunks_, share);
     int cand = 0;
+    // The first loop launch follows the set-up without a look at the states
+    // (a kernel whose systems are all done returns at once): one wait for the
+    // stream per launch, one copy of barrier and states per wait.
+    const KState *h_st = reinterpret_cast<const KState *>(h_bar_.p + 1);
+    bool any_paused = false;
     while (true) {
-        NS3D_CUDA_CHECK(cudaMemcpyAsync(h_st_.p, st_.p, ns * sizeof(KState), cudaMemcpyDeviceToHost, st));
-        NS3D_CUDA_CHECK(cudaMemcpyAsync(h_err_.p, &bar_.p->err, sizeof(int), cudaMemcpyDeviceToHost, st));
-        NS3D_CUDA_CHECK(cudaStreamSynchronize(st));
-        // the flag belongs to this run's last loop launch (before the first
-        // one it still holds the previous run's: a timed-out solve must not
-        // poison the next)
-        if (loops > 0 && h_err_.p[0])
-            throw ApiError(NS3D_ERR_TIMEOUT, "BiCGSTAB loop kernel: a grid barrier timed out");
-        bool all_done = true, any_paused = false;
-        int progress = 0;
-        int64_t rows = 0;
-        for (int i = 0; i < ns; ++i) {
-            const KState &k = h_st_.p[i];
-            if (!k.done) all_done = false;
-            if (k.paused && !k.done) any_paused = true;
-            if (loops > 0) {
+        if (loops > 0) {
+            NS3D_CUDA_CHECK(cudaMemcpyAsync(h_bar_.p, bar_.p, sizeof(GridBar) + ns * sizeof(KState),
+                                            cudaMemcpyDeviceToHost, st));
+            NS3D_CUDA_CHECK(cudaStreamSynchronize(st));
+            // (no launch, no flag: an empty set leaves an earlier run's)
+            if (total_chunks_ > 0 && h_bar_.p->err)
+                throw ApiError(NS3D_ERR_TIMEOUT, "BiCGSTAB loop kernel: a grid barrier timed out");
+            bool all_done = true;
+            any_paused = false;
+            int progress = 0;
+            int64_t rows = 0;
+            for (int i = 0; i < ns; ++i) {
+                const KState &k = h_st[i];
+                if (!k.done) all_done = false;
+                if (k.paused && !k.done) any_paused = true;
                 progress = std::max(progress, k.work - work_before[i]);
                 rows += (int64_t)set_.sys[i].n * (k.work - work_before[i]);
+                work_before[i] = k.work;
             }
-            work_before[i] = k.work;
+            if (tune || profiling) {
+                float ms = 0;
+                NS3D_CUDA_CHECK(cudaEventElapsedTime(&ms, ev_[0], ev_[1]));
+                if (tune) grid_tuner().report(tkey, cand, ms, (double)rows);
+                if (profiling && rows > 0) {
+                    prof.launches[5] += 1;
+                    prof.ms[5] += ms;
+                    prof.rows[5] += rows;
+                    for (int k = 0; k < 5; ++k) prof.rows[k] += rows;
+                }
+            }
+            issued += progress;
+            if (all_done) break;
+            if (progress == 0 && !any_paused)
+                throw ApiError(NS3D_ERR_TIMEOUT, "BiCGSTAB loop kernel made no progress");
+            if (issued >= cap) throw ApiError(NS3D_ERR_TIMEOUT, "BiCGSTAB driver exceeded its iteration bound");
         }
-        if (tune && loops > 0) {
-            float ms = 0;
-            NS3D_CUDA_CHECK(cudaEventElapsedTime(&ms, ev_[0], ev_[1]));
-            grid_tuner().report(tkey, cand, ms, (double)rows);
-        }
-        if (profiling && loops > 0) {
-            float ms = 0;
-            NS3D_CUDA_CHECK(cudaEventElapsedTime(&ms, ev_[0], ev_[1]));
-            prof.launches[5] += 1;
-            prof.ms[5] += ms;
-            prof.rows[5] += rows;
-            for (int k = 0; k < 5; ++k) prof.rows[k] += rows;
-        }
-        issued += progress;
-        if (all_done) break;
-        if (loops > 0 && progress == 0 && !any_paused)
-            throw ApiError(NS3D_ERR_TIMEOUT, "BiCGSTAB loop kernel made no progress");
-        if (issued >= cap) throw ApiError(NS3D_ERR_TIMEOUT, "BiCGSTAB driver exceeded its iteration bound");
         if (any_paused) {
             launch_krylov_restart(set_, st);
             launches_ += 1;
@@ -230,7 +232,7 @@ void KrylovSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st,
         }
     }
     for (int i = 0; i < ns; ++i) {
-        const KState &k = h_st_.p[i];
+        const KState &k = h_st[i];
         out[i].iters = k.iter;
         out[i].info = k.info;
         out[i].error = k.error;
@@ -462,11 +464,6 @@ void ns3d_handle::compute_pressure_field() {
 }
 
 // CorrectPressureField, src/NSBase.cxx:2367-2380
-void ns3d_handle::correct_pressure_field() {
-    correct_pressure_launch();
-    correct_pressure_read();
-}
-
 void ns3d_handle::correct_pressure_launch() {
     launch_correct_pressure(P.view(), pc.p, p.p, beta, diag_part.p, diag.p, stream);
 }
@@ -474,9 +471,17 @@ void ns3d_handle::correct_pressure_launch() {
 // Each *_read copies the reduction results to the host and waits for the
 // stream: with many instances on one stream, the first read waits for every
 // instance's launches and the others find them done.
-void ns3d_handle::correct_pressure_read() {
+void ns3d_handle::diag_fetch() {
     NS3D_CUDA_CHECK(cudaMemcpyAsync(h_diag.p, diag.p, sizeof(DiagOut), cudaMemcpyDeviceToHost, stream));
     sync();
+}
+
+void ns3d_handle::correct_pressure_read() {
+    diag_fetch();
+    correct_pressure_result();
+}
+
+void ns3d_handle::correct_pressure_result() {
     const DiagOut &d = *h_diag.p;
     pcmax = beta * d.pcmax;
     pcmin = beta * d.pcmin;
@@ -495,8 +500,11 @@ void ns3d_handle::permeability(Scalars &s) {
 void ns3d_handle::permeability_launch() { launch_permeability(grid(), u.p, p.p, border, diag_part.p, diag.p, stream); }
 
 void ns3d_handle::permeability_read(Scalars &s) {
-    NS3D_CUDA_CHECK(cudaMemcpyAsync(h_diag.p, diag.p, sizeof(DiagOut), cudaMemcpyDeviceToHost, stream));
-    sync();
+    diag_fetch();
+    permeability_result(s);
+}
+
+void ns3d_handle::permeability_result(Scalars &s) {
     const DiagOut &d = *h_diag.p;
     const double sx = dy * dz;
     double v_moy = d.v_sum;
@@ -530,8 +538,11 @@ void ns3d_handle::divergence_launch() {
 }
 
 void ns3d_handle::divergence_read(Scalars &s) {
-    NS3D_CUDA_CHECK(cudaMemcpyAsync(h_diag.p, diag.p, sizeof(DiagOut), cudaMemcpyDeviceToHost, stream));
-    sync();
+    diag_fetch();
+    divergence_result(s);
+}
+
+void ns3d_handle::divergence_result(Scalars &s) {
     const DiagOut &d = *h_diag.p;
     s.normdiv = std::sqrt(d.sumdiv2);
     s.velocityNorm = d.sumvel / np;
@@ -539,9 +550,13 @@ void ns3d_handle::divergence_read(Scalars &s) {
     s.MaxDeltaV = d.maxdv;
 }
 
+// (one read-back for both reductions)
 void ns3d_handle::diagnostics(Scalars &s) {
-    permeability(s);
-    divergence(s);
+    permeability_launch();
+    divergence_launch();
+    diag_fetch();
+    permeability_result(s);
+    divergence_result(s);
     diagnostics_end(s);
 }
 
@@ -741,9 +756,12 @@ void ns3d_handle::run_simplec() {
         launch_correct_velocity(0, 1, g, ph, U.view(), pc.p, u.p, dvmax, stream);
         launch_correct_velocity(1, 1, g, ph, V.view(), pc.p, v.p, dvmax, stream);
         if (nw > 0) launch_correct_velocity(2, 1, g, ph, W.view(), pc.p, w.p, dvmax, stream);
-        correct_pressure_field();
+        correct_pressure_launch();
+        divergence_launch();
+        diag_fetch();  // one read-back for both
+        correct_pressure_result();
         Scalars after = s;
-        divergence(after);
+        divergence_result(after);
         s.MaxDeltaV = after.MaxDeltaV; s.normdiv = after.normdiv; s.velocityNorm = after.velocityNorm;
         s.maxdiv = after.maxdiv;
         save_snapshot(it, savecounter);
