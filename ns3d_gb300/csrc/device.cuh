@@ -134,7 +134,7 @@ constexpr int KMAX_MERGED = 64;
 template <int CAP>
 struct KSetArgT {
     int nsys, total_chunks;
-    int one_per_block, pad_;  // the loop kernel of this solve (plan_krylov)
+    int one_per_block, pad_;  // blocks per chunk, 0: several chunks per block (plan_krylov)
     KSys sys[CAP];
 };
 using KSetArg = KSetArgT<KMAX>;

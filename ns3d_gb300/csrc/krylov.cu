@@ -919,14 +919,67 @@ static int krylov_loop_grid(int total_chunks, int occ, int share) {
     return loop_grid(total_chunks, 1, occ);
 }
 
+// blocks the device can hold at once of the one-chunk kernel split over F blocks
+template <int CAP, int F>
+static int split_blocks() {
+    static std::atomic<int> blocks{-1};
+    int b = blocks.load();
+    if (b >= 0) return b;
+    b = 0;
+    const void *fn = (const void *)k_kr_chunk<CAP, F>;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kChunkSmemBytes<F>) == cudaSuccess) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(F);
+        cfg.blockDim = dim3(kChunkRows<F>);
+        cfg.dynamicSmemBytes = kChunkSmemBytes<F>;
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = F;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) == cudaSuccess) b = n * F;
+    }
+    cudaGetLastError();
+    blocks = b;
+    return b;
+}
+
 // A set whose share of the SMs gives every chunk a block runs one chunk per
 // block (krylov_chunk.cuh), a larger one several chunks per block: a block has
 // one thread per row of its chunk, and the exchange needs every block
-// resident.  Measured, us per iteration, several per block -> one: 5 chunks
-// 35.4 -> 15.0, 44 chunks 38.4 -> 17.5, 141 chunks 39.9 -> 19.2.
+// resident.  While the share allows two or four blocks per chunk, a chunk is
+// split over a cluster of them.  Measured, us per iteration, several per
+// block -> one -> split: 5 chunks 35.4 -> 14.4 -> 12.5 (four blocks; 15.0 with
+// two), 44 chunks 38.4 -> 17.5 -> 13.3 (two), 141 chunks 39.9 -> 19.3.
 template <int CAP>
 void plan_krylov(KSetArgT<CAP> &A, int share) {
-    A.one_per_block = A.total_chunks <= device_sm_count() && krylov_loop_grid<CAP>(A.total_chunks, 1, share) >= A.total_chunks;
+    A.one_per_block = 0;
+    const int n = A.total_chunks, sms = device_sm_count();
+    if (n > sms || krylov_loop_grid<CAP>(n, 1, share) < n) return;
+    const int avail = CAP > KMAX ? sms / std::max(share, 1) : sms / std::max(1, active_solves());
+    if (4 * n <= std::min(avail, split_blocks<CAP, 4>())) A.one_per_block = 4;
+    else if (2 * n <= std::min(avail, split_blocks<CAP, 2>())) A.one_per_block = 2;
+    else A.one_per_block = 1;
+}
+
+template <int CAP, int F>
+static cudaError_t launch_chunk(KSetArgT<CAP> &a, GridBar *bar, LoopProf *prof, int max_iters, cudaStream_t st) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(a.total_chunks * F);
+    cfg.blockDim = dim3(kChunkRows<F>);
+    cfg.dynamicSmemBytes = kChunkSmemBytes<F>;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = F;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = F > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, k_kr_chunk<CAP, F>, a, bar, prof, max_iters);
 }
 
 template <int CAP>
@@ -940,7 +993,7 @@ cudaError_t launch_krylov_loop(const KSetArgT<CAP> &A, GridBar *bar, LoopProf *p
         size_t smem;
         int chunks_per_block;  // at most (0: any number)
     };
-    static const Kernel kernels[] = {{(const void *)k_kr_chunk<CAP>, kChunkSmemBytes, 1},
+    static const Kernel kernels[] = {{(const void *)k_kr_chunk<CAP, 1>, kChunkSmemBytes<1>, 1},
                                      {(const void *)k_kr_loop<CAP, 4>, kNbrSmemBytes<4>, LOOP_GROUPS / 4},
                                      {(const void *)k_kr_loop<CAP, 2>, kNbrSmemBytes<2>, LOOP_GROUPS / 2},
                                      {(const void *)k_kr_loop<CAP, 1>, kNbrSmemBytes<1>, LOOP_GROUPS},
@@ -963,9 +1016,12 @@ cudaError_t launch_krylov_loop(const KSetArgT<CAP> &A, GridBar *bar, LoopProf *p
     KSetArgT<CAP> a = A;
     void *args[] = {&a, &bar, &prof, &max_iters};
     count_launches(1);
-    const int grid = A.one_per_block ? A.total_chunks : krylov_loop_grid<CAP>(A.total_chunks, 1, share);
-    int k = A.one_per_block ? 0 : 1;
-    while (!A.one_per_block && kernels[k].chunks_per_block && A.total_chunks > grid * kernels[k].chunks_per_block) ++k;
+    if (A.one_per_block == 4) return launch_chunk<CAP, 4>(a, bar, prof, max_iters, st);
+    if (A.one_per_block == 2) return launch_chunk<CAP, 2>(a, bar, prof, max_iters, st);
+    if (A.one_per_block == 1) return launch_chunk<CAP, 1>(a, bar, prof, max_iters, st);
+    const int grid = krylov_loop_grid<CAP>(A.total_chunks, 1, share);
+    int k = 1;
+    while (kernels[k].chunks_per_block && A.total_chunks > grid * kernels[k].chunks_per_block) ++k;
     return cudaLaunchCooperativeKernel(kernels[k].fn, grid, LOOP_THREADS, args, kernels[k].smem, st);
 }
 

@@ -19,7 +19,8 @@ pytestmark = pytest.mark.gpu
 
 # all-fluid boxes of exactly 1024 k (+ 1) cells, a line of cells (W = row - 1,
 # E = row + 1), and porous images
-BOXES = [(16, 8, 8), (41, 5, 5), (32, 32, 32), (33, 32, 32), (64, 32, 32), (65, 32, 32), (64, 64, 32), (43, 96, 32),
+# (up to 36 and 76 chunks the loop splits a chunk over four and two blocks)
+BOXES = [(16, 8, 8), (41, 5, 5), (36, 32, 32), (37, 32, 32), (75, 32, 32), (76, 32, 32), (77, 32, 32), (32, 32, 32), (33, 32, 32), (64, 32, 32), (65, 32, 32), (64, 64, 32), (43, 96, 32),
          (152, 32, 32), (153, 32, 32), (1100, 1, 1)]
 
 
