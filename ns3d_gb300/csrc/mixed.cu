@@ -1302,10 +1302,10 @@ void launch_m32_init(const MSetArgT<CAP> &A, cudaStream_t st) {
 
 
 // Sets up to kFusedRows rows run the three-phase loop (fewer barriers; the
-// recomputed neighbour operands are cache hits); larger sets run the
-// five-phase loop, whose smaller working set stays in the L2 (measured: a
-// 42 K-row solve 9% faster fused, a 1 M-row solve 16% slower).
-constexpr long kFusedRows = 1L << 19;
+// recomputed neighbour operands are cache hits), larger ones the five-phase
+// loop (157 K rows: 47 ms three-phase, 51 five-phase for two SIMPLER outer
+// iterations; 440 K rows: 35 and 31 ms for one).
+constexpr long kFusedRows = 1L << 18;
 
 // (the V-cycle runs in the five-phase loop)
 bool m32_fused(long rows, bool mg) { return rows <= kFusedRows && !mg; }
@@ -1313,28 +1313,25 @@ bool m32_fused(long rows, bool mg) { return rows <= kFusedRows && !mg; }
 // at most 21 words a row and one more a level (mg_tail_words)
 constexpr size_t kTailSmemMax = ((size_t)21 * MG_TAIL_ROWS + MG_MAX) * 4;
 
-// Sets without a multilevel system whose share of the SMs holds one or two
-// chunks per block run the loop with resident chunks (mixed_chunk.cuh).
-// Ten SIMPLEC outer iterations of a 56^3 image (pressure 103 chunks, momentum
-// 284): 85 -> 68 ms.
+// Sets without a multilevel system whose share of the SMs gives every chunk a
+// block run the loop with resident chunks (mixed_chunk.cuh).  Ten SIMPLEC
+// outer iterations of a 56^3 image (pressure 103 chunks): 85 -> 68 ms.
 template <int CAP>
 void plan_mixed(MSetArgT<CAP> &A, int variant, int share) {
     A.resident = 0;
     for (int i = 0; i < A.nsys; ++i)
         if (A.sys[i].mg.nlev > 0) return;
     const int sharers = CAP > KMAX ? std::max(share, 1) : std::max(1, active_solves());
-    const int blocks = std::max(1, device_sm_count() / sharers);
-    if (A.total_chunks <= blocks) A.resident = 1;
-    else if (A.total_chunks <= 2 * blocks) A.resident = 2;
+    A.resident = A.total_chunks <= std::max(1, device_sm_count() / sharers);
 }
 
-template <int CAP, int R>
+template <int CAP>
 static cudaError_t launch_m32_resident(const MSetArgT<CAP> &A, GridBar *bar, int max_iters, cudaStream_t st) {
-    const void *fn = (const void *)k_m32_chunk<CAP, R>;
+    const void *fn = (const void *)k_m32_chunk<CAP>;
     static std::atomic<bool> ready{false};
     cudaError_t e = cudaSuccess;
     if (!ready.load()) {
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMChunkSmemBytes<R>);
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMChunkSmemBytes);
         if (e != cudaSuccess) return e;
         ready = true;
     }
@@ -1343,15 +1340,14 @@ static cudaError_t launch_m32_resident(const MSetArgT<CAP> &A, GridBar *bar, int
     MSetArgT<CAP> a = A;
     void *args[] = {&a, &bar, &max_iters};
     count_launches(1);
-    return cudaLaunchCooperativeKernel(fn, (A.total_chunks + R - 1) / R, CH, args, kMChunkSmemBytes<R>, st);
+    return cudaLaunchCooperativeKernel(fn, A.total_chunks, CH, args, kMChunkSmemBytes, st);
 }
 
 template <int CAP>
 cudaError_t launch_m32_loop(const MSetArgT<CAP> &A, GridBar *bar, int max_iters, cudaStream_t st, int variant,
                             int share) {
     if (A.total_chunks <= 0 || max_iters <= 0) return cudaSuccess;
-    if (A.resident == 1) return launch_m32_resident<CAP, 1>(A, bar, max_iters, st);
-    if (A.resident == 2) return launch_m32_resident<CAP, 2>(A, bar, max_iters, st);
+    if (A.resident) return launch_m32_resident(A, bar, max_iters, st);
     long rows = 0;
     bool mg = false;
     for (int i = 0; i < A.nsys; ++i) {

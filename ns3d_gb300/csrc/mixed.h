@@ -83,7 +83,7 @@ constexpr int KMAX_MERGED_M = 32;
 template <int CAP>
 struct MSetArgT {
     int nsys, total_chunks;
-    int resident, pad_;  // chunks per block of the loop with resident chunks; 0: the other loops (plan_mixed)
+    int resident, pad_;  // 1: the loop with resident chunks, 0: the other loops (plan_mixed)
     MSys sys[CAP];
 };
 using MSetArg = MSetArgT<KMAX>;
