@@ -1304,7 +1304,7 @@ void launch_m32_init(const MSetArgT<CAP> &A, cudaStream_t st) {
 // Sets up to kFusedRows rows run the three-phase loop (fewer barriers; the
 // recomputed neighbour operands are cache hits), larger ones the five-phase
 // loop (157 K rows: 47 ms three-phase, 51 five-phase for two SIMPLER outer
-// iterations; 440 K rows: 35 and 31 ms for one).
+// iterations; 498 K rows: 100 and 88 ms for one SIMPLERR outer iteration).
 constexpr long kFusedRows = 1L << 18;
 
 // (the V-cycle runs in the five-phase loop)
