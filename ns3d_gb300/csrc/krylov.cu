@@ -966,20 +966,9 @@ void plan_krylov(KSetArgT<CAP> &A, int share) {
 
 template <int CAP, int F>
 static cudaError_t launch_chunk(KSetArgT<CAP> &a, GridBar *bar, LoopProf *prof, int max_iters, cudaStream_t st) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(a.total_chunks * F);
-    cfg.blockDim = dim3(kChunkRows<F>);
-    cfg.dynamicSmemBytes = kChunkSmemBytes<F>;
-    cfg.stream = st;
-    cudaLaunchAttribute at[2];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    at[1].id = cudaLaunchAttributeClusterDimension;
-    at[1].val.clusterDim.x = F;
-    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = F > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, k_kr_chunk<CAP, F>, a, bar, prof, max_iters);
+    void *args[] = {&a, &bar, &prof, &max_iters};
+    return cudaLaunchCooperativeKernel((const void *)k_kr_chunk<CAP, F>, a.total_chunks * F, kChunkRows<F>, args,
+                                       kChunkSmemBytes<F>, st);
 }
 
 template <int CAP>

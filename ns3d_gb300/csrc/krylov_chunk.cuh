@@ -184,8 +184,10 @@ __device__ __forceinline__ double dot_all(const KSys &S, int lc, int kind, bool 
     return group_tree(sum, min(n, LANES), lane, red + LANES / 32, sync);
 }
 
+// (The cluster's size is part of the kernel: as an attribute of a cooperative
+// launch it made the launch fail under a profiler.)
 template <int CAP, int F>
-__global__ void __launch_bounds__(kChunkRows<F>, 1)
+__global__ void __cluster_dims__(F, 1, 1) __launch_bounds__(kChunkRows<F>, 1)
     k_kr_chunk(const __grid_constant__ KSetArgT<CAP> A, GridBar *bar, LoopProf *prof, int max_iters) {
     static_assert(CH == 1024, "one thread per row of a chunk");
     extern __shared__ double sm_chunk[];
@@ -282,13 +284,16 @@ __global__ void __launch_bounds__(kChunkRows<F>, 1)
     // accumulated; false when a wait ran out
     int bad = 0;
     unsigned int parity = 0;
+    bool late = false;  // the wait for the operands ran out
     auto handed = [&](unsigned int count) {
         if (F > 1 && first) {
             if (t == 0) mbar_expect(&s_handed, count * CH * (unsigned int)sizeof(double));
             PollLimit limit(bar, bad);
-            while (!mbar_done(&s_handed, parity) && limit.again()) {
+            bool done;
+            while (!(done = mbar_done(&s_handed, parity)) && limit.again()) {
             }
-            parity ^= 1u;
+            if (done) parity ^= 1u;
+            else late = true;
         }
         return __syncthreads_or(bad) == 0;
     };
@@ -430,8 +435,17 @@ __global__ void __launch_bounds__(kChunkRows<F>, 1)
         prof->iters += it;
         prof->ok = bad ? 0 : 1;
     }
-    // the first block's shared memory stays until the others' last store to it
-    if (F > 1) cluster_barrier();
+    // The first block's shared memory stays until the others' last store to it.
+    // It has waited for all of them, unless a wait ran out: stores that were
+    // issued before the barrier may then still be on their way (bounded wait).
+    if (F > 1) {
+        cluster_barrier();
+        if (late) {
+            PollLimit limit(bar, bad);
+            while (!mbar_done(&s_handed, parity) && limit.again()) {
+            }
+        }
+    }
 }
 
 }  // namespace ns3d
