@@ -595,19 +595,25 @@ __device__ bool mg_apply(const MSys &S, const float *b0, float *x0, TailLevels &
                          int *s_ok) {
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const int gth = gridDim.x * blockDim.x;
+    // a level of at most one row per thread: warps of consecutive rows go round
+    // the blocks, so that a few thousand rows do not end up on a few SMs (205 K
+    // rows, five levels: 73.5 -> 72.0 ms; large levels lose 0.2% this way)
+    const int spread = ((threadIdx.x / 32) * gridDim.x + blockIdx.x) * 32 + (threadIdx.x & 31);
+    auto first = [&](int n) { return n <= gth ? spread : gtid; };
     const int K = S.mg.nlev, tail = S.mg.tail;
     const float w = S.mg.omega;
     const float *cx = S.mg.lev[K].x;  // the coarse correction: the coarsest level's x, the other levels' xo
     for (int k = 0; k < K; ++k) {
         const MGView L = mg_level(S, k, b0, x0);
         const MGLevel &C = S.mg.lev[k + 1];
-        mg_pass(L.n, gtid, gth, [&](int r) { return mg_down(L, r); }, [&](int r, float v) { C.t8[ro(C.pos + r)] = v; });
+        mg_pass(L.n, first(L.n), gth, [&](int r) { return mg_down(L, r); },
+                [&](int r, float v) { C.t8[ro(C.pos + r)] = v; });
         if (!grid_sync(bar, target, s_ok)) return false;
         if (k + 1 == tail) {
             cx = mg_tail(S.mg, T);
             break;
         }
-        for (int I = gtid; I < C.n; I += gth) mg_restrict(C, w, I);
+        for (int I = first(C.n); I < C.n; I += gth) mg_restrict(C, w, I);
         if (!grid_sync(bar, target, s_ok)) return false;
     }
     if (tail > K) {
@@ -617,7 +623,8 @@ __device__ bool mg_apply(const MSys &S, const float *b0, float *x0, TailLevels &
     for (int k = min(K, tail) - 1; k >= 0; --k) {
         const MGView L = mg_level(S, k, b0, x0);
         const int *pos = S.mg.lev[k + 1].pos;
-        mg_pass(L.n, gtid, gth, [&](int r) { return mg_up(L, pos, cx, w, r); }, [&](int r, float v) { L.xo[r] = v; });
+        mg_pass(L.n, first(L.n), gth, [&](int r) { return mg_up(L, pos, cx, w, r); },
+                [&](int r, float v) { L.xo[r] = v; });
         if (!grid_sync(bar, target, s_ok)) return false;
         cx = L.xo;
     }
