@@ -92,6 +92,19 @@ __device__ __forceinline__ double row_ordered(int row, int nW, int nE, int nS, i
     return acc;
 }
 
+// The six columns of a row from 8 bytes: the distances to W and E (16 bits),
+// S and N (15 bits), and one bit each for B and T, which are the rows before
+// and after it.  W, S and B columns lie before the row, E, N and T columns
+// after it; 0 is a missing entry, for which this returns the row itself.
+__device__ __forceinline__ void packed_columns(ushort4 q, int row, int (&c)[6]) {
+    c[0] = row - q.x;
+    c[1] = row + q.y;
+    c[2] = row - (q.z & 0x7fff);
+    c[3] = row + (q.w & 0x7fff);
+    c[4] = row - (q.z >> 15);
+    c[5] = row + (q.w >> 15);
+}
+
 // ---- BiCGSTAB state of one system ---------------------------------------
 struct KState {
     double rho, alpha, w, beta;   // Krylov scalars (beta = next step's beta)

@@ -160,6 +160,24 @@ __global__ void k_hb_nbr(const int *__restrict__ ccell, int nc, int npad, CellBo
     }
 }
 
+// The six columns of a row in 8 bytes (packed_columns).  *far is set when one
+// does not fit; the table is not used then.
+__global__ void k_pack_columns(const int *__restrict__ nbr, int npad, ushort4 *__restrict__ pack, int *far) {
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < npad; r += gridDim.x * blockDim.x) {
+        int d[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            const int c = nbr[(size_t)k * npad + r];
+            d[k] = c < 0 ? 0 : (k & 1) ? c - r : r - c;
+        }
+        if (d[0] < 0 || d[0] > 0xffff || d[1] < 0 || d[1] > 0xffff || d[2] < 0 || d[2] > 0x7fff || d[3] < 0 ||
+            d[3] > 0x7fff || d[4] < 0 || d[4] > 1 || d[5] < 0 || d[5] > 1)
+            *far = 1;
+        pack[r] = make_ushort4((unsigned short)d[0], (unsigned short)d[1], (unsigned short)(d[2] | d[4] << 15),
+                               (unsigned short)(d[3] | d[5] << 15));
+    }
+}
+
 static int hb_grid(long n) { return (int)std::max(1L, std::min((n + 255) / 256, (long)device_sm_count() * 16)); }
 
 void build_hierarchy(DevSys &S, cudaStream_t st) {
@@ -168,6 +186,15 @@ void build_hierarchy(DevSys &S, cudaStream_t st) {
     DBuf<int> cells[2];  // the row -> cell tables of the level being aggregated and of the new one
     const int *cell = S.cell.p;
     int nf = S.n, flip = 0;
+    DBuf<int> dfar;
+    int far = 0;
+    if (nf >= kPackRows) {
+        H->pack.alloc((size_t)S.npad, st);
+        dfar.alloc_zero(1, st);
+        count_launches(1);
+        k_pack_columns<<<hb_grid(S.npad), 256, 0, st>>>(S.nbr.p, S.npad, H->pack.p, dfar.p);
+        NS3D_CUDA_CHECK(cudaMemcpyAsync(&far, dfar.p, sizeof far, cudaMemcpyDeviceToHost, st));
+    }
     while (H->nlev < MG_MAX && nf > kMGCoarsest) {
         const CellBox cbox = box.coarse();
         const long nb = cbox.cells();
@@ -185,6 +212,10 @@ void build_hierarchy(DevSys &S, cudaStream_t st) {
         int2 total;
         NS3D_CUDA_CHECK(cudaMemcpyAsync(&total, tiles.p + ntiles, sizeof total, cudaMemcpyDeviceToHost, st));
         NS3D_CUDA_CHECK(cudaStreamSynchronize(st));
+        if (far) {  // (copied before the totals)
+            H->pack.release();
+            far = 0;
+        }
         const int nc = total.x;
         MGHostLevel &L = H->lev[++H->nlev];
         L.n = nc;

@@ -27,22 +27,38 @@
 
 namespace ns3d {
 
+// The six columns of a row, slots W, E, S, N, B, T, a missing one replaced by
+// the row itself: from the packed table where there is one (PACKED), or from
+// the table of columns.
+template <bool PACKED>
+__device__ __forceinline__ void row_columns(const int *nbr, const ushort4 *pack, int row, size_t np, int (&c)[6]) {
+    if (PACKED && pack) {
+        packed_columns(ro(pack + row), row, c);
+        return;
+    }
+#pragma unroll
+    for (int d = 0; d < 6; ++d) {
+        const int k = ro(nbr + d * np + row);
+        c[d] = k >= 0 ? k : row;
+    }
+}
+
 // FP32 row product.  A missing entry has a zero coefficient; its gather
 // reads the row's own (finite) element, so all seven products are issued
 // without branches (FP32 issue is plentiful on GB300).
+template <bool PACKED>
 __device__ __forceinline__ float spmv_f32_row(const MSys &S, int row, const float *__restrict__ x) {
     const size_t np = (size_t)S.npad;
-    const int *nb = S.nbr + row;
     const float *cf = S.coef32 + row;
-    const int nW = ro(nb + 0 * np), nE = ro(nb + 1 * np), nS = ro(nb + 2 * np), nN = ro(nb + 3 * np),
-              nB = ro(nb + 4 * np), nT = ro(nb + 5 * np);
+    int c[6];
+    row_columns<PACKED>(S.nbr, S.mg.pack, row, np, c);
     float acc = ro(cf) * x[row];
-    acc = __fmaf_rn(ro(cf + 1 * np), x[nW >= 0 ? nW : row], acc);
-    acc = __fmaf_rn(ro(cf + 3 * np), x[nS >= 0 ? nS : row], acc);
-    acc = __fmaf_rn(ro(cf + 5 * np), x[nB >= 0 ? nB : row], acc);
-    acc = __fmaf_rn(ro(cf + 6 * np), x[nT >= 0 ? nT : row], acc);
-    acc = __fmaf_rn(ro(cf + 4 * np), x[nN >= 0 ? nN : row], acc);
-    acc = __fmaf_rn(ro(cf + 2 * np), x[nE >= 0 ? nE : row], acc);
+    acc = __fmaf_rn(ro(cf + 1 * np), x[c[0]], acc);
+    acc = __fmaf_rn(ro(cf + 3 * np), x[c[2]], acc);
+    acc = __fmaf_rn(ro(cf + 5 * np), x[c[4]], acc);
+    acc = __fmaf_rn(ro(cf + 6 * np), x[c[5]], acc);
+    acc = __fmaf_rn(ro(cf + 4 * np), x[c[3]], acc);
+    acc = __fmaf_rn(ro(cf + 2 * np), x[c[1]], acc);
     return acc;
 }
 
@@ -312,6 +328,7 @@ __global__ void __launch_bounds__(LANES *G, 8 / G) k_m32_init(const __grid_const
 struct MGView {
     int n, npad;
     const int *nbr;
+    const ushort4 *pack;
     const float *coef, *invdiag;
     float *x, *b, *t, *xo;  // Jacobi start, right-hand side, residual, result
 };
@@ -324,6 +341,7 @@ __device__ __forceinline__ MGView mg_level(const MSys &S, int k, const float *b0
         L.n = S.n;
         L.npad = S.npad;
         L.nbr = S.nbr;
+        L.pack = S.mg.pack;
         L.coef = S.coef32;
         L.invdiag = S.invdiag32;
         L.x = S.p2;
@@ -335,6 +353,7 @@ __device__ __forceinline__ MGView mg_level(const MSys &S, int k, const float *b0
         L.n = G.n;
         L.npad = G.npad;
         L.nbr = G.nbr;
+        L.pack = nullptr;
         L.coef = G.coef;
         L.invdiag = G.invdiag;
         L.x = G.x;
@@ -348,21 +367,26 @@ __device__ __forceinline__ MGView mg_level(const MSys &S, int k, const float *b0
 // row of A x at one level, x given by a function of the row (slot d+1 couples
 // through neighbour d; a missing neighbour has a zero coefficient and takes
 // the row itself)
-template <class F>
+template <bool PACKED, class F>
 __device__ __forceinline__ float mg_spmv_fn(const MGView &L, int row, F xf) {
     const size_t np = (size_t)L.npad;
-    const int *nb = L.nbr + row;
     const float *cf = L.coef + row;
+    int c[6];
+    if (PACKED) row_columns<PACKED>(L.nbr, L.pack, row, np, c);
     float acc = ro(cf) * xf(row);
 #pragma unroll
     for (int d = 0; d < 6; ++d) {
-        const int c = ro(nb + d * np);
-        acc = __fmaf_rn(ro(cf + (d + 1) * np), xf(c >= 0 ? c : row), acc);
+        if (!PACKED) {
+            c[d] = ro(L.nbr + d * np + row);
+            if (c[d] < 0) c[d] = row;
+        }
+        acc = __fmaf_rn(ro(cf + (d + 1) * np), xf(c[d]), acc);
     }
     return acc;
 }
+template <bool PACKED>
 __device__ __forceinline__ float mg_spmv(const MGView &L, int row, const float *x) {
-    return mg_spmv_fn(L, row, [&](int c) { return x[c]; });
+    return mg_spmv_fn<PACKED>(L, row, [&](int c) { return x[c]; });
 }
 
 // The passes of a V-cycle, one row each.  Down: the residual of the level's
@@ -371,7 +395,10 @@ __device__ __forceinline__ float mg_spmv(const MGView &L, int row, const float *
 // a member list and scattered residuals), then the restriction with the next
 // level's Jacobi start.  Up: x with the coarse correction cx added on the fly
 // and one damped Jacobi sweep, into xo (the neighbours still read x).
-__device__ __forceinline__ float mg_down(const MGView &L, int r) { return L.b[r] - mg_spmv(L, r, L.x); }
+template <bool PACKED>
+__device__ __forceinline__ float mg_down(const MGView &L, int r) {
+    return L.b[r] - mg_spmv<PACKED>(L, r, L.x);
+}
 // sum over a coarse row's members in ascending order; the unused places add +0
 // to a sum that starts at +0, which changes nothing
 __device__ __forceinline__ float mg_sum8(const float *t8, int I) {
@@ -386,9 +413,10 @@ __device__ __forceinline__ void mg_restrict(const MGLevel &C, float w, int I) {
     C.b[I] = acc;
     C.x[I] = w * C.invdiag[I] * acc;
 }
+template <bool PACKED>
 __device__ __forceinline__ float mg_up(const MGView &L, const int *pos, const float *cx, float w, int r) {
     const float x = L.x[r] + cx[ro(pos + r) >> 3];
-    const float t = L.b[r] - mg_spmv_fn(L, r, [&](int c) { return c == r ? x : L.x[c] + cx[ro(pos + c) >> 3]; });
+    const float t = L.b[r] - mg_spmv_fn<PACKED>(L, r, [&](int c) { return c == r ? x : L.x[c] + cx[ro(pos + c) >> 3]; });
     return x + w * L.invdiag[r] * t;
 }
 // store(r, value(r)) for the rows r < n of the calling thread, two at a time
@@ -414,7 +442,7 @@ __device__ void mg_coarsest(const MGView &L, float w, int sweeps) {
     for (int r = threadIdx.x; r < L.n; r += blockDim.x) L.x[r] = w * L.invdiag[r] * L.b[r];
     __syncthreads();
     for (int it = 0; it < sweeps; ++it) {
-        for (int r = threadIdx.x; r < L.n; r += blockDim.x) L.t[r] = L.b[r] - mg_spmv(L, r, L.x);
+        for (int r = threadIdx.x; r < L.n; r += blockDim.x) L.t[r] = L.b[r] - mg_spmv<false>(L, r, L.x);
         __syncthreads();
         for (int r = threadIdx.x; r < L.n; r += blockDim.x) L.x[r] += w * L.invdiag[r] * L.t[r];
         __syncthreads();
@@ -591,6 +619,7 @@ __device__ const float *mg_tail(const MGSet &G, TailLevels &T) {
 // With the tail in shared memory an iteration of a 205 K-row system (five
 // levels) has 21 grid barriers instead of 53 with three passes each way and
 // every level in the grid: 117 -> 78 us.
+template <bool PACKED>
 __device__ bool mg_apply(const MSys &S, const float *b0, float *x0, TailLevels &T, GridBar *bar, unsigned int &target,
                          int *s_ok) {
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -606,7 +635,7 @@ __device__ bool mg_apply(const MSys &S, const float *b0, float *x0, TailLevels &
     for (int k = 0; k < K; ++k) {
         const MGView L = mg_level(S, k, b0, x0);
         const MGLevel &C = S.mg.lev[k + 1];
-        mg_pass(L.n, first(L.n), gth, [&](int r) { return mg_down(L, r); },
+        mg_pass(L.n, first(L.n), gth, [&](int r) { return mg_down<PACKED>(L, r); },
                 [&](int r, float v) { C.t8[ro(C.pos + r)] = v; });
         if (!grid_sync(bar, target, s_ok)) return false;
         if (k + 1 == tail) {
@@ -623,7 +652,7 @@ __device__ bool mg_apply(const MSys &S, const float *b0, float *x0, TailLevels &
     for (int k = min(K, tail) - 1; k >= 0; --k) {
         const MGView L = mg_level(S, k, b0, x0);
         const int *pos = S.mg.lev[k + 1].pos;
-        mg_pass(L.n, first(L.n), gth, [&](int r) { return mg_up(L, pos, cx, w, r); },
+        mg_pass(L.n, first(L.n), gth, [&](int r) { return mg_up<PACKED>(L, pos, cx, w, r); },
                 [&](int r, float v) { L.xo[r] = v; });
         if (!grid_sync(bar, target, s_ok)) return false;
         cx = L.xo;
@@ -675,7 +704,7 @@ __device__ bool mg_apply_set(const MSetArgT<CAP> &A, const KState *sst, const in
         mg_rows(A, part, [&](int q) { return k == 0 ? A.sys[q].n : A.sys[q].mg.lev[k].n; },
                 [&](int q, int r) {
                     const MGLevel &C = A.sys[q].mg.lev[k + 1];
-                    C.t8[ro(C.pos + r)] = mg_down(lvl(q, k), r);
+                    C.t8[ro(C.pos + r)] = mg_down<false>(lvl(q, k), r);
                 });
         if (!grid_sync(bar, target, s_ok)) return false;
         mg_rows(A, part, [&](int q) { return A.sys[q].mg.lev[k + 1].n; },
@@ -697,7 +726,7 @@ __device__ bool mg_apply_set(const MSetArgT<CAP> &A, const KState *sst, const in
         mg_rows(A, part, rows, [&](int q, int r) {
             const MGLevel &C = A.sys[q].mg.lev[k + 1];
             const MGView L = lvl(q, k);
-            L.xo[r] = mg_up(L, C.pos, k + 1 == A.sys[q].mg.nlev ? C.x : C.xo, A.sys[q].mg.omega, r);
+            L.xo[r] = mg_up<false>(L, C.pos, k + 1 == A.sys[q].mg.nlev ? C.x : C.xo, A.sys[q].mg.omega, r);
         });
         if (!grid_sync(bar, target, s_ok)) return false;
     }
@@ -705,13 +734,13 @@ __device__ bool mg_apply_set(const MSetArgT<CAP> &A, const KState *sst, const in
 }
 
 // y = M^-1 p (which = 0) or z = M^-1 s (1) for the multilevel systems of a set
-template <int CAP>
+template <bool PACKED, int CAP>
 __device__ __forceinline__ bool mg_precondition(const MSetArgT<CAP> &A, const KState *sst, const int *sdc,
                                                 int which, TailLevels &T, GridBar *bar, unsigned int &target,
                                                 int *s_ok) {
     if constexpr (CAP <= KMAX) {  // one solver instance's set: a single system
         const MSys &S = A.sys[0];
-        return which == 0 ? mg_apply(S, S.p, S.y, T, bar, target, s_ok) : mg_apply(S, S.s, S.z, T, bar, target, s_ok);
+        return which == 0 ? mg_apply<PACKED>(S, S.p, S.y, T, bar, target, s_ok) : mg_apply<PACKED>(S, S.s, S.z, T, bar, target, s_ok);
     } else {
         return mg_apply_set(A, sst, sdc, which, bar, target, s_ok);
     }
@@ -799,7 +828,7 @@ struct UnitPair {
     __device__ __forceinline__ const MSys &S(const MSetArgT<CAP> &A, int h) const { return A.sys[si[h]]; }
 };
 
-template <bool FUSED, int CAP>
+template <bool FUSED, int CAP, bool PACKED = false>
 __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
     k_m32_loop(const __grid_constant__ MSetArgT<CAP> A, GridBar *bar, int max_iters) {
     static_assert(CAP <= LOOP_THREADS, "one thread copies each system's state");
@@ -1001,7 +1030,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
             });
             if (!grid_sync(bar, target, &s_ok)) break;
             // multilevel preconditioning: y = M^-1 p (replaces the Jacobi y)
-            if (mg_on && !mg_precondition(A, sst, sdc, 0, s_tail, bar, target, &s_ok)) break;
+            if (mg_on && !mg_precondition<PACKED>(A, sst, sdc, 0, s_tail, bar, target, &s_ok)) break;
             // v = A y, <r0, v>
             unit_phase([&](auto units) {
                 constexpr int H = decltype(units)::value;
@@ -1014,7 +1043,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
 #pragma unroll
                         for (int m = 0; m < MRPL; ++m) {
                             const int row = U.lc[h] * MUNIT + lane + m * LANES;
-                            v[h][m] = spmv_f32_row(U.S(A, h), row, U.S(A, h).y);
+                            v[h][m] = spmv_f32_row<PACKED>(U.S(A, h), row, U.S(A, h).y);
                             q[h][m] = U.S(A, h).r0[row];
                         }
 #pragma unroll
@@ -1054,7 +1083,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
                 return Pair4{S.s, out, sv, z};
             });
             if (!grid_sync(bar, target, &s_ok)) break;
-            if (mg_on && !mg_precondition(A, sst, sdc, 1, s_tail, bar, target, &s_ok)) break;
+            if (mg_on && !mg_precondition<PACKED>(A, sst, sdc, 1, s_tail, bar, target, &s_ok)) break;
             // t = A z, <t, t>, <t, s>
             unit_phase([&](auto units) {
                 constexpr int H = decltype(units)::value;
@@ -1067,7 +1096,7 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
 #pragma unroll
                         for (int m = 0; m < MRPL; ++m) {
                             const int row = U.lc[h] * MUNIT + lane + m * LANES;
-                            t[h][m] = spmv_f32_row(U.S(A, h), row, U.S(A, h).z);
+                            t[h][m] = spmv_f32_row<PACKED>(U.S(A, h), row, U.S(A, h).z);
                             q[h][m] = U.S(A, h).s[row];
                         }
 #pragma unroll
@@ -1362,11 +1391,15 @@ cudaError_t launch_m32_loop(const MSetArgT<CAP> &A, GridBar *bar, int max_iters,
         mg = mg || A.sys[i].mg.nlev > 0;
     }
     const bool fused = variant < 0 ? m32_fused(rows, mg) : (variant == 1 && !mg);
+    const bool packed = CAP <= KMAX && A.sys[0].mg.nlev > 0 && A.sys[0].mg.pack;
     const void *fn = fused ? (const void *)k_m32_loop<true, CAP> : (const void *)k_m32_loop<false, CAP>;
-    static std::atomic<int> occ_cache[2];
+    if constexpr (CAP <= KMAX)
+        if (packed) fn = (const void *)k_m32_loop<false, CAP, true>;
+    static std::atomic<int> occ_cache[3];
+    const int form = packed ? 2 : fused;
     const size_t tail_max = CAP <= KMAX && !fused ? kTailSmemMax : 0;
     const size_t smem = tail_max && A.sys[0].mg.nlev > 0 ? mg_tail_words(A.sys[0].mg) * 4 : 0;
-    int occ = occ_cache[fused].load();
+    int occ = occ_cache[form].load();
     if (occ == 0) {
         cudaError_t e = cudaSuccess;
         if (tail_max) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tail_max);
@@ -1374,7 +1407,7 @@ cudaError_t launch_m32_loop(const MSetArgT<CAP> &A, GridBar *bar, int max_iters,
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, LOOP_THREADS, tail_max);
         if (e != cudaSuccess) return e;
         if (occ <= 0) return cudaErrorLaunchOutOfResources;
-        occ_cache[fused] = occ;
+        occ_cache[form] = occ;
     }
     // a merged set (many solves' systems) spreads over its share of the SMs
     const int grid = CAP > KMAX

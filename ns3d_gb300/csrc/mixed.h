@@ -41,6 +41,7 @@ struct MGSet {
     int nlev;             // coarse levels (0: Jacobi preconditioning)
     int sweeps;           // Jacobi sweeps on the coarsest level
     float omega;          // damping of the Jacobi smoother
+    const ushort4 *pack;  // the system's columns in 8 bytes a row (row_columns) or null
     int tail;             // levels tail..nlev run in every block's shared memory (nlev + 1: none do)
     MGLevel lev[MG_MAX + 1];  // lev[1..nlev]; lev[0] unused (the system itself)
 };

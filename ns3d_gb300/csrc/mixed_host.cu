@@ -71,6 +71,7 @@ void MixedSetT<CAP>::configure(const std::vector<SolveItem> &items, cudaStream_t
         if (mg) {
             if (!S.mg) build_hierarchy(S, st);
             m.mg.nlev = S.mg->nlev;
+            m.mg.pack = S.mg->pack.p;
             m.mg.sweeps = 30;
             m.mg.omega = 0.6f;
             for (int k = 1; k <= S.mg->nlev; ++k) {

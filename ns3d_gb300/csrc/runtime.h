@@ -104,6 +104,7 @@ struct MGHostLevel {
 };
 struct MGHost {
     int nlev = 0;
+    DBuf<ushort4> pack;  // large systems: the columns of level 0 in 8 bytes a row
     MGHostLevel lev[MG_MAX + 1];
 };
 struct DevSys;
@@ -112,6 +113,12 @@ struct DevSys;
 // coordinates, until a level has at most kMGCoarsest rows or MG_MAX levels
 // exist.
 constexpr int kMGCoarsest = 512;
+// Systems of this many rows also get their columns in 8 instead of 24 bytes a
+// row, with a loop kernel of their own: their passes are bound by bytes once
+// the set outgrows L2, and the decoding costs what it saves below that.  Two
+// SIMPLEC outer iterations, 24 -> 8 bytes: 0.53 M rows 12.5 -> 12.5 ms, 0.8 M
+// 16.5 -> 16.2, 1.3 M 24.9 -> 23.4, 3.6 M 68.6 -> 65.9.
+constexpr int kPackRows = 1 << 19;
 void build_hierarchy(DevSys &S, cudaStream_t st);
 
 struct DevSys {
