@@ -34,7 +34,7 @@ next `--steps K` requests are timed in every leg.
               images, every request's fields read back to host memory
   rate_sweep  throughput and p50/p99 latency at the arrival rates of
               SWEEP_RATES (SWEEP_REQUESTS further requests of the stream each)
-  roofline    the FP64 BiCGSTAB loop kernel k_kr_loop of the plain FP64 leg
+  roofline    the FP64 BiCGSTAB loop kernels (k_kr_loop, k_kr_chunk) of the plain FP64 leg
               (one persistent cooperative launch per pressure solve): 408 B
               per row-iteration by the fixed (45s+48) formula over its
               CUDA-event time, against MEASURED_PEAKS.json
@@ -623,7 +623,7 @@ def run_gpu(args):
             "e2e": {"value": None if e2e_elapsed is None else world * K / e2e_elapsed, "unit": "solves/s",
                     "h2d_bytes_per_step": int(sum(it["nbytes"] for it in timed) / K),
                     "d2h_bytes_per_step": int(sum(8 * sum(s) for s in sizes) / K), "failed": e2e_failed},
-            "roofline": {"bound": "hbm", "kernel": "k_kr_loop (BiCGSTAB iterations of the pressure solves, "
+            "roofline": {"bound": "hbm", "kernel": "k_kr_loop, k_kr_chunk (BiCGSTAB iterations of the pressure solves, "
                                                    "plain FP64 leg)",
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "peak_kind": peak_kind,

@@ -20,8 +20,10 @@
 //   K3 s = r - alpha v; z = D^-1 s
 //   K4 t = A z, <t,t>, <t,s>                -> w
 //   K5 x += alpha y + w z; r = s - w t, <r0,r>, <r,r> -> convergence, beta
-// All iterations of a solve run in one persistent cooperative launch
-// (k_kr_loop), the phases separated by bounded grid barriers (loop.cuh).
+// All iterations of a solve run in one persistent cooperative launch:
+// k_kr_loop, the phases separated by bounded grid barriers (loop.cuh), or for
+// sets of at most one chunk per SM k_kr_chunk (krylov_chunk.cuh, included
+// below), which needs none.
 // The set-up (r = b - A x, norms) and the restart after |rho| breakdown are
 // separate launches whose last block to finish (one atomic counter per
 // system) combines the partials, so they wait on no other block.

@@ -10,7 +10,8 @@
 //                last block: convergence test, scale = 1/|r64|, inner target
 //   k_m32_init   f = float(r64 * scale); r = r0 = f; d = 0; p = v = 0; |f|^2
 //   k_m32_loop   the BiCGSTAB iterations in FP32 on A32 d = f (one
-//                persistent cooperative launch per round)
+//                persistent cooperative launch per round; small sets:
+//                k_m32_chunk, mixed_chunk.cuh)
 //   k_dc_step    theta minimizing |r64 - theta A64 delta|, delta = double(d) / scale
 //   k_dc_update  x += theta delta
 // An inner solve stops at its relative target, at the iteration budget, or
