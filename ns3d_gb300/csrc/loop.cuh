@@ -44,7 +44,8 @@ __device__ __forceinline__ void grid_arrive(GridBar *bar, unsigned int &target) 
 }
 
 // The second half.  Between the two a block may work on what no other block
-// reads or writes.
+// reads or writes before a later barrier of the launch: this one orders only
+// what came before the arrivals.
 __device__ __forceinline__ bool grid_wait(GridBar *bar, unsigned int target, int *s_ok) {
     if (threadIdx.x == 0) {
         int ok = 1;

@@ -889,22 +889,30 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
         }
         __syncthreads();
     };
+    // A walk over whole chunks: op(system index, system, i) for the chunks of
+    // the systems with on(system index), which takes elements 4 i .. 4 i + 3
+    // and 4 (i + LANES) .. 4 (i + LANES) + 3.  An element belongs to the same
+    // thread in every such walk.
+    auto each_chunk = [&](auto on, auto op) {
+        for (int c = cbegin; c < A.total_chunks; c += gstride) {
+            const int si = msys_of_chunk(A, c);
+            if (!on(si)) continue;
+            const MSys &S = A.sys[si];
+            op(si, S, (c - S.chunk_begin) * (CH / 4) + lane);
+        }
+    };
     // An element-wise phase: op(system index, system, i) computes elements
     // 4 i .. 4 i + 3 of one or two result vectors.  A group takes whole chunks,
     // a lane two float4 of each vector at once: with one row in flight per
     // thread K1, K3 and K5 took 30, 28 and 58 us at 3.6 M rows, now 11, 9 and 32.
     auto stream_chunks = [&](auto op) {
-        for (int c = cbegin; c < A.total_chunks; c += gstride) {
-            const int si = msys_of_chunk(A, c);
-            if (!inner_active(sst[si], sdc[si])) continue;
-            const MSys &S = A.sys[si];
-            const int i = (c - S.chunk_begin) * (CH / 4) + lane;
+        each_chunk([&](int si) { return inner_active(sst[si], sdc[si]); }, [&](int si, const MSys &S, int i) {
             const Pair4 e0 = op(si, S, i), e1 = op(si, S, i + LANES);
             reinterpret_cast<float4 *>(e0.pa)[i] = e0.a;
             if (e0.pb) reinterpret_cast<float4 *>(e0.pb)[i] = e0.b;
             reinterpret_cast<float4 *>(e1.pa)[i + LANES] = e1.a;
             if (e1.pb) reinterpret_cast<float4 *>(e1.pb)[i + LANES] = e1.b;
-        }
+        });
     };
     static_assert(CH == 8 * LANES, "two float4 a lane");
     {  // a launch that finds every system done returns at once
@@ -1190,7 +1198,10 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
                 }
             });
             grid_arrive(bar, target);
-            // x += alpha y + w z, while the other blocks arrive
+            // x += alpha y + w z, while the other blocks arrive.  The loop may end
+            // behind this barrier, which does not order what is written here: in
+            // this launch an element of x is read by the thread that wrote it, and
+            // by no other (each_chunk).
             stream_chunks([&](int si, const MSys &S, int i) {
                 const float alpha = (float)sst[si].alpha, w = (float)sst[si].w;
                 const float4 x = at4(S.x, i), y = at4(S.y, i), z = at4(S.z, i);
@@ -1221,16 +1232,31 @@ __global__ void __launch_bounds__(LOOP_THREADS, LOOP_MIN_BLOCKS)
     __shared__ double s_inv[CAP];
     if (threadIdx.x < A.nsys) s_inv[threadIdx.x] = 1.0 / A.sys[threadIdx.x].dc->scale;
     __syncthreads();
-    for (int u = cbegin; u < total_units; u += gstride) {
-        const int si = msys_of_chunk(A, u / MSUB);
-        if (sdc[si] || sst[si].info != 0) continue;
-        const MSys &S = A.sys[si];
-        const int r0 = (u - S.chunk_begin * MSUB) * MUNIT + lane;
-        float x[MRPL];
+    // (each element by the thread that last updated x there)
+    auto corrected = [&](int si) { return !sdc[si] && sst[si].info == 0; };
+    if constexpr (FUSED) {
+        for (int u = cbegin; u < total_units; u += gstride) {
+            const int si = msys_of_chunk(A, u / MSUB);
+            if (!corrected(si)) continue;
+            const MSys &S = A.sys[si];
+            const int r0 = (u - S.chunk_begin * MSUB) * MUNIT + lane;
+            float x[MRPL];
 #pragma unroll
-        for (int m = 0; m < MRPL; ++m) x[m] = S.x[r0 + m * LANES];
+            for (int m = 0; m < MRPL; ++m) x[m] = S.x[r0 + m * LANES];
 #pragma unroll
-        for (int m = 0; m < MRPL; ++m) S.d64[r0 + m * LANES] = (double)x[m] * s_inv[si];
+            for (int m = 0; m < MRPL; ++m) S.d64[r0 + m * LANES] = (double)x[m] * s_inv[si];
+        }
+    } else {
+        each_chunk(corrected, [&](int si, const MSys &S, int i) {
+            const float4 x[2] = {at4(S.x, i), at4(S.x, i + LANES)};
+            const double inv = s_inv[si];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                double2 *const d = reinterpret_cast<double2 *>(S.d64) + 2 * (i + h * LANES);
+                d[0] = make_double2((double)x[h].x * inv, (double)x[h].y * inv);
+                d[1] = make_double2((double)x[h].z * inv, (double)x[h].w * inv);
+            }
+        });
     }
     if (blockIdx.x == 0 && threadIdx.x < A.nsys) {
         KState k = sst[threadIdx.x];
