@@ -439,8 +439,10 @@ NS3D_API int ns3d_autotune_table(char *buf, int32_t cap);
  * context intact.  While extra_arrivals > 0, every barrier of every loop-kernel
  * launch in the process waits for that many arrivals beyond the grid's own,
  * which never come, and gives up after limit_s seconds (> 0, at most 10), so
- * a test can watch that path end without a fault.  extra_arrivals = 0
- * restores normal launches.  Not for use while other solves run.
+ * a test can watch that path end without a fault (small FP64 sets, which have
+ * no grid barriers: every wait for a dot product's partials, with
+ * extra_arrivals > 1 only those of the first block of each cluster).
+ * extra_arrivals = 0 restores normal launches.  Not for use while other solves run.
  */
 NS3D_API int ns3d_debug_barrier_timeout(int32_t extra_arrivals, double limit_s);
 /* ns3d_batch_solve with the solves merged in a group of `lanes` lanes;

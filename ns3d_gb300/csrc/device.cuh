@@ -176,6 +176,7 @@ struct GridBar {  // arrival counter and error flag on separate 128-byte lines
     // Zero in normal launches.  A test (ns3d_debug_barrier_timeout) sets
     // `bias`, arrivals every barrier waits for beyond the grid's own, which
     // never come, and `limit_ns`, a short wait limit (0 = kBarrierLimitNs).
+    // (The loops without grid barriers: krylov_chunk.cuh, mixed_chunk.cuh.)
     unsigned int bias;
     unsigned long long limit_ns;
     unsigned int pad0_[28];

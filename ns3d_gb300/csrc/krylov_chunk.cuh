@@ -40,7 +40,8 @@
 // the cluster made every block wait: 14.4 instead of 13.3 us at 44 chunks).
 // The operands of a reduction overwrite those of the one before, which the
 // first block has accumulated: its partial is part of the scalar that every
-// block needed to get there.
+// block needed to get there.  So no block is ever more than one hand-over
+// ahead of the first one, also when waits run out.
 //
 // What bounds it now: per block and iteration 27 FP64 operations a row at two
 // per clock (6.7 us for a whole chunk), three reductions of about 2.3 us (a chain of eight
@@ -79,6 +80,11 @@ __device__ __forceinline__ void mbar_init(unsigned long long *m) {
 __device__ __forceinline__ void mbar_expect(unsigned long long *m, unsigned int bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared.b64 _, [%0], %1;" ::"r"(smem_addr(m)), "r"(bytes) : "memory");
 }
+// bytes that will not arrive count as arrived
+__device__ __forceinline__ void mbar_forgo(unsigned long long *m, unsigned int bytes) {
+    asm volatile("mbarrier.complete_tx.relaxed.cluster.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(m)), "r"(bytes)
+                 : "memory");
+}
 __device__ __forceinline__ bool mbar_done(unsigned long long *m, unsigned int parity) {
     unsigned int ok;
     asm volatile(
@@ -91,7 +97,8 @@ __device__ __forceinline__ bool mbar_done(unsigned long long *m, unsigned int pa
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
 }
-// v to p, an address in this block's shared memory, in the cluster's first block
+// v to p, an address in this block's shared memory, in the cluster's first
+// block: counted by the barrier m there, or ordered by the next cluster barrier
 __device__ __forceinline__ void store_first(double *p, double v, unsigned long long *m) {
     unsigned int a, b;
     asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_addr(p)));
@@ -99,6 +106,11 @@ __device__ __forceinline__ void store_first(double *p, double v, unsigned long l
     asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(a),
                  "l"(__double_as_longlong(v)), "r"(b)
                  : "memory");
+}
+__device__ __forceinline__ void store_first(unsigned int *p, unsigned int v) {
+    unsigned int a;
+    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_addr(p)));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 
 // The column values of the thread's row, slots W, E, S, N, B, T: neighbours
@@ -204,6 +216,7 @@ __global__ void __cluster_dims__(F, 1, 1) __launch_bounds__(kChunkRows<F>, 1)
     __shared__ KState st;
     __shared__ double s_red[2][2 * (LANES / 32)], s_other, s_ratio;
     __shared__ __align__(8) unsigned long long s_handed;  // in the cluster's first block
+    __shared__ unsigned int s_sent[F];                    // there too
     const int t = threadIdx.x, gi = t / LANES;
     const int chunk = (int)blockIdx.x / F, part = (int)blockIdx.x % F;
     const KSys &S = A.sys[sys_of_chunk(A, chunk)];
@@ -276,8 +289,9 @@ __global__ void __cluster_dims__(F, 1, 1) __launch_bounds__(kChunkRows<F>, 1)
     };
     if (timing) s_tp[5] = global_ns();
     // a test (ns3d_debug_barrier_timeout) makes every wait for a chunk partial
-    // run out: it waits for epochs that are never written
-    const unsigned int never = bar->bias ? 0x80000000u : 0u;
+    // run out, or those of the clusters' first blocks: it waits for epochs that
+    // are never written
+    const unsigned int never = (bar->bias > 1 ? first : bar->bias == 1) ? 0x80000000u : 0u;
     const GroupSync sync{gi + 1};
     auto nothing = [] {};
     // the operands of a dot product (`count` a row) are complete where it is
@@ -285,6 +299,9 @@ __global__ void __cluster_dims__(F, 1, 1) __launch_bounds__(kChunkRows<F>, 1)
     int bad = 0;
     unsigned int parity = 0;
     bool late = false;  // the wait for the operands ran out
+    // in the iteration that ends the loop because a wait ran out: operands a
+    // row that the block has handed over, and that the first block has got
+    unsigned int sent = 0, taken = 0;
     auto handed = [&](unsigned int count) {
         if (F > 1 && first) {
             if (t == 0) mbar_expect(&s_handed, count * CH * (unsigned int)sizeof(double));
@@ -296,6 +313,10 @@ __global__ void __cluster_dims__(F, 1, 1) __launch_bounds__(kChunkRows<F>, 1)
             else late = true;
         }
         return __syncthreads_or(bad) == 0;
+    };
+    auto gave_up = [&](unsigned int before, unsigned int after) {
+        sent = after;
+        taken = late ? before : after;
     };
     if (F > 1) cluster_barrier();  // every block of the cluster runs
     int it = 0;
@@ -320,13 +341,19 @@ __global__ void __cluster_dims__(F, 1, 1) __launch_bounds__(kChunkRows<F>, 1)
             s_v[t] = v;
             if (F > 1) store_first(o_a + part * RB + t, v, &s_handed);
         }
-        if (!handed(1)) break;
+        if (!handed(1)) {
+            gave_up(0, 1);
+            break;
+        }
         if (gi == 0) {
             const double d = dot_all(S, lc, 0, first, o_r0, F == 1 ? s_v : o_a, t, ep, ep | never, s_red[0], sync, bar, bad,
                                      nothing);
             if (t == 0) st.alpha = st.rho / d;
         }
-        if (__syncthreads_or(bad)) break;
+        if (__syncthreads_or(bad)) {
+            gave_up(0, 1);
+            break;
+        }
         mark(1);
         // K3: s = r - alpha v; z = D^-1 s
         {
@@ -349,7 +376,10 @@ __global__ void __cluster_dims__(F, 1, 1) __launch_bounds__(kChunkRows<F>, 1)
                 store_first(o_b + part * RB + t, s_s[t], &s_handed);
             }
         }
-        if (!handed(2)) break;
+        if (!handed(2)) {
+            gave_up(1, 3);
+            break;
+        }
         if (gi < 2) {
             const double *ot = F == 1 ? s_t : o_a, *os = F == 1 ? s_s : o_b;
             const double d = dot_all(S, lc, 1 + gi, first, ot, gi == 0 ? ot : os, t % LANES, ep, ep | never, s_red[gi],
@@ -358,7 +388,10 @@ __global__ void __cluster_dims__(F, 1, 1) __launch_bounds__(kChunkRows<F>, 1)
             asm volatile("bar.sync 3, %0;" ::"n"(2 * LANES) : "memory");
             if (t == 0) st.w = (d > 0.0) ? s_other / d : 0.0;
         }
-        if (__syncthreads_or(bad)) break;
+        if (__syncthreads_or(bad)) {
+            gave_up(1, 3);
+            break;
+        }
         mark(3);
         // K5: r = s - w t, <r0, r>, <r, r>; x += alpha y + w z
         const double alpha = st.alpha, w = st.w;
@@ -367,7 +400,10 @@ __global__ void __cluster_dims__(F, 1, 1) __launch_bounds__(kChunkRows<F>, 1)
             s_r[t] = r;
             if (F > 1) store_first(o_a + part * RB + t, r, &s_handed);
         }
-        if (!handed(1)) break;
+        if (!handed(1)) {
+            gave_up(3, 4);
+            break;
+        }
         // x and the second ratio of beta in the time the partials travel: before
         // they are published this FP64 work would delay them
         auto update_x = [&](int q) { s_x[q] = __fma_rn(w, s_z[q], __fma_rn(alpha, s_y[q], s_x[q])); };
@@ -415,7 +451,10 @@ __global__ void __cluster_dims__(F, 1, 1) __launch_bounds__(kChunkRows<F>, 1)
                 update_x(t);
             }
         }
-        if (__syncthreads_or(bad)) break;
+        if (__syncthreads_or(bad)) {
+            gave_up(3, 4);
+            break;
+        }
         mark(4);
         if (!state_active(st)) {
             ++it;
@@ -435,14 +474,29 @@ __global__ void __cluster_dims__(F, 1, 1) __launch_bounds__(kChunkRows<F>, 1)
         prof->iters += it;
         prof->ok = bad ? 0 : 1;
     }
-    // The first block's shared memory stays until the others' last store to it.
-    // It has waited for all of them, unless a wait ran out: stores that were
-    // issued before the barrier may then still be on their way (bounded wait).
+    // The first block's shared memory stays until the last store to it has
+    // arrived.  At a regular end it has waited for all of them.  When a wait
+    // ran out, operands may be on their way that it did not wait for: of a
+    // hand-over whose wait ran out there (the barrier expects all blocks'
+    // bytes, some may never have been sent), or of the one after its last (its
+    // wait for the partials ran out, another block's did not; the barrier
+    // expects nothing).  Every block stores the operands of all its rows or of
+    // none, so the blocks' counts say what is still to come; it is waited for
+    // before the block ends.
     if (F > 1) {
+        if (t == 0) store_first(&s_sent[part], 4u * it + sent);
         cluster_barrier();
-        if (late) {
-            PollLimit limit(bar, bad);
-            while (!mbar_done(&s_handed, parity) && limit.again()) {
+        if (first && t == 0) {
+            unsigned int open = 0;
+#pragma unroll
+            for (int q = 0; q < F; ++q) open += s_sent[q] - (4u * it + taken);
+            if (open > 0) {
+                constexpr unsigned int bytes = RB * sizeof(double);
+                if (sent == taken) mbar_expect(&s_handed, open * bytes);
+                else if (open < (sent - taken) * F) mbar_forgo(&s_handed, ((sent - taken) * F - open) * bytes);
+                PollLimit limit(bar, bad);
+                while (!mbar_done(&s_handed, parity) && limit.again()) {
+                }
             }
         }
     }
