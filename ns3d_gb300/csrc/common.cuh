@@ -189,9 +189,3 @@ __device__ __forceinline__ void lanes_final_sum2(const double *part, int n, int 
 inline int ceil_div(long a, long b) { return (int)((a + b - 1) / b); }
 
 }  // namespace ns3d
-
-#define NS3D_CUDA_CHECK(expr)                                                          \
-    do {                                                                               \
-        cudaError_t _e = (expr);                                                       \
-        if (_e != cudaSuccess) throw ns3d::CudaError(_e, #expr, __FILE__, __LINE__);   \
-    } while (0)

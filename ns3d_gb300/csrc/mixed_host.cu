@@ -10,9 +10,9 @@ namespace ns3d {
 
 void DevSys::allocate_f32(cudaStream_t st) {
     if (coef32.n) return;
-    coef32.alloc_zero((size_t)7 * npad, st);
     invdiag32.alloc_zero(npad, st);
     for (DBuf<float> *b : {&fx, &fr, &fr0, &fp, &fv, &fy, &fs, &fz, &ft, &fp2, &fv2}) b->alloc_zero(npad, st);
+    coef32.alloc_zero((size_t)7 * npad, st);  // last: it stands for all of them
 }
 
 template <int CAP>
@@ -30,14 +30,10 @@ void MixedSetT<CAP>::configure(const std::vector<SolveItem> &items, cudaStream_t
     if (ns > CAP) throw ApiError(NS3D_ERR_ARG, "too many systems in one solve set");
     std::vector<MSys> ms(ns);
     int chunk = 0;
-    if (cap_ < ns) {
-        cap_ = ns;
-        const size_t lines = (state_bytes() + sizeof(GridBar) - 1) / sizeof(GridBar);
-        bar_.alloc_zero(lines, st);
-        h_bar_.alloc(lines);
-        out_st_.alloc_zero(ns, st);
-        h_out_.alloc(ns);
-    }
+    key_.clear();  // set_ may name freed buffers until the end of this set-up, should an allocation fail
+    bar_.reserve(ns, state_bytes(ns), st);
+    if ((int)out_st_.n < ns) out_st_.alloc_zero(ns, st);
+    if ((int)h_out_.n < ns) h_out_.alloc(ns);
     for (int i = 0; i < ns; ++i) {
         DevSys &S = *items[i].sys;
         S.allocate_f32(st);
@@ -62,8 +58,8 @@ void MixedSetT<CAP>::configure(const std::vector<SolveItem> &items, cudaStream_t
         m.p2 = S.fp2.p; m.v2 = S.fv2.p;
         m.y = S.fy.p; m.s = S.fs.p; m.z = S.fz.p; m.t = S.ft.p;
         m.part = S.part.p;
-        m.st = st_of(bar_.p) + i;
-        m.dc = dc_of(bar_.p) + i;
+        m.st = st_of(bar_.dev.p) + i;
+        m.dc = dc_of(bar_.dev.p) + i;
         // a solver instance's own set: the multilevel preconditioner for a
         // single system; a merged set: what each system's own set chose
         const bool mg = CAP > KMAX ? (items[i].mg && S.mg)
@@ -127,9 +123,9 @@ void MixedSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st, s
     configure(items, st);
     const int ns = nsys_;
     int maxit = 0;
-    DCState *const h_dc = dc_of(h_bar_.p);
-    KState *const h_st = st_of(h_bar_.p);
-    std::memset(h_bar_.p, 0, state_bytes());
+    DCState *const h_dc = dc_of(bar_.host.p);
+    KState *const h_st = st_of(bar_.host.p);
+    std::memset(bar_.host.p, 0, state_bytes(bar_.cap));
     for (int i = 0; i < ns; ++i) {
         DevSys &S = *items[i].sys;
         launch_to_f32(S.coef.p, S.invdiag.p, S.npad, S.coef32.p, S.invdiag32.p, st);
@@ -149,7 +145,7 @@ void MixedSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st, s
         h_dc[i] = d;
         maxit = std::max(maxit, items[i].maxit);
     }
-    NS3D_CUDA_CHECK(cudaMemcpyAsync(bar_.p, h_bar_.p, state_bytes(), cudaMemcpyHostToDevice, st));
+    NS3D_CUDA_CHECK(cudaMemcpyAsync(bar_.dev.p, bar_.host.p, state_bytes(bar_.cap), cudaMemcpyHostToDevice, st));
     plan_mixed(set_, variant, share);
     launch_dc_resid(set_, 1, st);
     // Every round runs at least one inner iteration per unfinished system, so
@@ -176,9 +172,9 @@ void MixedSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st, s
     // kernels skip the systems that are done already.
     while (true) {
         if (rounds > 0) {
-            NS3D_CUDA_CHECK(cudaMemcpyAsync(h_bar_.p, bar_.p, state_bytes(), cudaMemcpyDeviceToHost, st));
+            NS3D_CUDA_CHECK(cudaMemcpyAsync(bar_.host.p, bar_.dev.p, state_bytes(bar_.cap), cudaMemcpyDeviceToHost, st));
             NS3D_CUDA_CHECK(cudaStreamSynchronize(st));
-            if (total_chunks_ > 0 && h_bar_.p->err)
+            if (total_chunks_ > 0 && bar_.host.p->err)
                 throw ApiError(NS3D_ERR_TIMEOUT, "FP32 BiCGSTAB loop kernel: a grid barrier timed out");
             if (tune) {  // inner iterations of the round, from the FP64 states
                 double rows = 0;
@@ -199,7 +195,7 @@ void MixedSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st, s
             cand = grid_tuner().choose(tkey);
             NS3D_CUDA_CHECK(cudaEventRecord(ev_[0], st));
         }
-        NS3D_CUDA_CHECK(launch_m32_loop(set_, bar_.p, maxit + 64, st, variant, share << cand));
+        NS3D_CUDA_CHECK(launch_m32_loop(set_, bar_.dev.p, maxit + 64, st, variant, share << cand));
         if (tune) NS3D_CUDA_CHECK(cudaEventRecord(ev_[1], st));
         launch_dc_update(set_, st);
         launch_dc_resid(set_, 0, st);

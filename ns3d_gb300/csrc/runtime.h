@@ -12,86 +12,18 @@
 #include <vector>
 
 #include "../../include/ns3d_capi.h"
+#include "buffers.h"
 #include "device.cuh"
 #include "kernels.h"
 #include "mixed.h"
 
 namespace ns3d {
 
-struct CudaError : std::runtime_error {
-    cudaError_t code;
-    CudaError(cudaError_t e, const char *expr, const char *file, int line)
-        : std::runtime_error(std::string(cudaGetErrorString(e)) + " in " + expr + " (" + file + ":" +
-                             std::to_string(line) + ")"),
-          code(e) {}
-};
-
-struct ApiError : std::runtime_error {
-    int code;
-    ApiError(int c, const std::string &m) : std::runtime_error(m), code(c) {}
-};
-
 // records the text ns3d_last_error() returns on this thread; returns code
 int report_error(int code, const std::string &m);
 
-// owning device buffer
-// Device memory of the library: one stream-ordered pool per device, kept
-// reserved between solves (no cudaMalloc / cudaFree, which synchronize the
-// whole device and would stall every other solve running in the process).
-cudaMemPool_t device_pool();
 // bytes the pool holds reserved but unused (free for new solves)
 size_t pool_cached_bytes();
-
-// Device array allocated on a stream from the library pool and freed on the
-// same stream (stream-ordered: it may be released while work that uses it
-// is still queued on that stream).
-template <class T>
-struct DBuf {
-    T *p = nullptr;
-    size_t n = 0;
-    cudaStream_t st_ = nullptr;
-    DBuf() = default;
-    DBuf(const DBuf &) = delete;
-    DBuf &operator=(const DBuf &) = delete;
-    ~DBuf() { release(); }
-    void alloc(size_t count, cudaStream_t st) {
-        release();
-        n = count;
-        st_ = st;
-        if (count == 0) return;
-        cudaError_t e = cudaMallocFromPoolAsync((void **)&p, count * sizeof(T), device_pool(), st);
-        if (e != cudaSuccess) {
-            p = nullptr;
-            n = 0;
-            cudaGetLastError();
-            throw ApiError(NS3D_ERR_OOM, "device allocation of " + std::to_string(count * sizeof(T)) + " bytes failed");
-        }
-    }
-    void alloc_zero(size_t count, cudaStream_t st) {
-        alloc(count, st);
-        if (count) NS3D_CUDA_CHECK(cudaMemsetAsync(p, 0, count * sizeof(T), st));
-    }
-    void release() {
-        if (p) cudaFreeAsync(p, st_);
-        p = nullptr;
-        n = 0;
-    }
-};
-
-// Host staging array of the small per-solve state copies.  Pageable memory:
-// a device-to-host copy into it returns once the copy is done, and freeing
-// it does not synchronize the device (cudaFreeHost would).
-template <class T>
-struct HBuf {
-    std::vector<T> v;
-    T *p = nullptr;
-    size_t n = 0;
-    void alloc(size_t count) {
-        v.assign(count, T());
-        p = count ? v.data() : nullptr;
-        n = count;
-    }
-};
 
 inline int pad_rows(int n) { return ((n + CH - 1) / CH) * CH; }
 
@@ -185,11 +117,11 @@ template <int CAP>
 class KrylovSetT {
   public:
     void run(const std::vector<SolveItem> &items, cudaStream_t st, std::vector<SolveOutcome> &out);
-    const KState *device_state(int i) const { return reinterpret_cast<const KState *>(bar_.p + 1) + i; }
+    const KState *device_state(int i) const { return reinterpret_cast<const KState *>(bar_.dev.p + 1) + i; }
     // allocates the per-system state of `items` (and records them) without
     // solving: a merged run copies the final states here
     void prepare(const std::vector<SolveItem> &items, cudaStream_t st) { configure(items, st); }
-    KState *state_buffer() { return reinterpret_cast<KState *>(bar_.p + 1); }
+    KState *state_buffer() { return reinterpret_cast<KState *>(bar_.dev.p + 1); }
     long launches() const { return launches_; }
     void reset_launch_count() { launches_ = 0; }
 
@@ -210,11 +142,9 @@ class KrylovSetT {
     void configure(const std::vector<SolveItem> &items, cudaStream_t st);
     cudaEvent_t ev_[2] = {nullptr, nullptr};
     KSetArgT<CAP> set_;  // passed to every kernel by value
-    // the loop kernel's barrier and behind it the cap_ systems' states: one copy reads both back
-    DBuf<GridBar> bar_;
-    HBuf<GridBar> h_bar_;
+    // the loop kernel's barrier and behind it the systems' states: one copy reads both back
+    StateBuf<GridBar> bar_;
     HBuf<KState> h_up_;
-    int cap_ = 0;
     DBuf<LoopProf> prof_;
     int nsys_ = 0, total_chunks_ = 0;
     long launches_ = 0;
@@ -259,14 +189,12 @@ class MixedSetT {
   private:
     void configure(const std::vector<SolveItem> &items, cudaStream_t st);
     cudaEvent_t ev_[2] = {nullptr, nullptr};  // around the FP32 loop launch (merged sets: autotuner timing)
-    // the loop kernel's barrier, the outer and the inner states of cap_
+    // the loop kernel's barrier, the outer and the inner states of bar_.cap
     // systems in one buffer: one copy reads or writes them all
-    DBuf<GridBar> bar_;
-    HBuf<GridBar> h_bar_;
-    int cap_ = 0;
+    StateBuf<GridBar> bar_;
     static DCState *dc_of(GridBar *b) { return reinterpret_cast<DCState *>(b + 1); }
-    KState *st_of(GridBar *b) const { return reinterpret_cast<KState *>(dc_of(b) + cap_); }
-    size_t state_bytes() const { return sizeof(GridBar) + cap_ * (sizeof(DCState) + sizeof(KState)); }
+    KState *st_of(GridBar *b) const { return reinterpret_cast<KState *>(dc_of(b) + bar_.cap); }
+    static size_t state_bytes(int systems) { return sizeof(GridBar) + systems * (sizeof(DCState) + sizeof(KState)); }
     DBuf<KState> out_st_;
     HBuf<KState> h_out_;
     std::vector<const double *> key_;

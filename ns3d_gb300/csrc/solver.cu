@@ -105,13 +105,8 @@ void KrylovSetT<CAP>::configure(const std::vector<SolveItem> &items, cudaStream_
     }
     const int ns = (int)ks.size();
     if (ns > CAP) throw ApiError(NS3D_ERR_ARG, "too many systems in one solve set");
-    if (cap_ < ns) {
-        cap_ = ns;
-        const size_t lines = 1 + (ns * sizeof(KState) + sizeof(GridBar) - 1) / sizeof(GridBar);
-        bar_.alloc_zero(lines, st);
-        h_bar_.alloc(lines);
-        h_up_.alloc(ns);
-    }
+    bar_.reserve(ns, sizeof(GridBar) + ns * sizeof(KState), st);
+    if ((int)h_up_.n < ns) h_up_.alloc(ns);
     if (!prof_.n) {
         prof_.alloc_zero(1, st);
         for (cudaEvent_t &e : ev_) NS3D_CUDA_CHECK(cudaEventCreate(&e));
@@ -171,15 +166,15 @@ void KrylovSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st,
     // The first loop launch follows the set-up without a look at the states
     // (a kernel whose systems are all done returns at once): one wait for the
     // stream per launch, one copy of barrier and states per wait.
-    const KState *h_st = reinterpret_cast<const KState *>(h_bar_.p + 1);
+    const KState *h_st = reinterpret_cast<const KState *>(bar_.host.p + 1);
     bool any_paused = false;
     while (true) {
         if (loops > 0) {
-            NS3D_CUDA_CHECK(cudaMemcpyAsync(h_bar_.p, bar_.p, sizeof(GridBar) + ns * sizeof(KState),
+            NS3D_CUDA_CHECK(cudaMemcpyAsync(bar_.host.p, bar_.dev.p, sizeof(GridBar) + ns * sizeof(KState),
                                             cudaMemcpyDeviceToHost, st));
             NS3D_CUDA_CHECK(cudaStreamSynchronize(st));
             // (no launch, no flag: an empty set leaves an earlier run's)
-            if (total_chunks_ > 0 && h_bar_.p->err)
+            if (total_chunks_ > 0 && bar_.host.p->err)
                 throw ApiError(NS3D_ERR_TIMEOUT, "BiCGSTAB loop kernel: a grid barrier timed out");
             bool all_done = true;
             any_paused = false;
@@ -216,7 +211,7 @@ void KrylovSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st,
         }
         if (tune) cand = grid_tuner().choose(tkey);
         if (profiling || tune) NS3D_CUDA_CHECK(cudaEventRecord(ev_[0], st));
-        NS3D_CUDA_CHECK(launch_krylov_loop(set_, bar_.p, profiling ? prof_.p : nullptr, (int)(cap - issued), st,
+        NS3D_CUDA_CHECK(launch_krylov_loop(set_, bar_.dev.p, profiling ? prof_.p : nullptr, (int)(cap - issued), st,
                                            share << cand));
         if (profiling || tune) NS3D_CUDA_CHECK(cudaEventRecord(ev_[1], st));
         launches_ += 1;
