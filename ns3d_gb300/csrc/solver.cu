@@ -158,10 +158,10 @@ void KrylovSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st,
     // merged sets: the grid of each loop launch comes from the autotuner,
     // which is told the launch's time per row-iteration
     const bool tune = CAP > KMAX;
-    // (a one-chunk-per-block set runs one grid whatever the candidate: its
-    // times stay out of the class of the larger sets that share its size
-    // bucket, 128 to 255 chunks)
-    const uint64_t tkey = tuner_key(0, set_.one_per_block ? std::min(total_chunks_, 127) : total_chunks_, share);
+    // (a one-chunk-per-block set runs one grid whatever the candidate)
+    const uint64_t tkey = tuner_key(
+        0, set_.one_per_block ? fixed_grid_units(total_chunks_, device_sm_count() / std::max(share, 1)) : total_chunks_,
+        share);
     int cand = 0;
     // The first loop launch follows the set-up without a look at the states
     // (a kernel whose systems are all done returns at once): one wait for the

@@ -58,4 +58,13 @@ inline uint64_t tuner_key(int kind, long units, int share) {
     return ((uint64_t)kind << 48) | ((uint64_t)bucket << 32) | (uint32_t)share;
 }
 
+// The units under which a set of at most `limit` units is filed whose grid
+// does not depend on the candidate: in a bucket below that of every larger
+// set, so that its times, all of one grid, do not decide for those.
+inline long fixed_grid_units(long units, long limit) {
+    long first = 1;  // of the bucket of limit + 1
+    while (2 * first <= limit + 1) first *= 2;
+    return units < first ? units : first - 1;
+}
+
 }  // namespace ns3d
