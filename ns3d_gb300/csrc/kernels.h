@@ -93,6 +93,7 @@ void launch_krylov_init(const KSetArgT<CAP> &set, cudaStream_t st);
 template <int CAP>
 cudaError_t launch_krylov_loop(const KSetArgT<CAP> &set, GridBar *bar, LoopProf *prof, int max_iters,
                                cudaStream_t st, int share = 1);
+cudaError_t load_krylov_kernels();  // on the current device
 template <int CAP>
 void launch_krylov_restart(const KSetArgT<CAP> &set, cudaStream_t st);
 // blocks of a loop-kernel launch over `units` work units, units_per_chunk

@@ -1026,6 +1026,22 @@ void launch_krylov_restart(const KSetArgT<CAP> &A, cudaStream_t st) {
         k_kr_restart<CAP, NARROW_G><<<kr_grid(A.total_chunks), LANES * NARROW_G, 0, st>>>(A);
 }
 
+// Loads the code of every kernel that a set of up to KMAX systems can run (CUDA
+// loads a kernel when it is first used, and may allocate for it).
+cudaError_t load_krylov_kernels() {
+    for (const void *fn : {(const void *)k_kr_init<KMAX, WIDE_G>, (const void *)k_kr_init<KMAX, NARROW_G>,
+                           (const void *)k_kr_init2<KMAX>, (const void *)k_kr_restart<KMAX, WIDE_G>,
+                           (const void *)k_kr_restart<KMAX, NARROW_G>, (const void *)k_kr_chunk<KMAX, 1>,
+                           (const void *)k_kr_chunk<KMAX, 2>, (const void *)k_kr_chunk<KMAX, 4>,
+                           (const void *)k_kr_loop<KMAX, 0>, (const void *)k_kr_loop<KMAX, 1>,
+                           (const void *)k_kr_loop<KMAX, 2>, (const void *)k_kr_loop<KMAX, 4>}) {
+        cudaFuncAttributes at;
+        const cudaError_t e = cudaFuncGetAttributes(&at, fn);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 template void plan_krylov<KMAX>(KSetArg &, int);
 template void plan_krylov<KMAX_MERGED>(KSetArgMerged &, int);
 template void launch_krylov_init<KMAX>(const KSetArg &, cudaStream_t);

@@ -15,9 +15,10 @@
 // host-side stand-in), so the first call on each device looks the address up
 // with cudaGetSymbolAddress while that device is current, checks the result
 // and caches it.  Under CUDA's default lazy module loading this lookup is
-// also what places the array (and this module's code) on the device, so the
-// first call should come before the host reserves the rest of the device's
-// memory, and before any stream capture.
+// also what places the array on the device, and a kernel's code follows when
+// it is first used; which kernels a call runs depends on its size, so the
+// first call loads all of them.  It should come before the host reserves the
+// rest of the device's memory, and before any stream capture.
 // Every call shares the one array and overwrites it: calls that overlap on
 // the GPU (two streams, two host threads) race, so serialize them.
 #include <cstring>
@@ -46,7 +47,16 @@ constexpr int kMaxDevices = 64;
 std::mutex g_mu;
 void *g_addr[kMaxDevices] = {nullptr};
 
-// device address of the scratch array for the current device
+// Jacobi inverse diagonal (1/a_rr, or 1 for a zero diagonal)
+__global__ void k_noalloc_invdiag(const double *__restrict__ diag, int n, double *__restrict__ inv) {
+    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
+        const double d = diag[r];
+        inv[r] = (d != 0.0) ? 1.0 / d : 1.0;
+    }
+}
+
+// device address of the scratch array for the current device; the first time
+// there, every kernel that a call can run is loaded too
 int scratch_address(unsigned char **out) {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return NS3D_ERR_CUDA;
@@ -55,18 +65,13 @@ int scratch_address(unsigned char **out) {
         void *p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess || !p) return NS3D_ERR_CUDA;
+        cudaFuncAttributes at;
+        if (cudaFuncGetAttributes(&at, k_noalloc_invdiag) != cudaSuccess || load_krylov_kernels() != cudaSuccess)
+            return NS3D_ERR_CUDA;
         g_addr[dev] = p;
     }
     *out = (unsigned char *)g_addr[dev];
     return NS3D_OK;
-}
-
-// Jacobi inverse diagonal (1/a_rr, or 1 for a zero diagonal)
-__global__ void k_noalloc_invdiag(const double *__restrict__ diag, int n, double *__restrict__ inv) {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        const double d = diag[r];
-        inv[r] = (d != 0.0) ? 1.0 / d : 1.0;
-    }
 }
 
 // messages are static strings: reporting an error allocates nothing either
@@ -101,7 +106,7 @@ extern "C" NS3D_API int ns3d_bicgstab_noalloc(const double *coef, const int32_t 
     }
     unsigned char *base = nullptr;
     int rc = scratch_address(&base);
-    if (rc != NS3D_OK) return fail(rc, "cudaGetSymbolAddress failed for the scratch array");
+    if (rc != NS3D_OK) return fail(rc, "the scratch array or a kernel could not be placed on the device");
     double *vec = (double *)base;
     double *part = (double *)(base + kVecBytes);
     KState *dst = (KState *)(base + kStateOffset);
