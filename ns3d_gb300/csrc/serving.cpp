@@ -37,12 +37,19 @@ namespace {
 
 using Clock = std::chrono::steady_clock;
 
-// device bytes of one solve, from the image size: index maps, four systems
-// (coefficients, neighbour columns, Krylov workspace) and the fields; the
-// mixed path adds its FP32 copies.  A conservative per-cell bound.
+// Device bytes of one solve, from the image size: index maps, four systems
+// (coefficients, neighbour columns, Krylov workspace) and the fields.  The
+// mixed modes add the FP32 copies of the systems, 76 B a row (eight
+// coefficients, eleven vectors); the multilevel one also the pressure system's
+// hierarchy: 16 B a row (packed columns, place and member list), per coarse row
+// 116 B (operator and columns 52, vectors 20, residuals 32, lists 12) for at
+// most a seventh as many of them, and the index tables while it is built; 48 B a
+// cell leave room for image sides that are not powers of two.  A conservative
+// per-cell bound: every cell counts as a row.
 size_t estimate_bytes(const ns3d_params &p, int nx, int ny, int nz) {
     const double cells = (double)(nx + 2 * std::max(p.border, 0) + 1) * ny * nz;
-    const double per_cell = 4 * 4 + 4 * 200.0 + (p.precision == NS3D_MIXED ? 4 * 72.0 : 0.0);
+    const bool mixed = p.precision != NS3D_FP64, multilevel = p.precision == NS3D_MIXED_MG;
+    const double per_cell = 4 * 4 + 4 * 200.0 + (mixed ? 4 * 76.0 : 0.0) + (multilevel ? 48.0 : 0.0);
     return (size_t)(cells * per_cell) + (64u << 20);
 }
 
