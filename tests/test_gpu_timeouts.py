@@ -1,11 +1,14 @@
-"""A bounded wait that runs out in the FP64 loop that splits a chunk over four
-or two blocks: the call returns NS3D_ERR_TIMEOUT, and the next solve on the same
-handle gives the bits of a fresh one.  The wait limit is short and set for the
-one call only; nothing faults or hangs (ns3d_debug_barrier_timeout).
+"""A bounded wait that runs out, in each of the loop kernels: the call returns
+NS3D_ERR_TIMEOUT, and the next solve on the same handle gives the bits of a
+fresh one.  The wait limit is short and set for the one call only; nothing
+faults or hangs (ns3d_debug_barrier_timeout).  The sizes pick the kernel on 152
+SMs: a chunk split over four and two blocks, a chunk per block, two, four, eight
+and more chunks per block in FP64; the three FP32 loops, the multilevel one with
+its columns unpacked and packed.
 
-`extra` 2 lets only the first block of each cluster give up on the partials: the
-others go on to the next hand-over of operands, and the first one has to outlast
-their stores.
+`extra` 2 (a chunk split over a cluster) lets only the first block of each
+cluster give up on the partials: the others go on to the next hand-over of
+operands, and the first one has to outlast their stores.
 """
 import ctypes
 
@@ -18,7 +21,11 @@ from ns3d_gb300 import capi
 pytestmark = pytest.mark.gpu
 
 CASES = [(capi.FP64, (20, 32, 32), 1), (capi.FP64, (20, 32, 32), 2), (capi.FP64, (16, 8, 8), 2),
-         (capi.FP64, (64, 32, 32), 1), (capi.FP64, (64, 32, 32), 2)]
+         (capi.FP64, (64, 32, 32), 1), (capi.FP64, (64, 32, 32), 2), (capi.FP64, (100, 32, 32), 1),
+         (capi.FP64, (300, 32, 32), 1), (capi.FP64, (600, 32, 32), 1), (capi.FP64, (1200, 32, 32), 1),
+         (capi.FP64, (1300, 32, 32), 1),
+         (capi.MIXED, (100, 32, 32), 1), (capi.MIXED, (200, 32, 32), 1), (capi.MIXED, (300, 32, 32), 1),
+         (capi.MIXED_MG, (70, 70, 70), 1), (capi.MIXED_MG, (600, 32, 32), 1)]
 
 
 @pytest.mark.parametrize("precision,shape,extra", CASES,
