@@ -812,9 +812,11 @@ __global__ void k_mg_galerkin(int npad_f, const int *__restrict__ nbr_f, const f
 // r, p, v (cheap in FP32) instead of waiting for a barrier after their owners
 // store them; p and v alternate between two buffers so that a phase never
 // overwrites what a neighbour still reads.  Otherwise the five phases of the
-// FP64 loop.  The FP32
-// results follow no fixed-order contract, so the work unit is a quarter
-// chunk (MUNIT = 256 rows, MRPL = 2 per lane): a group finishes a unit in one
+// FP64 loop.  All
+// FP32 loops (also mixed_chunk.cuh) do the same arithmetic and add in the same
+// order, so a system's bits do not depend on the loop that solves it.  That
+// order is theirs, not the FP64 loops': the work unit is a quarter chunk
+// (MUNIT = 256 rows, MRPL = 2 per lane), so a group finishes a unit in one
 // round of loads, and a small system spreads over 4x more groups.  Every
 // block keeps a copy of the inner state; the kernel ends when every inner
 // solve of the round is done or after `max_iters` iterations.
@@ -1402,7 +1404,7 @@ constexpr size_t kTailSmemMax = ((size_t)21 * MG_TAIL_ROWS + MG_MAX) * 4;
 // block run the loop with resident chunks (mixed_chunk.cuh).  Ten SIMPLEC
 // outer iterations of a 56^3 image (pressure 103 chunks): 85 -> 68 ms.
 template <int CAP>
-void plan_mixed(MSetArgT<CAP> &A, int variant, int share) {
+void plan_mixed(MSetArgT<CAP> &A, int share) {
     A.resident = 0;
     for (int i = 0; i < A.nsys; ++i)
         if (A.sys[i].mg.nlev > 0) return;
@@ -1481,8 +1483,8 @@ void launch_dc_update(const MSetArgT<CAP> &A, cudaStream_t st) {
     k_dc_update<CAP><<<m_grid(A.total_chunks), LANES, 0, st>>>(A);
 }
 
-template void plan_mixed<KMAX>(MSetArg &, int, int);
-template void plan_mixed<KMAX_MERGED_M>(MSetArgMerged &, int, int);
+template void plan_mixed<KMAX>(MSetArg &, int);
+template void plan_mixed<KMAX_MERGED_M>(MSetArgMerged &, int);
 template void launch_dc_resid<KMAX>(const MSetArg &, int, cudaStream_t);
 template void launch_dc_resid<KMAX_MERGED_M>(const MSetArgMerged &, int, cudaStream_t);
 template void launch_m32_init<KMAX>(const MSetArg &, cudaStream_t);

@@ -99,18 +99,19 @@ void launch_to_f32(const double *coef, const double *invdiag, int npad, float *c
 // chooses the FP32 loop of a solve of the set (kept for all its rounds);
 // before the other launches
 template <int CAP>
-void plan_mixed(MSetArgT<CAP> &set, int variant, int share);
+void plan_mixed(MSetArgT<CAP> &set, int share);
 template <int CAP>
 void launch_dc_resid(const MSetArgT<CAP> &set, int first, cudaStream_t st);
 template <int CAP>
 void launch_m32_init(const MSetArgT<CAP> &set, cudaStream_t st);
-// The FP32 loop variant of a set: fused (three phases per iteration) when
-// the set has at most kFusedRows rows and no multilevel system, else the
-// five-phase loop.  A merged set runs the variant its members chose alone.
+// The FP32 loop variant of a set without resident chunks: fused (three phases
+// per iteration) when the set has at most kFusedRows rows and no multilevel
+// system, else the five-phase loop.  A merged set runs the variant its members
+// chose alone, which is a matter of speed: the bits are the same.
 bool m32_fused(long rows, bool mg);
 // FP32 inner iterations until every inner solve of the round is done
-// (variant: -1 from the set's own rows, 0 five-phase, 1 fused; a merged set
-// takes 1/share of the SMs)
+// (variant: -1 from the set's own rows, 0 five-phase, 1 fused, not asked for
+// with resident chunks; a merged set takes 1/share of the SMs)
 template <int CAP>
 cudaError_t launch_m32_loop(const MSetArgT<CAP> &set, GridBar *bar, int max_iters, cudaStream_t st,
                             int variant = -1, int share = 1);

@@ -146,7 +146,7 @@ void MixedSetT<CAP>::run(const std::vector<SolveItem> &items, cudaStream_t st, s
         maxit = std::max(maxit, items[i].maxit);
     }
     NS3D_CUDA_CHECK(cudaMemcpyAsync(bar_.dev.p, bar_.host.p, state_bytes(bar_.cap), cudaMemcpyHostToDevice, st));
-    plan_mixed(set_, variant, share);
+    plan_mixed(set_, share);
     launch_dc_resid(set_, 1, st);
     // Every round runs at least one inner iteration per unfinished system, so
     // maxit + 2 rounds bound the loop; each round's inner loop is bounded by

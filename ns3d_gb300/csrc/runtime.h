@@ -168,7 +168,8 @@ using KrylovSetMerged = KrylovSetT<KMAX_MERGED>;
 template <int CAP>
 class MixedSetT {
   public:
-    // variant: -1 from the set's own rows, 0 five-phase, 1 fused FP32 loop
+    // variant: -1 from the set's own rows, 0 five-phase, 1 fused FP32 loop (a set
+    // that fits the loop with resident chunks runs that one)
     void run(const std::vector<SolveItem> &items, cudaStream_t st, std::vector<SolveOutcome> &out,
              int variant = -1);
     // FP64 outcome of system i, mirrored into a KState (iter, info) for the
