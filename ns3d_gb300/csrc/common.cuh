@@ -36,8 +36,9 @@ __device__ __forceinline__ double warp_tree_sum(double v) {
 }
 
 // Tree sum over LANES threads (lane = this thread's index among them) that
-// synchronize with `sync`, the named barrier of their group.  Returns the tree sum in lane 0 (other lanes get an
-// unspecified value).  `sm` needs LANES doubles.
+// synchronize with `sync`, the named barrier of their group.  Returns the tree
+// sum in lane 0 (other lanes get an unspecified value).  `sm` needs one value
+// per warp.
 template <class T, class Sync>
 __device__ __forceinline__ T lanes_tree_sum(T v, int lane, T *sm, Sync sync) {
     v = v + __shfl_down_sync(0xffffffffu, v, 16);
@@ -59,7 +60,8 @@ __device__ __forceinline__ T lanes_tree_sum(T v, int lane, T *sm, Sync sync) {
 // Two tree sums at once, each with exactly the pairings of lanes_tree_sum.
 // After the first level of a warp, lanes 0-15 carry the first sum and lanes
 // 16-31 the second, so every later level is one shuffle and one add for
-// both (FP64 issue is scarce on this GPU).  Results valid in lane 0.
+// both (FP64 issue is scarce on this GPU).  Results valid in lane 0.  `sm`
+// needs two values per warp.
 template <class T, class Sync>
 __device__ __forceinline__ void lanes_tree_sum2(T a, T b, int lane, T *sm, T &ra, T &rb, Sync sync) {
     static_assert(2 * (LANES / 32) <= 32, "warp sums of both trees fit one warp");
@@ -124,7 +126,9 @@ __device__ __forceinline__ double lanes_extreme(double v, int lane, double *sm, 
 // (k_divergence) whatever the size, with eight 11, 17, 21 and 24 us.  Above
 // WIDE_CHUNKS_PER_SM chunks per SM the other blocks cover that latency and a
 // wide block only waits for its own reduction (10.5 M rows: k_dc_resid 426 us
-// with eight groups, 287 with two).
+// with eight groups, 287 with two).  The launch bounds ask for 1024 threads per
+// SM in either form, so 64 registers a thread: k_kr_init, k_kr_restart,
+// k_dc_resid and k_dc_step with two groups spill 110 to 200 bytes a thread.
 constexpr int WIDE_CHUNKS_PER_SM = 2;
 constexpr int WIDE_G = 8, NARROW_G = 2;
 inline bool wide_chunks(int nchunks, int sms) { return nchunks <= WIDE_CHUNKS_PER_SM * sms; }

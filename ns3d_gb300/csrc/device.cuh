@@ -154,7 +154,6 @@ using KSetArg = KSetArgT<KMAX>;
 using KSetArgMerged = KSetArgT<KMAX_MERGED>;
 static_assert(sizeof(KSetArgMerged) <= 32000, "kernel parameter space");
 
-// The persistent BiCGSTAB loop kernel: block shape and its grid barrier.
 // Loads of global data that no thread writes during the kernel (matrix
 // coefficients, neighbour tables, the multilevel hierarchy) go through the
 // read-only data path (measured 0.6% faster in the FP64 loop, 1.3% in the
@@ -163,13 +162,11 @@ static_assert(sizeof(KSetArgMerged) <= 32000, "kernel parameter space");
 template <class T>
 __device__ __forceinline__ T ro(const T *p) { return __ldg(p); }
 
-#ifndef NS3D_LOOP_THREADS
-#define NS3D_LOOP_THREADS 1024
-#endif
-constexpr int LOOP_THREADS = NS3D_LOOP_THREADS;
+// One block of 1024 threads per SM (64 registers a thread): the loops with
+// resident chunks need a thread per row, the tensor-memory layout eight groups.
+constexpr int LOOP_THREADS = 1024;
 constexpr int LOOP_GROUPS = LOOP_THREADS / LANES;
-// blocks per SM the loop kernels are compiled for (64 registers a thread)
-constexpr int LOOP_MIN_BLOCKS = LOOP_THREADS >= 1024 ? 1 : 1024 / LOOP_THREADS;
+constexpr int LOOP_MIN_BLOCKS = 1;
 static_assert(LOOP_GROUPS >= KMAX, "the FP32 loop kernel: group s combines the partials of system s");
 struct GridBar {  // arrival counter and error flag on separate 128-byte lines
     unsigned int count;

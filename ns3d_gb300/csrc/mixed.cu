@@ -812,14 +812,13 @@ __global__ void k_mg_galerkin(int npad_f, const int *__restrict__ nbr_f, const f
 // r, p, v (cheap in FP32) instead of waiting for a barrier after their owners
 // store them; p and v alternate between two buffers so that a phase never
 // overwrites what a neighbour still reads.  Otherwise the five phases of the
-// FP64 loop.  All
-// FP32 loops (also mixed_chunk.cuh) do the same arithmetic and add in the same
-// order, so a system's bits do not depend on the loop that solves it.  That
+// FP64 loop.  Every block keeps a copy of the inner state; the kernel ends when
+// every inner solve of the round is done or after `max_iters` iterations.
+// All FP32 loops (also mixed_chunk.cuh) do the same arithmetic and add in the
+// same order, so a system's bits do not depend on the loop that solves it.  The
 // order is theirs, not the FP64 loops': the work unit is a quarter chunk
 // (MUNIT = 256 rows, MRPL = 2 per lane), so a group finishes a unit in one
-// round of loads, and a small system spreads over 4x more groups.  Every
-// block keeps a copy of the inner state; the kernel ends when every inner
-// solve of the round is done or after `max_iters` iterations.
+// round of loads, and a small system spreads over 4x more groups.
 
 struct Pair4 {  // four elements of one or two result vectors
     float *pa, *pb;
