@@ -34,10 +34,14 @@ next `--steps K` requests are timed in every leg.
               images, every request's fields read back to host memory
   rate_sweep  throughput and p50/p99 latency at the arrival rates of
               SWEEP_RATES (SWEEP_REQUESTS further requests of the stream each)
-  roofline    the FP64 BiCGSTAB loop kernels (k_kr_loop, k_kr_chunk) of the plain FP64 leg
-              (one persistent cooperative launch per pressure solve): 408 B
-              per row-iteration by the fixed (45s+48) formula over its
-              CUDA-event time, against MEASURED_PEAKS.json
+  roofline    the FP64 BiCGSTAB loop kernels (k_kr_loop, k_kr_chunk) of the
+              plain FP64 leg (one persistent cooperative launch per pressure
+              solve), by size of the pressure system: up to eight 1024-row
+              chunks per SM the matrix stays on the SMs and the bound is FP64
+              issue (27 operations per row-iteration, 2 per clock and SM),
+              above that the bytes of the fused phases (360 per row-iteration
+              against MEASURED_PEAKS.json).  Over CUDA-event time; the line's
+              own figures are those of the class that takes most of it
   cpu_baseline  complete CPU-oracle solves of the 64^3 sphere pack
               (workloads.sphere64: radius 6, porosity 0.55, SIMPLEC,
               tolerances 1e-8, RMR < 1e-6) with every physical host core
@@ -86,13 +90,18 @@ SWEEP_REQUESTS = 6         # requests per rate of the sweep
 SERVE_ACTIVE = 8           # solves in flight at most
 SERVE_PRECISION = 2        # mixed precision with the multilevel pressure preconditioner
 K_TOL = 1e-4               # |dK/K| bar of the metric
-# algorithmic bytes of one FP64 BiCGSTAB iteration per row, by the fixed
-# formula (45s + 48) with s = 8: two SpMVs of (9s + 24) (7 coefficients, 6
-# indices, x in, y out), two Jacobi applications of 3s, 21s of vector
-# traffic.  The fused phases of the loop kernel touch 360 B (K1 48, K2 104,
-# K3 40, K4 104, K5 64: the Jacobi products ride in the p and s updates).
+# One FP64 BiCGSTAB iteration per row: operations on the FP64 pipe (two row
+# products of 7, 13 in the dot products and vector updates), and bytes by the
+# fixed formula (45s + 48) with s = 8: two SpMVs of (9s + 24) (7 coefficients, 6
+# indices, x in, y out), two Jacobi applications of 3s, 21s of vector traffic.
+# The fused phases of the loop kernel touch 360 B (K1 48, K2 104, K3 40, K4 104,
+# K5 64: the Jacobi products ride in the p and s updates) when nothing stays on
+# the SMs.
+LOOP_FP64_PER_ROW = 27
+FP64_PER_CLOCK = 2         # per SM
 LOOP_BYTES_PER_ROW = 408
 LOOP_FUSED_BYTES_PER_ROW = 360
+RESIDENT_CHUNKS_PER_SM = 8  # chunks of 1024 rows whose coefficients and columns stay on the SMs
 
 
 class Clocks:
@@ -190,15 +199,53 @@ def load_peaks():
 
 
 def ncu_traffic():
-    """DRAM bytes per row-iteration of the loop kernel from the committed ncu summary, if any."""
+    """(rows, DRAM bytes per row-iteration) of the loop kernel at the one size
+    that the committed ncu summary was captured at, if any."""
     path = os.path.join(ROOT, "profiles", "krylov_loop_fp64_128.md")
+    found = {}
     try:
         for line in open(path):
-            if line.startswith("dram_bytes_per_row_iteration:"):
-                return float(line.split(":")[1])
+            for key in ("captured_rows", "dram_bytes_per_row_iteration"):
+                if line.startswith(key + ":"):
+                    found[key] = float(line.split(":")[1])
     except OSError:
         pass
-    return None
+    if len(found) < 2:
+        return None
+    return {"rows": int(found["captured_rows"]), "bytes_per_row_iteration": found["dram_bytes_per_row_iteration"]}
+
+
+def roofline(prof, sms, clk):
+    """The loop kernels of the plain leg against their bounds, per size class."""
+    hbm, kind = load_peaks()
+    mhz = float((clk or {}).get("sm_max_mhz") or 2070.0)
+    classes = []
+    for name, q in prof.items():
+        if not q["launches"] or q["ms"] <= 0:
+            continue
+        sec = q["ms"] * 1e-3
+        gops = LOOP_FP64_PER_ROW * q["rows"] / sec / 1e9
+        gops_peak = FP64_PER_CLOCK * sms * mhz * 1e-3
+        gbs = LOOP_FUSED_BYTES_PER_ROW * q["rows"] / sec / 1e9
+        resident = name != "streamed"
+        classes.append({
+            "sets": name, "bound": "fp64" if resident else "hbm", "achieved": gops if resident else gbs,
+            "peak": gops_peak if resident else hbm, "unit": "G FP64 operations/s" if resident else "GB/s",
+            "frac": gops / gops_peak if resident else gbs / hbm,
+            "peak_kind": "2 per clock and SM at %g MHz" % mhz if resident else kind,
+            "fp64_frac": gops / gops_peak, "launches": q["launches"], "ms": q["ms"],
+            "avg_launch_ms": q["ms"] / q["launches"], "row_iterations_per_launch": q["rows"] / q["launches"],
+            "phase_us_per_iteration": [round(1e3 * m / max(q["iters"], 1), 2) for m in q["phase_ms"]]})
+    if not classes:
+        return None
+    top = max(classes, key=lambda c: c["ms"])
+    line = {k: top[k] for k in ("bound", "achieved", "peak", "unit", "frac", "peak_kind", "sets")}
+    line.update({"kernel": "k_kr_loop, k_kr_chunk (BiCGSTAB iterations of the pressure solves, plain FP64 leg)",
+                 "traffic": None, "traffic_captured": ncu_traffic(), "fp64_per_row_iteration": LOOP_FP64_PER_ROW,
+                 "bytes_per_row_iteration": LOOP_BYTES_PER_ROW,
+                 "fused_bytes_per_row_iteration": LOOP_FUSED_BYTES_PER_ROW,
+                 "launches": sum(c["launches"] for c in classes), "by_size": classes})
+    return line
 
 
 def physical_cores():
@@ -240,8 +287,13 @@ def describe(it):
 
 def plain_leg(capi, workloads, lib, items, torch):
     """Every request solved alone on the plain FP64 path; the loop kernel's
-    CUDA-event time and row-iterations of the pressure solves."""
-    recs, prof = [], {"ms": 0.0, "launches": 0, "rows": 0, "phase_ms": [0.0] * 5, "iters": 0}
+    CUDA-event time and row-iterations of the pressure solves, by the size of
+    the pressure system in chunks per SM (one: k_kr_chunk; up to eight and
+    more: k_kr_loop)."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    recs = []
+    prof = {k: {"ms": 0.0, "launches": 0, "rows": 0, "phase_ms": [0.0] * 5, "iters": 0}
+            for k in ("one_chunk_per_sm", "resident", "streamed")}
     total = 0.0
     for it in items:
         torch.cuda.synchronize()
@@ -254,12 +306,15 @@ def plain_leg(capi, workloads, lib, items, torch):
         s.close()
         dt = time.perf_counter() - t
         total += dt
-        prof["ms"] += p.ms[5]
-        prof["launches"] += p.launches[5]
-        prof["rows"] += p.rows[5]
-        prof["iters"] += p.launches[0]
+        chunks = (sizes[0] + 1023) // 1024
+        q = prof["one_chunk_per_sm" if chunks <= sms else
+                 "resident" if chunks <= RESIDENT_CHUNKS_PER_SM * sms else "streamed"]
+        q["ms"] += p.ms[5]
+        q["launches"] += p.launches[5]
+        q["rows"] += p.rows[5]
+        q["iters"] += p.launches[0]
         for k in range(5):
-            prof["phase_ms"][k] += p.ms[k]
+            q["phase_ms"][k] += p.ms[k]
         recs.append({"seconds": dt, "K": r.K, "outer_iterations": int(r.iterations), "converged": int(r.converged),
                      "sizes": sizes})
     return total, recs, prof
@@ -544,9 +599,6 @@ def run_gpu(args):
     errs = [abs(s["K"] - p["K"]) / abs(p["K"]) if (s and p["K"] != 0) else None for s, p in zip(served, plain)]
     valid = [e for e in errs if e is not None]
     p50, p99 = latency_stats(served)
-    peak, peak_kind = load_peaks()
-    achieved = LOOP_BYTES_PER_ROW * prof["rows"] / (prof["ms"] * 1e-3) / 1e9 if prof["ms"] > 0 else 0.0
-    traffic = ncu_traffic()
     cells = sum(p["sizes"][0] * (p["outer_iterations"] + 1) for p in plain)
     if rank == 0:
         sweep = None
@@ -623,19 +675,7 @@ def run_gpu(args):
             "e2e": {"value": None if e2e_elapsed is None else world * K / e2e_elapsed, "unit": "solves/s",
                     "h2d_bytes_per_step": int(sum(it["nbytes"] for it in timed) / K),
                     "d2h_bytes_per_step": int(sum(8 * sum(s) for s in sizes) / K), "failed": e2e_failed},
-            "roofline": {"bound": "hbm", "kernel": "k_kr_loop, k_kr_chunk (BiCGSTAB iterations of the pressure solves, "
-                                                   "plain FP64 leg)",
-                         "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "peak_kind": peak_kind,
-                         "traffic": None if traffic is None else traffic * prof["rows"] / max(prof["launches"], 1),
-                         "traffic_bytes_per_row_iteration": traffic,
-                         "bytes_per_row_iteration": LOOP_BYTES_PER_ROW,
-                         "fused_bytes_per_row_iteration": LOOP_FUSED_BYTES_PER_ROW,
-                         "avg_launch_ms": prof["ms"] / max(prof["launches"], 1),
-                         "row_iterations_per_launch": prof["rows"] / max(prof["launches"], 1),
-                         "launches": prof["launches"],
-                         "phase_us_per_iteration": [round(1e3 * m / max(prof["iters"], 1), 2)
-                                                    for m in prof["phase_ms"]]},
+            "roofline": roofline(prof, torch.cuda.get_device_properties(0).multi_processor_count, clk),
             "gpu_launches": int(launches),
             "cpu_baseline": cpu,
             "sphere64": sphere64,
