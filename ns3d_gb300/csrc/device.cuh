@@ -173,10 +173,13 @@ struct GridBar {  // arrival counter and error flag on separate 128-byte lines
     // Zero in normal launches.  A test (ns3d_debug_barrier_timeout) sets
     // `bias`, arrivals every barrier waits for beyond the grid's own, which
     // never come, and `limit_ns`, a short wait limit (0 = kBarrierLimitNs).
-    // (The loops without grid barriers: krylov_chunk.cuh, mixed_chunk.cuh.)
+    // The loops without grid barriers (krylov_chunk.cuh, mixed_chunk.cuh) wait
+    // for partials that never come; `bias_others` is the bias of the blocks of a
+    // cluster that are not its first.
     unsigned int bias;
     unsigned long long limit_ns;
-    unsigned int pad0_[28];
+    unsigned int bias_others;
+    unsigned int pad0_[27];
     int err, pad1_[31];
 };
 static_assert(sizeof(GridBar) == 256, "GridBar: two 128-byte lines");

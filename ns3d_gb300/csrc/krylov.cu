@@ -855,6 +855,7 @@ cudaError_t reset_grid_bar(GridBar *bar, cudaStream_t st) {
     std::memset(&h, 0, sizeof h);
     h.bias = bias;
     h.limit_ns = g_bar_limit_ns.load();
+    h.bias_others = bias > 1 ? 0 : bias;
     // pageable source: the copy is staged before the call returns
     return cudaMemcpyAsync(bar, &h, sizeof h, cudaMemcpyHostToDevice, st);
 }
